@@ -253,13 +253,13 @@ __global__ void __launch_bounds__(128, 5) k_batch_pairs32(const BatchDisc *__res
     }
 }
 
-template <int STRAT>
-__global__ void __launch_bounds__(128) k_batch_pairs64(const BatchDisc *__restrict__ discs,
+template <int STRAT, int KT, int CAT>
+__global__ void __launch_bounds__(128, minb64<CAT>()) k_batch_pairs64(const BatchDisc *__restrict__ discs,
                                                        const int64_t *__restrict__ starts,
                                                        const uint32_t *__restrict__ slot_disc, int ndisc, int64_t s0,
                                                        int64_t m, RunPool P, SliceOrder O, unsigned long long *counter)
 {
-    __shared__ double s_term[BATCH_WARPS][32 * (NT + 1)];
+    __shared__ __align__(16) double s_term[BATCH_WARPS][nterms64<CAT>() * TROW];
     __shared__ BatchDisc s_desc[BATCH_WARPS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int64_t first = *O.nheavy, end = m - (int64_t)*O.nover;
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(128) k_batch_pairs64(const BatchDisc *__restri
         const DevTree &T = D.T;
         const int64_t qi = j - __ldg(starts + lo);
         const double px = __ldg(D.qx + qi), py = __ldg(D.qy + qi), pz = __ldg(D.qz + qi);
-        pairs64_query<STRAT>(T, D.C64, P, t, qi, px, py, pz, STRAT != SCATTER ? (int64_t)__ldg(P.bnear + t) : -1,
+        pairs64_query<STRAT, KT, CAT>(T, D.C64, P, t, qi, px, py, pz, STRAT != SCATTER ? (int64_t)__ldg(P.bnear + t) : -1,
                              s_term[wib], lane);
     }
 }
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(128) k_batch_over(const BatchDisc *__restrict_
                                                     unsigned light_max, int leaf_size, unsigned long long *counter)
 {
     __shared__ double s_acc[ACC_SLOTS * ACC_STRIDE];
-    __shared__ double s_term[BATCH_WARPS][32 * (NT + 1)];
+    __shared__ __align__(16) double s_term[BATCH_WARPS][TBUF];
     __shared__ BatchDisc s_desc[BATCH_WARPS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int64_t first = m - (int64_t)*O.nover;
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(128) k_batch_over(const BatchDisc *__restrict_
         const double px = __ldg(D.qx + qi), py = __ldg(D.qy + qi), pz = __ldg(D.qz + qi);
         const int64_t bnear = STRAT != SCATTER ? (int64_t)__ldg(P.bnear + t) : -1;
         const bool fp64 = fp64_only || count_accepted<STRAT>(T, px, py, pz, bnear, leaf_size) <= (int64_t)light_max;
-        if (fp64) points64_query<STRAT>(T, D.C64, px, py, pz, bnear, qi, s_term[wib], lane, leaf_size);
+        if (fp64) points64_query<STRAT, KT>(T, D.C64, px, py, pz, bnear, qi, s_term[wib], lane, leaf_size);
         else points32_query<STRAT, KT>(T, D.C32, D.pay, D.stride, px, py, pz, bnear, qi, s_acc, lane, leaf_size);
     }
 }
@@ -324,14 +324,17 @@ static int persistent_blocks_of(KERN kern, int cap)
 }
 
 template <int STRAT, int KT>
-static void launch_slice_pairs(Handle *H, int cat, const BatchDisc *discs, const int64_t *starts, const uint32_t *slot_disc,
+static void launch_slice_pairs(Handle *H, int cat, int cat64, const BatchDisc *discs, const int64_t *starts, const uint32_t *slot_disc,
                                int ndisc, int64_t s0, int64_t m, const RunPool &P, const SliceOrder &O, int fp64_only,
                                unsigned light_max, int leaf_size, int blocks_per_sm, unsigned long long *ctr)
 {
-    if (!fp64_only) {
 #define PB_PAIRS32(CAT)                                                                                            \
     k_batch_pairs32<STRAT, KT, CAT><<<persistent_blocks_of(k_batch_pairs32<STRAT, KT, CAT>, blocks_per_sm), 128, 0,     \
                                       H->stream>>>(discs, starts, slot_disc, ndisc, s0, P, O, ctr)
+#define PB_PAIRS64(CAT)                                                                                            \
+    k_batch_pairs64<STRAT, KT, CAT><<<persistent_blocks_of(k_batch_pairs64<STRAT, KT, CAT>, blocks_per_sm), 128, 0,     \
+                                      H->stream>>>(discs, starts, slot_disc, ndisc, s0, m, P, O, ctr + 1)
+    if (!fp64_only) {
         switch (cat) {
         case CAT_GDC4: PB_PAIRS32(CAT_GDC4); break;
         case CAT_C4: PB_PAIRS32(CAT_C4); break;
@@ -339,10 +342,16 @@ static void launch_slice_pairs(Handle *H, int cat, const BatchDisc *discs, const
         case CAT_SG1: PB_PAIRS32(CAT_SG1); break;
         default: PB_PAIRS32(CAT_ANY); break;
         }
-#undef PB_PAIRS32
     }
-    k_batch_pairs64<STRAT><<<persistent_blocks_of(k_batch_pairs64<STRAT>, blocks_per_sm), 128, 0, H->stream>>>(
-        discs, starts, slot_disc, ndisc, s0, m, P, O, ctr + 1);
+    switch (cat64) {
+    case CAT_GDC4: PB_PAIRS64(CAT_GDC4); break;
+    case CAT_C4: PB_PAIRS64(CAT_C4); break;
+    case CAT_S1: PB_PAIRS64(CAT_S1); break;
+    case CAT_SG1: PB_PAIRS64(CAT_SG1); break;
+    default: PB_PAIRS64(CAT_ANY); break;
+    }
+#undef PB_PAIRS32
+#undef PB_PAIRS64
     k_batch_over<STRAT, KT><<<persistent_blocks_of(k_batch_over<STRAT, KT>, blocks_per_sm), 128, 0, H->stream>>>(
         discs, starts, slot_disc, ndisc, s0, m, P, O, fp64_only, light_max, leaf_size, ctr + 2);
 }
@@ -389,13 +398,13 @@ static cudaError_t launch_walk_batch(Handle *H, const BatchDisc *discs, const in
 }
 
 template <int STRAT>
-static void launch_slice_strat(Handle *H, int kernel, int cat, const BatchDisc *discs, const int64_t *starts,
+static void launch_slice_strat(Handle *H, int kernel, int cat, int cat64, const BatchDisc *discs, const int64_t *starts,
                                const uint32_t *slot_disc, int ndisc, int64_t s0, int64_t m, const RunPool &P,
                                const SliceOrder &O, int fp64_only, unsigned light_max, int leaf_size,
                                int blocks_per_sm, unsigned long long *ctr)
 {
 #define PB_SLICE(KT)                                                                                               \
-    launch_slice_pairs<STRAT, KT>(H, cat, discs, starts, slot_disc, ndisc, s0, m, P, O, fp64_only, light_max,       \
+    launch_slice_pairs<STRAT, KT>(H, cat, cat64, discs, starts, slot_disc, ndisc, s0, m, P, O, fp64_only, light_max,       \
                                   leaf_size, blocks_per_sm, ctr)
     switch (kernel) {
     case 0: PB_SLICE(0); break;
@@ -413,7 +422,7 @@ static void launch_slice_strat(Handle *H, int kernel, int cat, const BatchDisc *
 // counted on the device), then the sums.  slot_of holds m ints.
 // ctr: [0..2] persistent pair-kernel counters, [3..4] pair split sums, [5] heavy count (low
 // word), [6] walk queue.
-cudaError_t launch_batch_slice(Handle *H, int strategy, int kernel, int cat, const BatchDisc *discs,
+cudaError_t launch_batch_slice(Handle *H, int strategy, int kernel, int cat, int cat64, const BatchDisc *discs,
                                const int64_t *starts, const uint32_t *slot_disc, int ndisc, int64_t s0, int64_t m,
                                const RunPool &P, int fp64_only, unsigned light_max, int leaf_size, int blocks_per_sm,
                                int *slot_of, unsigned long long *ctr)
@@ -454,15 +463,15 @@ cudaError_t launch_batch_slice(Handle *H, int strategy, int kernel, int cat, con
     SliceOrder O{ord, slot_of, nheavy, P.n_deferred};
     switch (strategy) {
     case GATHER:
-        launch_slice_strat<GATHER>(H, kernel, cat, discs, starts, slot_disc, ndisc, s0, m, P, O, fp64_only, light_max,
+        launch_slice_strat<GATHER>(H, kernel, cat, cat64, discs, starts, slot_disc, ndisc, s0, m, P, O, fp64_only, light_max,
                                    leaf_size, blocks_per_sm, ctr);
         break;
     case SCATTER:
-        launch_slice_strat<SCATTER>(H, kernel, cat, discs, starts, slot_disc, ndisc, s0, m, P, O, fp64_only, light_max,
+        launch_slice_strat<SCATTER>(H, kernel, cat, cat64, discs, starts, slot_disc, ndisc, s0, m, P, O, fp64_only, light_max,
                                     leaf_size, blocks_per_sm, ctr);
         break;
     default:
-        launch_slice_strat<SYMMETRIC>(H, kernel, cat, discs, starts, slot_disc, ndisc, s0, m, P, O, fp64_only,
+        launch_slice_strat<SYMMETRIC>(H, kernel, cat, cat64, discs, starts, slot_disc, ndisc, s0, m, P, O, fp64_only,
                                       light_max, leaf_size, blocks_per_sm, ctr);
         break;
     }
@@ -470,8 +479,8 @@ cudaError_t launch_batch_slice(Handle *H, int strategy, int kernel, int cat, con
     return cudaGetLastError();
 }
 
-// compile-time catalog shape of the batch's FP32C pair kernel (the host-side view of the catalog)
-int batch_catalog_shape(const DevCatalog &C32) { return catalog_shape(C32); }
+// compile-time catalog shape of the batch's pair kernels (the host-side view of a catalog)
+int batch_catalog_shape(const DevCatalog &C) { return catalog_shape(C); }
 
 // the FP32-compensated payload of one disc (the single-disc launchers build it the same way)
 cudaError_t launch_batch_payload(Handle *H, const DevTree &T, const DevCatalog &C, float4 **pay, int *stride)

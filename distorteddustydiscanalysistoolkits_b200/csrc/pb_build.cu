@@ -465,16 +465,20 @@ cudaError_t launch_dedupe(Handle *H, uint64_t *codes, int64_t n)
 // permuted leaves and particle columns
 __global__ void k_gather(int64_t n, const uint32_t *__restrict__ idx, const double *__restrict__ x,
                          const double *__restrict__ y, const double *__restrict__ z, const double *__restrict__ h,
-                         const double *__restrict__ m, const double *__restrict__ rho, double4 *leaf, double *ms,
-                         double *rhos)
+                         const double *__restrict__ m, const double *__restrict__ rho, double4 *leaf, double4 *aux,
+                         double *rhos, int *odd)
 {
+    bool bad = false;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         uint32_t o = idx[i];
         if (o >= (uint64_t)n) o = 0;   // unreachable for a valid permutation; keeps reads in bounds
-        leaf[i] = make_double4(x[o], y[o], z[o], h[o]);
-        ms[i] = m[o];
-        rhos[i] = rho[o];
+        const double ho = h[o], ro = rho[o];
+        leaf[i] = make_double4(x[o], y[o], z[o], ho);
+        aux[i] = make_double4(1.0 / ho, 1.0 / ro, m[o], ro);
+        rhos[i] = ro;
+        bad |= !aux_regular(ho, ro);
     }
+    if (bad) atomicOr(odd, 1);
 }
 
 __global__ void k_gather_col(int64_t n, const uint32_t *__restrict__ idx, const double *__restrict__ src, double *dst)
@@ -490,7 +494,7 @@ cudaError_t launch_gather(Handle *H, int64_t n, const double *x, const double *y
 {
     const uint32_t *idx = H->idx.as<uint32_t>();
     k_gather<<<grid_for(n, 256), 256, 0, H->stream>>>(n, idx, x, y, z, h, m, rho, H->leaf.as<double4>(),
-                                                       H->m_s.as<double>(), H->rho_s.as<double>());
+                                                       H->leaf_aux.as<double4>(), H->rho_s.as<double>(), H->odd.as<int>());
     H->launches += 1;
     for (size_t c = 0; c < cols.size(); ++c) {
         k_gather_col<<<grid_for(n, 256), 256, 0, H->stream>>>(n, idx, cols[c], H->cols_s[c].as<double>());

@@ -21,8 +21,8 @@ using namespace pb;
 pb::Handle::~Handle()
 {
     DBuf *all[] = {&in_x, &in_y, &in_z, &in_h, &in_m, &in_rho, &codes, &codes_alt, &idx, &idx_alt, &scan_tmp,
-                   &scan_part, &hist, &bbox_part, &qparams, &status, &leaf, &leaf_escape, &node, &node_hmax, &node_child, &node_range, &payload, &counter, &left,
-                   &right, &escape, &parent, &bmin64, &bmax64, &hmax64, &counters, &m_s, &rho_s, &col_ptrs,
+                   &scan_part, &hist, &bbox_part, &qparams, &status, &leaf, &leaf_aux, &odd, &leaf_escape, &node, &node_hmax, &node_child, &node_range, &payload, &counter, &left,
+                   &right, &escape, &parent, &bmin64, &bmax64, &hmax64, &counters, &rho_s, &col_ptrs,
                    &q_x, &q_y, &q_z, &q_keys, &q_keys_alt, &q_perm, &q_perm_alt, &q_out, &q_aux,
                    &pool_runs, &pool_next, &pool_ctr, &items, &wbnear, &qacc, &qflag, &cut, &defer_a, &defer_b,
                    &lpt_k, &lpt_v, &lpt_ka, &lpt_va, &iota, &grid_ax, &grid_out, &wl_cnt, &wl_off, &wl_s, &wl_j, &wl_sa, &wl_ja, &mlp_w, &mlp_m, &mlp_v, &mlp_g, &mlp_norm,
@@ -32,6 +32,9 @@ pb::Handle::~Handle()
     batch_starts.release();
     batch_slots.release();
     batch_ctr.release();
+    for (DBuf *b : {&batch_slot_of, &batch_bcnt, &batch_boff, &batch_bcur, &batch_list, &batch_mk, &batch_mka, &batch_mv,
+                    &batch_mva})
+        b->release();
     if (batch_host) cudaFreeHost(batch_host);
     for (auto &b : in_cols) b.release();
     for (auto &b : cols_s) b.release();
@@ -115,9 +118,9 @@ DevTree make_tree(Handle &H)
     T.node = H.node.as<NodeF>();
     T.node_hmax = H.node_hmax.as<float>();
     T.child = H.node_child.as<int2>();
+    T.aux = H.leaf_aux.as<double4>();
+    T.odd = H.odd.as<int>();
     T.range = H.node_range.as<int2>();
-    T.m = H.m_s.as<double>();
-    T.rho = H.rho_s.as<double>();
     T.kernel = H.kernel;
     T.status = H.status.as<int>();
     return T;
@@ -412,6 +415,8 @@ int do_build(Handle &H, const pb_input *in, int32_t flags)
     CK(H.idx.reserve(4 * n));
     CK(H.idx_alt.reserve(4 * n));
     CK(H.leaf.reserve(32 * n));
+    CK(H.leaf_aux.reserve(32 * n));
+    CK(H.odd.reserve(sizeof(int)));
     CK(H.leaf_escape.reserve(4 * n));
     CK(H.node.reserve(sizeof(NodeF) * nin));
     CK(H.node_hmax.reserve(4 * nin));
@@ -425,11 +430,11 @@ int do_build(Handle &H, const pb_input *in, int32_t flags)
     CK(H.bmax64.reserve(24 * nin));
     CK(H.hmax64.reserve(8 * nin));
     CK(H.counters.reserve(4 * nin));
-    CK(H.m_s.reserve(nb));
     CK(H.rho_s.reserve(nb));
     CK(H.qparams.reserve(sizeof(QuantParams)));
     CK(H.status.reserve(sizeof(int)));
     CK(cudaMemsetAsync(H.status.p, 0, sizeof(int), H.stream));
+    CK(cudaMemsetAsync(H.odd.p, 0, sizeof(int), H.stream));
     ev_record(H, 0);
     CK(launch_bbox(&H, n, (const double *)x, (const double *)y, (const double *)z, (const double *)h));
     CK(launch_encode(&H, n, (const double *)x, (const double *)y, (const double *)z));
@@ -607,6 +612,11 @@ bool grow_pool(Handle &H)
     return true;
 }
 
+// A query of more accepted leaves than an even share of the launch's FP64 pairs over the resident
+// warps (148 x 28), and of at least BLOCK64_MIN, is summed by a whole block: one warp would still be
+// at it when the others have finished.
+constexpr int64_t BLOCK64_SHARE = 4096, BLOCK64_MIN = 8192;
+
 // FP32-compensated points in two phases: the walk kernels write every (query, subtree) item's
 // accepted runs, the pair kernel evaluates them (once per catalog launch).  Queries go through
 // in slices of H.slice (Morton order when sorted), which bounds the item and pool memory.
@@ -710,7 +720,12 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
             H.interp_launches++;
             uint32_t *order = nullptr;
             int64_t m_heavy = 0;
-            CK(launch_split_order(&H, P, m, (unsigned)H.light_max, mode == 0, &order, &m_heavy, ctr + 4));
+            int64_t light_pairs = 0;
+            CK(launch_split_order(&H, P, m, (unsigned)H.light_max, mode == 0, &order, &m_heavy, &light_pairs, ctr + 4));
+            // the plain order is not sorted: no block queries there
+            const unsigned block_min =
+                mode == 0 ? 0xffffffffu
+                          : (unsigned)std::min<int64_t>(std::max(light_pairs / BLOCK64_SHARE, BLOCK64_MIN), 0x7fffffff);
             ev_record(H, 6);
             if (m_heavy > 0)
                 for (const Launch &Lc : launches) {
@@ -721,7 +736,7 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
             if (m_heavy < m)
                 for (const Launch &Lc : launches64) {   // light queries: FP64, the reference's arithmetic
                     DevCatalog C = dev_catalog(H, Lc, dev.data());
-                    CK(launch_pairs_fp64(&H, T, C, strategy, P, m - m_heavy, ql, order + m_heavy, dx, dy, dz));
+                    CK(launch_pairs_fp64(&H, T, C, strategy, P, m - m_heavy, block_min, ql, order + m_heavy, dx, dy, dz));
                     H.interp_launches++;
                 }
             ev_record(H, 7);
@@ -1552,7 +1567,7 @@ int32_t pb_batch_points(pb_handle *const *discs, int32_t ndiscs, const pb_catalo
         }
         hd[k] = D;
     }
-    const int cat_shape = batch_catalog_shape(hd[0].C32);
+    const int cat_shape = batch_catalog_shape(hd[0].C32), cat_shape64 = batch_catalog_shape(hd[0].C64);
     CK(cudaMemcpyAsync(H.batch_desc.p, H.batch_host, desc_bytes, cudaMemcpyHostToDevice, H.stream));
     CK(cudaMemcpyAsync(H.batch_starts.p, hs, start_bytes, cudaMemcpyHostToDevice, H.stream));
     CK(cudaMemcpyAsync(H.batch_slots.p, ho, slot_bytes, cudaMemcpyHostToDevice, H.stream));
@@ -1590,7 +1605,7 @@ int32_t pb_batch_points(pb_handle *const *discs, int32_t ndiscs, const pb_catalo
             CK(cudaMemsetAsync(ctr, 0, 16, H.stream));
             CK(cudaMemsetAsync(P.qacc, 0, sizeof(unsigned) * m, H.stream));
             CK(cudaMemsetAsync(P.qflag, 0, sizeof(int) * m, H.stream));
-            CK(launch_batch_slice(&H, strategy, H.kernel, cat_shape, H.batch_desc.as<BatchDisc>(),
+            CK(launch_batch_slice(&H, strategy, H.kernel, cat_shape, cat_shape64, H.batch_desc.as<BatchDisc>(),
                                   H.batch_starts.as<int64_t>(), H.batch_slots.as<uint32_t>(), ndiscs, s0, m, P,
                                   precision == PB_FP64 ? 1 : 0, (unsigned)H.light_max, H.leaf_size, H.batch_blocks,
                                   H.batch_slot_of.as<int>(), H.batch_ctr.as<unsigned long long>()));

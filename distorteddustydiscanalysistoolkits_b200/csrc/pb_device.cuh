@@ -7,7 +7,8 @@
 //   node[n-1]      NodeF {lo.xyz, left | hi.xyz, escape}, 32 bytes, FP32 boxes rounded
 //                  outward so every pruning test is conservative against the FP64 tree
 //   node_hmax[n-1] float, max smoothing length of the subtree, rounded up
-//   m, rho, quant  FP64 particle columns in sorted order
+//   aux[n]         double4 {1/h, 1/rho, m, rho}, read by the pair and line kernels
+//   quant          FP64 particle columns in sorted order
 // Unified ids follow the reference (BinaryRadixTree.jl:36-51): internal 1..n-1,
 // leaf n..2n-1, 0 = none.
 #pragma once
@@ -50,9 +51,9 @@ struct DevTree {
     const NodeF *node;
     const float *node_hmax;
     const int2 *child;      // (left, right) unified ids of each internal node
+    const double4 *aux;     // {1/h, 1/rho, m, rho} of each sorted particle (reciprocals correctly rounded)
+    const int *odd;         // nonzero: some particle's h or rho is outside aux_regular's range
     const int2 *range;      // 0-based sorted leaf range [lo, hi] of each internal node's subtree
-    const double *m;
-    const double *rho;
     int kernel;
     int *status;
 };
@@ -103,13 +104,23 @@ struct DevCatalog {
     double *out[MAXL];
 };
 
-// read-only 32-byte leaf record as two 16-byte loads
+// read-only 32-byte record (32-byte aligned) in one 256-bit load: half the requests of two
+// 16-byte loads, and a warp reading consecutive records takes 8 L1 wavefronts instead of 16
 __device__ __forceinline__ double4 ldg4(const double4 *p)
 {
-    const double2 *q = reinterpret_cast<const double2 *>(p);
-    double2 a = __ldg(q), b = __ldg(q + 1);
-    return make_double4(a.x, a.y, b.x, b.y);
+    double4 r;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    return r;
 }
+
+// |x| in [2^-250, 2^250): products of a few such numbers and of their reciprocals stay normal
+__device__ __forceinline__ bool exp_safe(double x)
+{
+    return (unsigned)((__double2hiint(x) & 0x7ff00000) - ((1023 - 250) << 20)) < (unsigned)(500 << 20);
+}
+
+// the particles the pair kernels take their short forms for (DevTree::odd is 0 if all are)
+__device__ __forceinline__ bool aux_regular(double h, double rho) { return h > 0.0 && exp_safe(h) && exp_safe(rho); }
 
 __host__ __device__ inline double kernel_valid(int k) { return k == 1 ? 2.5 : (k == 2 ? 3.0 : 2.0); }
 
@@ -355,20 +366,5 @@ __device__ __forceinline__ void gradW(int k, R dx, R dy, R dz, R r, R h, R &gx, 
     gy = inv_hDp1 * cy;
     gz = inv_hDp1 * cz;
 }
-
-// error-free transformation accumulator (Knuth TwoSum with a running compensation term)
-struct CSum {
-    float s, c;
-    __device__ __forceinline__ void zero() { s = 0.f; c = 0.f; }
-    __device__ __forceinline__ void add(float x)
-    {
-        float t = __fadd_rn(s, x);
-        float bp = __fsub_rn(t, s);
-        float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bp)), __fsub_rn(x, bp));
-        s = t;
-        c = __fadd_rn(c, e);
-    }
-    __device__ __forceinline__ double val() const { return (double)s + (double)c; }
-};
 
 }  // namespace pb

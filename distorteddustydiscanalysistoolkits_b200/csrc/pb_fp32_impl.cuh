@@ -96,57 +96,18 @@ __device__ __forceinline__ const float4 *rec_of(const float4 *pay, int stride, u
     return pay + (uint64_t)(b >> 5) * (uint32_t)(stride * PAY_BLOCK) + (b & (PAY_BLOCK - 1));
 }
 
-// Compile-time shape of a launch's catalog, for the pair kernels.  CAT 0 reads everything from
-// the DevCatalog at run time; 1: four columns, gradient + divergence + curl; 2: four columns,
-// curl only; 3: one column, scalars only.  A specialised kernel performs exactly the
-// operations, in the same order, that the generic one performs for such a catalog.
-constexpr int CAT_ANY = 0, CAT_GDC4 = 1, CAT_C4 = 2, CAT_S1 = 3, CAT_SG1 = 4;   // SG1: one column, scalar + gradient
-
-template <int CAT>
-struct CatShape {
-    __device__ static __forceinline__ int nu(const DevCatalog &C)
-    {
-        return (CAT == CAT_GDC4 || CAT == CAT_C4) ? 4 : ((CAT == CAT_S1 || CAT == CAT_SG1) ? 1 : C.nU);
-    }
-    __device__ static __forceinline__ bool grad(const DevCatalog &C)
-    {
-        return (CAT == CAT_GDC4 || CAT == CAT_SG1) ? true : (CAT == CAT_ANY ? C.n_grad > 0 : false);
-    }
-    __device__ static __forceinline__ bool div(const DevCatalog &C)
-    {
-        return CAT == CAT_GDC4 ? true : (CAT == CAT_ANY ? C.n_div > 0 : false);
-    }
-    __device__ static __forceinline__ bool curl(const DevCatalog &C)
-    {
-        return (CAT == CAT_GDC4 || CAT == CAT_C4) ? true : (CAT == CAT_ANY ? C.n_curl > 0 : false);
-    }
-    __device__ static __forceinline__ bool any(const DevCatalog &C) { return grad(C) || div(C) || curl(C); }
-    __device__ static __forceinline__ int stride(int s)
-    {
-        return (CAT == CAT_GDC4 || CAT == CAT_C4) ? 4 : ((CAT == CAT_S1 || CAT == CAT_SG1) ? 3 : s);
-    }
-};
-
-inline int catalog_shape(const DevCatalog &C)
-{
-    if (C.nU == 4 && C.n_grad == 1 && C.g_u[0] == 0 && C.n_div == 1 && C.n_curl == 1) return CAT_GDC4;
-    if (C.nU == 4 && C.n_grad == 0 && C.n_div == 0 && C.n_curl == 1) return CAT_C4;
-    if (C.nU == 1 && C.n_grad == 0 && C.n_div == 0 && C.n_curl == 0) return CAT_S1;
-    if (C.nU == 1 && C.n_grad == 1 && C.g_u[0] == 0 && C.n_div == 0 && C.n_curl == 0) return CAT_SG1;
-    return CAT_ANY;
-}
-
 // internal linkage: each unit that includes this header gets its own copy of the kernel
 static __global__ void k_payload(int64_t n, DevTree T, DevCatalog C, float4 *pay, int stride)
 {
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < n; b += (int64_t)gridDim.x * blockDim.x) {
         double4 L = T.leaf[b];
-        double ih = 1.0 / L.w;
+        const double4 X = T.aux[b];
+        double ih = X.x;
         float xh = (float)L.x, yh = (float)L.y, zh = (float)L.z;
         float4 *rec = const_cast<float4 *>(rec_of(pay, stride, (uint32_t)b));
         rec[0] = make_float4(xh, yh, zh, (float)ih);
         rec[PAY_BLOCK] = make_float4((float)(L.x - (double)xh), (float)(L.y - (double)yh), (float)(L.z - (double)zh),
-                                     (float)(T.m[b] / T.rho[b]));
+                                     (float)(X.z / X.w));
         float v[2 * MAXU + 4];
 #pragma unroll
         for (int u = 0; u < MAXU; ++u) {

@@ -80,12 +80,12 @@ struct Handle {
     std::vector<DBuf> in_cols;
     DBuf codes, codes_alt, idx, idx_alt, scan_tmp, scan_part, hist;
     DBuf bbox_part, qparams, status;
-    DBuf leaf, leaf_escape, node, node_hmax, node_child, node_range;
+    DBuf leaf, leaf_aux, odd, leaf_escape, node, node_hmax, node_child, node_range;
     DBuf payload;       // per-call FP32 particle payload of the FP32-compensated path
     DBuf counter;       // work-queue counter of the warp-per-query kernels
     DBuf left, right, escape, parent;
     DBuf bmin64, bmax64, hmax64, counters;
-    DBuf m_s, rho_s;
+    DBuf rho_s;
     std::vector<DBuf> cols_s;
     DBuf col_ptrs;      // device array of sorted column pointers
 
@@ -175,11 +175,11 @@ cudaError_t launch_walk_list(Handle *H, const DevTree &T, int strategy, const Ru
                              unsigned long long *counter);
 cudaError_t launch_lpt_order(Handle *H, const RunPool &P, int64_t m, uint32_t **order);
 cudaError_t launch_split_order(Handle *H, const RunPool &P, int64_t m, unsigned light_max, bool plain,
-                               uint32_t **order, int64_t *m_heavy, unsigned long long *pairs);
+                               uint32_t **order, int64_t *m_heavy, int64_t *light_pairs, unsigned long long *pairs);
 cudaError_t launch_iota(Handle *H, int64_t m, uint32_t *out);
 cudaError_t launch_count_heavy(Handle *H, const RunPool &P, int64_t m, unsigned light_max, unsigned *count,
                                unsigned long long *pairs);
-int batch_catalog_shape(const DevCatalog &C32);
+int batch_catalog_shape(const DevCatalog &C);
 
 // ---- launchers (pb_sched.cu) ----
 cudaError_t launch_sched_features(Handle *H, const DevTree &T, int64_t m, const uint32_t *ql, const double *qx,
@@ -201,9 +201,11 @@ cudaError_t launch_pairs_fp32(Handle *H, const DevTree &T, const DevCatalog &C, 
 cudaError_t launch_points_fp64(Handle *H, const DevTree &T, const DevCatalog &C, int strategy, int64_t nq,
                                const double *qx, const double *qy, const double *qz, const uint32_t *perm,
                                int64_t npts);
+// queries of more than block_min accepted leaves (the first of the order, sorted by descending
+// count) are taken by whole blocks; 0xffffffff: none
 cudaError_t launch_pairs_fp64(Handle *H, const DevTree &T, const DevCatalog &C, int strategy, const RunPool &P,
-                              int64_t m, const uint32_t *ql, const uint32_t *order, const double *qx,
-                              const double *qy, const double *qz);
+                              int64_t m, unsigned block_min, const uint32_t *ql, const uint32_t *order,
+                              const double *qx, const double *qy, const double *qz);
 cudaError_t launch_points_fp32(Handle *H, const DevTree &T, const DevCatalog &C, int strategy, int64_t nq,
                                const double *qx, const double *qy, const double *qz, const uint32_t *perm,
                                int64_t npts);
@@ -223,7 +225,7 @@ cudaError_t launch_stats(Handle *H, const DevTree &T, int strategy, int64_t nq, 
 struct LineFrame {
     double c[3], e1[3], e2[3], d[3];
 };
-cudaError_t launch_batch_slice(Handle *H, int strategy, int kernel, int cat, const BatchDisc *discs,
+cudaError_t launch_batch_slice(Handle *H, int strategy, int kernel, int cat, int cat64, const BatchDisc *discs,
                                const int64_t *starts, const uint32_t *slot_disc, int ndisc, int64_t s0, int64_t m,
                                const RunPool &P, int fp64_only, unsigned light_max, int leaf_size, int blocks_per_sm,
                                int *slot_of, unsigned long long *ctr);

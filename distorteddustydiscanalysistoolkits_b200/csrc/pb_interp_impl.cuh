@@ -6,7 +6,7 @@
 //
 // Included by pb_interp64.cu (-fmad=false; FP64 terms in the reference's expressions and
 // order, bit-exact with the FP64 oracle), pb_interp32.cu (FP32 per-pair terms with double-float
-// offsets, FP64 accumulation of FP32 chunk sums; the FP32 line kernel uses TwoSum) and
+// offsets, FP64 accumulation of FP32 chunk sums) and
 // pb_walk.cu (the walk kernels).
 //
 // Accepted neighbours are visited in ascending sorted-leaf order (DFS preorder), exactly as
@@ -28,15 +28,54 @@ __device__ __forceinline__ T pick(const T (&a)[N], int i)
     return r;
 }
 
+// Compile-time shape of a launch's catalog, for the pair kernels (FP64 and FP32C).  CAT 0 reads everything from
+// the DevCatalog at run time; 1: four columns, gradient + divergence + curl; 2: four columns,
+// curl only; 3: one column, scalars only.  A specialised kernel performs exactly the
+// operations, in the same order, that the generic one performs for such a catalog.
+constexpr int CAT_ANY = 0, CAT_GDC4 = 1, CAT_C4 = 2, CAT_S1 = 3, CAT_SG1 = 4;   // SG1: one column, scalar + gradient
+
+template <int CAT>
+struct CatShape {
+    __device__ static __forceinline__ int nu(const DevCatalog &C)
+    {
+        return (CAT == CAT_GDC4 || CAT == CAT_C4) ? 4 : ((CAT == CAT_S1 || CAT == CAT_SG1) ? 1 : C.nU);
+    }
+    __device__ static __forceinline__ bool grad(const DevCatalog &C)
+    {
+        return (CAT == CAT_GDC4 || CAT == CAT_SG1) ? true : (CAT == CAT_ANY ? C.n_grad > 0 : false);
+    }
+    __device__ static __forceinline__ bool div(const DevCatalog &C)
+    {
+        return CAT == CAT_GDC4 ? true : (CAT == CAT_ANY ? C.n_div > 0 : false);
+    }
+    __device__ static __forceinline__ bool curl(const DevCatalog &C)
+    {
+        return (CAT == CAT_GDC4 || CAT == CAT_C4) ? true : (CAT == CAT_ANY ? C.n_curl > 0 : false);
+    }
+    __device__ static __forceinline__ bool any(const DevCatalog &C) { return grad(C) || div(C) || curl(C); }
+    __device__ static __forceinline__ int stride(int s)
+    {
+        return (CAT == CAT_GDC4 || CAT == CAT_C4) ? 4 : ((CAT == CAT_S1 || CAT == CAT_SG1) ? 3 : s);
+    }
+};
+
+inline int catalog_shape(const DevCatalog &C)
+{
+    if (C.nU == 4 && C.n_grad == 1 && C.g_u[0] == 0 && C.n_div == 1 && C.n_curl == 1) return CAT_GDC4;
+    if (C.nU == 4 && C.n_grad == 0 && C.n_div == 0 && C.n_curl == 1) return CAT_C4;
+    if (C.nU == 1 && C.n_grad == 0 && C.n_div == 0 && C.n_curl == 0) return CAT_S1;
+    if (C.nU == 1 && C.n_grad == 1 && C.g_u[0] == 0 && C.n_div == 0 && C.n_curl == 0) return CAT_SG1;
+    return CAT_ANY;
+}
+
 __device__ __forceinline__ void flag(int *status, int bit) { atomicOr(status, bit); }
 
 __device__ __forceinline__ NodeF load_node(const NodeF *p)
 {
-    const float4 *q = reinterpret_cast<const float4 *>(p);
-    float4 a = __ldg(q), c = __ldg(q + 1);
-    NodeF nd;
-    nd.lox = a.x; nd.loy = a.y; nd.loz = a.z; nd.left = __float_as_int(a.w);
-    nd.hix = c.x; nd.hiy = c.y; nd.hiz = c.z; nd.escape = __float_as_int(c.w);
+    NodeF nd;   // the 32-byte record in one 256-bit load
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(nd.lox), "=f"(nd.loy), "=f"(nd.loz), "=r"(nd.left), "=f"(nd.hix), "=f"(nd.hiy), "=f"(nd.hiz), "=r"(nd.escape)
+        : "l"(p));
     return nd;
 }
 
@@ -151,82 +190,16 @@ __device__ __forceinline__ int64_t nearest_leaf(const DevTree &T, double px, dou
     return bi;
 }
 
-// Largest squared distance from the point to any point of the (outward-rounded) box,
-// with the rounding sequence of d2_point: every leaf inside has d2_point <= this value.
-__device__ __forceinline__ double far_d2_box(double px, double py, double pz, const NodeF &nd)
-{
-    double ax = fmax(fabs(__dsub_rn(px, (double)nd.lox)), fabs(__dsub_rn(px, (double)nd.hix)));
-    double ay = fmax(fabs(__dsub_rn(py, (double)nd.loy)), fabs(__dsub_rn(py, (double)nd.hiy)));
-    double az = fmax(fabs(__dsub_rn(pz, (double)nd.loz)), fabs(__dsub_rn(pz, (double)nd.hiz)));
-    double s = __dmul_rn(ax, ax);
-    s = __dadd_rn(s, __dmul_rn(ay, ay));
-    s = __dadd_rn(s, __dmul_rn(az, az));
-    return s;
-}
-
-
 // --------------------------------------------------------------------------------------
-// DFS walker of the main pass ("while-while" form): each call advances the stackless
-// left/escape traversal (LinearBVHTraversalMacros.jl:135-371) until the next accepted leaf
-// and returns it, so all lanes of a warp evaluate their pair terms together.  A subtree
-// lying entirely inside the query's radius is turned into a cursor over its contiguous
-// sorted-leaf range, which is exactly the DFS order of its leaves.  The sequence of
-// accepted leaves is therefore the reference's.
+// State of a stackless left/escape traversal (LinearBVHTraversalMacros.jl:135-371).  A subtree
+// lying entirely inside the query's radius is turned into its contiguous sorted-leaf range,
+// which is exactly the DFS order of its leaves, so the sequence of accepted leaves is the
+// reference's.
 struct Walk {
     int node;
     int64_t cur, end, guard, limit;
     int stop = 0;   // node where the walk ends: 0 for the whole tree, a subtree's escape target for a subtree
 };
-
-template <int STRAT>
-__device__ __forceinline__ int64_t next_accepted(const DevTree &T, Walk &w, double px, double py, double pz,
-                                                 double K, double r2a, double4 &L, double &d2)
-{
-    const int64_t n = T.n;
-    for (;;) {
-        if (w.cur <= w.end) {
-            int64_t b = w.cur++;
-            L = ldg4(T.leaf + b);
-            d2 = d2_point(px, py, pz, L);
-            return b;
-        }
-        if (w.node == 0) return -1;
-        if (++w.guard > w.limit) { flag(T.status, ST_TRAVERSAL); w.node = 0; return -1; }
-        const int node = w.node;
-        if (node >= n) {
-            int64_t b = node - n;
-            L = ldg4(T.leaf + b);
-            w.node = __ldg(T.leaf_escape + b);
-            double r2;
-            if (STRAT == GATHER) r2 = r2a;
-            else {
-                double r = __dmul_rn(K, L.w);
-                double rr = __dmul_rn(r, r);
-                r2 = STRAT == SCATTER ? rr : (r2a > rr ? r2a : rr);
-            }
-            d2 = d2_point(px, py, pz, L);
-            if (d2 <= r2) return b;
-            continue;
-        }
-        NodeF nd = load_node(T.node + (node - 1));
-        double r2;
-        if (STRAT == GATHER) r2 = r2a;
-        else {
-            double r = __dmul_rn(K, (double)__ldg(T.node_hmax + (node - 1)));
-            double rr = __dmul_rn(r, r);
-            r2 = STRAT == SCATTER ? rr : (r2a > rr ? r2a : rr);
-        }
-        if (d2_box(px, py, pz, nd) > r2) { w.node = nd.escape; continue; }
-        if (STRAT != SCATTER && far_d2_box(px, py, pz, nd) <= r2a) {
-            int2 rg = __ldg(T.range + (node - 1));
-            w.cur = rg.x;
-            w.end = rg.y;
-            w.node = nd.escape;
-            continue;
-        }
-        w.node = nd.left;
-    }
-}
 
 // The walk's pruning decision for internal node `node` (box `nd`): FP32 box distance with
 // directed rounding against the node radius (query radius and/or K * hmax) with the 2^-20
@@ -420,17 +393,64 @@ __device__ __forceinline__ int64_t next_query(unsigned long long *counter, int l
 }
 
 // --------------------------------------------------------------------------------------
+// One chunk of up to 32 runs of an item, one run per lane (lanes past the last run hold an
+// empty one), with the inclusive prefix sums of the run lengths: leaf position t of the chunk,
+// 0 <= t < tot, lies in the first run r with inc[r] > t.  Leaf indices and counts are 32-bit
+// (n <= 2^30; an item's accepted leaves lie in one subtree).
+struct RunWindow {
+    int lo, inc, ex, tot;          // this lane's run: first leaf, inclusive and exclusive prefix
+    int r0 = -1, end0 = 0;         // run of the last position looked up, and where it ends
+    int lo0 = 0, ex0 = 0;
+
+    __device__ __forceinline__ RunWindow(const RunPool &P, int c, int cnt, int lane)
+    {
+        const uint2 rn = lane < cnt ? __ldg(P.runs + (int64_t)c * RUN_CHUNK + lane) : make_uint2(0u, 0u);
+        lo = (int)rn.x;
+        inc = (int)rn.y;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            int v = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += v;
+        }
+        tot = __shfl_sync(0xffffffffu, inc, 31);
+        ex = inc - (int)rn.y;
+    }
+    // makes r0 the run of position t (t >= the previous one); warp-uniform
+    __device__ __forceinline__ void seek(int t)
+    {
+        if (end0 > t) return;
+        r0 = __popc(__ballot_sync(0xffffffffu, inc <= t));   // prefix sums ascend: runs that end before t
+        end0 = __shfl_sync(0xffffffffu, inc, r0);
+        lo0 = __shfl_sync(0xffffffffu, lo, r0);
+        ex0 = __shfl_sync(0xffffffffu, ex, r0);
+    }
+    // the leaf of position tb + lane into `mine`, on the lanes whose position lies in this chunk;
+    // r0 is the run of position max(tb, 0)
+    __device__ __forceinline__ void leaf_of(int tb, int lane, int &mine) const
+    {
+        const int tl = tb + lane;
+        if (tb >= 0 && tb + 32 <= end0) {
+            mine = lo0 + (tl - ex0);
+            return;
+        }
+        // batch positions (after its first one in this chunk) at which a run starts: a lane's run
+        // is r0 plus the starts up to its position
+        const int first = tb < 0 ? -tb : 0, s = ex - tb;
+        const unsigned starts = __reduce_or_sync(0xffffffffu, s > first && s < 32 && inc > ex ? 1u << s : 0u);
+        const int r = r0 + __popc(starts & (0xffffffffu >> (31 - lane)));
+        const int l = __shfl_sync(0xffffffffu, lo, r), e = __shfl_sync(0xffffffffu, ex, r);
+        if (tl >= 0 && tl < tot) mine = l + (tl - e);
+    }
+};
+
 // Dealing of a walked query's accepted leaves (its items in subtree order, the runs of each
 // item chunk by chunk) to the 32 lanes in DFS order: the k-th accepted leaf goes to lane
 // k mod 32.  first(b) is called with the first leaf of every non-empty item (the callee uses
 // the very first one); one(mine) for every full batch (every lane holds a leaf); two(m1) for
 // two consecutive full batches inside one run (lane leaves m1 and m1 + 32) when cantwo()
 // allows it, and four(m1) for four of them (m1, m1 + 32, m1 + 64, m1 + 96) when canfour()
-// does.  Within a chunk, lane l finds the run holding its leaf through a uniform run cursor,
-// or a binary search over the inclusive prefix sums of the run lengths held one per lane
-// when a batch spans several runs.  Leaf indices are 32-bit (n <= 2^30), and so is every
-// count: an item's accepted leaves lie in one subtree.  Returns the fill of the last,
-// partial batch, whose leaves are left in `mine` (-1 on empty lanes).
+// does.  Returns the fill of the last, partial batch, whose leaves are left in `mine` (-1 on
+// empty lanes).
 template <typename FIRST, typename ONE, typename TWO, typename CANTWO, typename FOUR, typename CANFOUR>
 __device__ __forceinline__ int deal_runs(const RunPool &P, int64_t j, int lane, FIRST &first, ONE &one, TWO &two,
                                          CANTWO &cantwo, FOUR &four, CANFOUR &canfour, int &mine)
@@ -449,36 +469,15 @@ __device__ __forceinline__ int deal_runs(const RunPool &P, int64_t j, int lane, 
             first((int)__ldg(&P.runs[(int64_t)c * RUN_CHUNK].x));
             while (left > 0) {
                 const int cnt = left < RUN_CHUNK ? left : RUN_CHUNK;
-                const uint2 rn = lane < cnt ? __ldg(P.runs + (int64_t)c * RUN_CHUNK + lane) : make_uint2(0u, 0u);
                 const int nextc = left > RUN_CHUNK ? __ldg(P.next + c) : -1;
-                int inc = (int)rn.y;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    int v = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += v;
-                }
-                const int tot = __shfl_sync(0xffffffffu, inc, 31);
-                const int ex_own = inc - (int)rn.y;
+                RunWindow R(P, c, cnt, lane);
                 int tb = -fill;
-                // uniform cursor: run r0 holds leaf position max(tb, 0) of the chunk; a batch
-                // inside one run needs no search
-                int r0 = -1, rc = -1;
-                int end0 = 0, lo0 = 0, ex0 = 0;
                 for (;;) {
                     // t0 < tot = inc[cnt - 1], so the cursor stops at a run of this chunk
-                    const int t0 = tb <= 0 ? 0 : (tb < tot ? tb : tot - 1);
-                    while (end0 <= t0 && r0 < 31) {
-                        ++r0;
-                        end0 = __shfl_sync(0xffffffffu, inc, r0);
-                    }
-                    if (tb >= 0 && tb + 64 <= end0) {
-                        if (rc != r0) {
-                            lo0 = __shfl_sync(0xffffffffu, (int)rn.x, r0);
-                            ex0 = __shfl_sync(0xffffffffu, ex_own, r0);
-                            rc = r0;
-                        }
-                        const int m1 = lo0 + (tb - ex0) + lane;
-                        if (tb + 128 <= end0 && canfour()) {   // four full batches inside one run
+                    R.seek(tb <= 0 ? 0 : (tb < R.tot ? tb : R.tot - 1));
+                    if (tb >= 0 && tb + 64 <= R.end0) {
+                        const int m1 = R.lo0 + (tb - R.ex0) + lane;
+                        if (tb + 128 <= R.end0 && canfour()) {   // four full batches inside one run
                             four(m1);
                             tb += 128;
                             continue;
@@ -489,33 +488,13 @@ __device__ __forceinline__ int deal_runs(const RunPool &P, int64_t j, int lane, 
                             continue;   // the next pass assigns or closes what is left of the chunk
                         }
                     }
-                    if (tb >= 0 && tb + 32 <= end0) {
-                        if (rc != r0) {
-                            lo0 = __shfl_sync(0xffffffffu, (int)rn.x, r0);
-                            ex0 = __shfl_sync(0xffffffffu, ex_own, r0);
-                            rc = r0;
-                        }
-                        mine = lo0 + (tb - ex0) + lane;
-                    } else {
-                        const int tl = tb + lane;
-                        const bool here = tl >= 0 && tl < tot;
-                        const int tt = here ? tl : 0;
-                        int r = 0;
-#pragma unroll
-                        for (int sh = 16; sh > 0; sh >>= 1) {
-                            int v = __shfl_sync(0xffffffffu, inc, r + sh - 1);
-                            if (v <= tt) r += sh;
-                        }
-                        const int lo = __shfl_sync(0xffffffffu, (int)rn.x, r);
-                        const int ex = __shfl_sync(0xffffffffu, ex_own, r);
-                        if (here) mine = lo + (tt - ex);
-                    }
-                    if (tb + 31 < tot) {
+                    R.leaf_of(tb, lane, mine);
+                    if (tb + 31 < R.tot) {
                         one(mine);   // full batch
                         mine = -1;
                         tb += 32;
                     } else {
-                        fill = tot - tb;
+                        fill = R.tot - tb;
                         break;
                     }
                 }
@@ -525,6 +504,52 @@ __device__ __forceinline__ int deal_runs(const RunPool &P, int64_t j, int lane, 
         }
     }
     return fill;
+}
+
+// The same dealing for one of W warps that share a query: warp w gets the batches b with
+// b mod W == w; one(mine) for every full one.  Returns the fill of the last, partial batch
+// if it is this warp's (its leaves in `mine`), else 0.
+template <int W, typename ONE>
+__device__ __forceinline__ int deal_runs_part(const RunPool &P, int64_t j, int lane, int w, ONE &one, int &mine)
+{
+    const int ns = P.ns;
+    int fill = 0, turn = 0;   // turn: the current batch's number mod W
+    mine = -1;
+    for (int s0 = 0; s0 < ns; s0 += 32) {
+        const int2 itm = s0 + lane < ns ? __ldg(P.items + j * ns + s0 + lane) : make_int2(-1, 0);
+        unsigned nonempty = __ballot_sync(0xffffffffu, itm.y > 0);
+        while (nonempty) {
+            const int l = __ffs(nonempty) - 1;
+            nonempty &= nonempty - 1;
+            int c = __shfl_sync(0xffffffffu, itm.x, l);
+            int left = __shfl_sync(0xffffffffu, itm.y, l);
+            while (left > 0) {
+                const int cnt = left < RUN_CHUNK ? left : RUN_CHUNK;
+                const int nextc = left > RUN_CHUNK ? __ldg(P.next + c) : -1;
+                RunWindow R(P, c, cnt, lane);
+                int tb = -fill;
+                for (;;) {
+                    if (turn == w && tb < R.tot) {
+                        R.seek(tb < 0 ? 0 : tb);
+                        R.leaf_of(tb, lane, mine);
+                    }
+                    if (tb + 31 >= R.tot) {
+                        fill = R.tot - tb;
+                        break;
+                    }
+                    if (turn == w) {
+                        one(mine);
+                        mine = -1;
+                    }
+                    tb += 32;
+                    turn = turn + 1 == W ? 0 : turn + 1;
+                }
+                left -= cnt;
+                c = nextc;
+            }
+        }
+    }
+    return turn == w ? fill : 0;
 }
 
 // the n == 1 tree has no internal node: its single leaf is tested directly
@@ -540,8 +565,7 @@ __device__ __forceinline__ bool single_leaf_accepted(const DevTree &T, double px
 }
 
 // --------------------------------------------------------------------------------------
-// Exact FP64 accumulator (the reference's arithmetic)
-template <int STRAT>
+// A query's FP64 sums and their finalisation (the reference's arithmetic)
 struct Exact64 {
     double S1;
     double SA[MAXU];
@@ -550,87 +574,6 @@ struct Exact64 {
     double Bd[3], Sd;
     double D[MAXD];
     double Cc[MAXC][3];
-
-    __device__ __forceinline__ void init()
-    {
-        S1 = 0.0;
-#pragma unroll
-        for (int u = 0; u < MAXU; ++u) SA[u] = 0.0;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) { Bq[d] = 0.0; Bd[d] = 0.0; }
-        Sd = 0.0;
-#pragma unroll
-        for (int j = 0; j < MAXG; ++j) Fg[j][0] = Fg[j][1] = Fg[j][2] = 0.0;
-#pragma unroll
-        for (int j = 0; j < MAXD; ++j) D[j] = 0.0;
-#pragma unroll
-        for (int j = 0; j < MAXC; ++j) Cc[j][0] = Cc[j][1] = Cc[j][2] = 0.0;
-    }
-
-    __device__ __forceinline__ void add(const DevTree &T, const DevCatalog &C, bool need_grad, double px, double py,
-                                        double pz, const double4 &L, int64_t b, double d2, double ha, double hb)
-    {
-        const int k = T.kernel;
-        double dx = px - L.x, dy = py - L.y, dz = pz - L.z;
-        double dr = sqrt(d2);
-        double mb = __ldg(T.m + b), rb = __ldg(T.rho + b);
-        double W;
-        if (STRAT == SYMMETRIC) W = 0.5 * (Wfun<double>(k, dr, ha) + Wfun<double>(k, dr, hb));
-        else W = Wfun<double>(k, dr, STRAT == GATHER ? ha : hb);
-        double w = mb * W / rb;
-        S1 += w;
-        double A[MAXU];
-#pragma unroll
-        for (int u = 0; u < MAXU; ++u) {
-            A[u] = (u < C.nU) ? __ldg(C.ucol[u] + b) : 0.0;
-            if (u < C.nU) SA[u] += A[u] * w;
-        }
-        if (!need_grad) return;
-        double gx, gy, gz;
-        if (STRAT == SYMMETRIC) {
-            double ax, ay, az, bx, by, bz;
-            gradW<double>(k, dx, dy, dz, dr, ha, ax, ay, az);
-            gradW<double>(k, dx, dy, dz, dr, hb, bx, by, bz);
-            gx = 0.5 * (ax + bx); gy = 0.5 * (ay + by); gz = 0.5 * (az + bz);
-        } else {
-            gradW<double>(k, dx, dy, dz, dr, STRAT == GATHER ? ha : hb, gx, gy, gz);
-        }
-        double invrb = 1.0 / rb;
-        double ml = mb * invrb;
-        double qx = ml * gx, qy = ml * gy, qz = ml * gz;
-        Bq[0] += qx; Bq[1] += qy; Bq[2] += qz;
-#pragma unroll
-        for (int j = 0; j < MAXG; ++j) {
-            if (j < C.n_grad) {
-                int u = C.g_u[j];
-                if (u < 0) {   // density gradient (gradient_accumulation.jl:160-182)
-                    double mx = mb * gx, my = mb * gy, mz = mb * gz;
-                    Fg[j][0] += mx; Fg[j][1] += my; Fg[j][2] += mz;
-                    Bd[0] += mx * invrb; Bd[1] += my * invrb; Bd[2] += mz * invrb;
-                    Sd += mb * W;
-                } else {
-                    double a = pick<MAXU>(A, u);
-                    Fg[j][0] += qx * a; Fg[j][1] += qy * a; Fg[j][2] += qz * a;
-                }
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < MAXD; ++j) {
-            if (j < C.n_div) {
-                double ax = pick<MAXU>(A, C.d_u[j][0]), ay = pick<MAXU>(A, C.d_u[j][1]), az = pick<MAXU>(A, C.d_u[j][2]);
-                D[j] += qx * ax + qy * ay + qz * az;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < MAXC; ++j) {
-            if (j < C.n_curl) {
-                double ax = pick<MAXU>(A, C.c_u[j][0]), ay = pick<MAXU>(A, C.c_u[j][1]), az = pick<MAXU>(A, C.c_u[j][2]);
-                Cc[j][0] += ay * qz - az * qy;
-                Cc[j][1] += az * qx - ax * qz;
-                Cc[j][2] += ax * qy - ay * qx;
-            }
-        }
-    }
 
     __device__ __forceinline__ void finalize(const DevCatalog &C, int64_t qi) const
     {
@@ -690,305 +633,5 @@ struct Exact64 {
         }
     }
 };
-
-// --------------------------------------------------------------------------------------
-// FP32 compensated accumulator
-template <int STRAT>
-struct Comp32 {
-    CSum S1;
-    CSum SA[MAXU];
-    CSum Bq[3];
-    CSum Fg[MAXG][3];
-    CSum D[MAXD];
-    CSum Cc[MAXC][3];
-    double Ahat[MAXU];
-    bool have;
-
-    __device__ __forceinline__ void init()
-    {
-        S1.zero();
-#pragma unroll
-        for (int u = 0; u < MAXU; ++u) { SA[u].zero(); Ahat[u] = 0.0; }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) Bq[d].zero();
-#pragma unroll
-        for (int j = 0; j < MAXG; ++j) { Fg[j][0].zero(); Fg[j][1].zero(); Fg[j][2].zero(); }
-#pragma unroll
-        for (int j = 0; j < MAXD; ++j) D[j].zero();
-#pragma unroll
-        for (int j = 0; j < MAXC; ++j) { Cc[j][0].zero(); Cc[j][1].zero(); Cc[j][2].zero(); }
-        have = false;
-    }
-
-    __device__ __forceinline__ void add(const DevTree &T, const DevCatalog &C, bool need_grad, double px, double py,
-                                        double pz, const double4 &L, int64_t b, double d2, double ha, double hb)
-    {
-        const int k = T.kernel;
-        float dx = (float)(px - L.x), dy = (float)(py - L.y), dz = (float)(pz - L.z);
-        float dr = sqrtf((float)d2);
-        float mb = (float)__ldg(T.m + b), rb = (float)__ldg(T.rho + b);
-        float fha = (float)ha, fhb = (float)hb;
-        float W;
-        if (STRAT == SYMMETRIC) W = 0.5f * (Wfun<float>(k, dr, fha) + Wfun<float>(k, dr, fhb));
-        else W = Wfun<float>(k, dr, STRAT == GATHER ? fha : fhb);
-        float w = mb * W / rb;
-        S1.add(w);
-        float a[MAXU];
-#pragma unroll
-        for (int u = 0; u < MAXU; ++u) {
-            double A = (u < C.nU) ? __ldg(C.ucol[u] + b) : 0.0;
-            if (!have) Ahat[u] = A;
-            a[u] = (float)(A - Ahat[u]);
-            if (u < C.nU) SA[u].add(a[u] * w);
-        }
-        have = true;
-        if (!need_grad) return;
-        float gx, gy, gz;
-        if (STRAT == SYMMETRIC) {
-            float ax, ay, az, bx, by, bz;
-            gradW<float>(k, dx, dy, dz, dr, fha, ax, ay, az);
-            gradW<float>(k, dx, dy, dz, dr, fhb, bx, by, bz);
-            gx = 0.5f * (ax + bx); gy = 0.5f * (ay + by); gz = 0.5f * (az + bz);
-        } else {
-            gradW<float>(k, dx, dy, dz, dr, STRAT == GATHER ? fha : fhb, gx, gy, gz);
-        }
-        float ml = mb / rb;
-        float qx = ml * gx, qy = ml * gy, qz = ml * gz;
-        Bq[0].add(qx); Bq[1].add(qy); Bq[2].add(qz);
-#pragma unroll
-        for (int j = 0; j < MAXG; ++j) {
-            if (j < C.n_grad) {
-                float av = pick<MAXU>(a, C.g_u[j]);
-                Fg[j][0].add(qx * av); Fg[j][1].add(qy * av); Fg[j][2].add(qz * av);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < MAXD; ++j) {
-            if (j < C.n_div) {
-                float ax = pick<MAXU>(a, C.d_u[j][0]), ay = pick<MAXU>(a, C.d_u[j][1]), az = pick<MAXU>(a, C.d_u[j][2]);
-                D[j].add(qx * ax + qy * ay + qz * az);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < MAXC; ++j) {
-            if (j < C.n_curl) {
-                float ax = pick<MAXU>(a, C.c_u[j][0]), ay = pick<MAXU>(a, C.c_u[j][1]), az = pick<MAXU>(a, C.c_u[j][2]);
-                Cc[j][0].add(ay * qz - az * qy);
-                Cc[j][1].add(az * qx - ax * qz);
-                Cc[j][2].add(ax * qy - ay * qx);
-            }
-        }
-    }
-
-    __device__ __forceinline__ void finalize(const DevCatalog &C, int64_t qi) const
-    {
-        int l = 0;
-        double S = S1.val();
-        if (S == 0.0) {
-            for (int o = 0; o < C.L; ++o) C.out[o][qi] = __longlong_as_double(0x7ff8000000000000LL);
-            return;
-        }
-        double abar[MAXU];
-#pragma unroll
-        for (int u = 0; u < MAXU; ++u) abar[u] = SA[u].val() / S;
-        double B[3] = {Bq[0].val(), Bq[1].val(), Bq[2].val()};
-#pragma unroll
-        for (int j = 0; j < MAXS; ++j) {
-            if (j < C.n_scalar) {
-                int u = C.s_u[j];
-                double ah = pick<MAXU>(Ahat, u);
-                C.out[l++][qi] = C.s_shep[j] ? ah + pick<MAXU>(abar, u) : ah * S + pick<MAXU>(abar, u) * S;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < MAXG; ++j) {
-            if (j < C.n_grad) {
-                double a = pick<MAXU>(abar, C.g_u[j]);
-                C.out[l++][qi] = Fg[j][0].val() - a * B[0];
-                C.out[l++][qi] = Fg[j][1].val() - a * B[1];
-                C.out[l++][qi] = Fg[j][2].val() - a * B[2];
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < MAXD; ++j) {
-            if (j < C.n_div) {
-                double ax = pick<MAXU>(abar, C.d_u[j][0]), ay = pick<MAXU>(abar, C.d_u[j][1]),
-                       az = pick<MAXU>(abar, C.d_u[j][2]);
-                C.out[l++][qi] = D[j].val() - (ax * B[0] + ay * B[1] + az * B[2]);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < MAXC; ++j) {
-            if (j < C.n_curl) {
-                double ax = pick<MAXU>(abar, C.c_u[j][0]), ay = pick<MAXU>(abar, C.c_u[j][1]),
-                       az = pick<MAXU>(abar, C.c_u[j][2]);
-                double bx = ay * B[2] - az * B[1];
-                double by = az * B[0] - ax * B[2];
-                double bz = ax * B[1] - ay * B[0];
-                C.out[l++][qi] = -(Cc[j][0].val() - bx);
-                C.out[l++][qi] = -(Cc[j][1].val() - by);
-                C.out[l++][qi] = -(Cc[j][2].val() - bz);
-            }
-        }
-    }
-};
-
-// --------------------------------------------------------------------------------------
-// point-sample kernel: one thread per (Morton-ordered) sample point
-template <template <int> class ACC, int STRAT>
-__global__ void __launch_bounds__(128) k_points(DevTree T, DevCatalog C, int64_t nq, const double *__restrict__ qx,
-                                                const double *__restrict__ qy, const double *__restrict__ qz,
-                                                const uint32_t *__restrict__ perm)
-{
-    const int64_t n = T.n;
-    const double K = kernel_valid(T.kernel);
-    const bool need_grad = (C.n_grad + C.n_div + C.n_curl) > 0;
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nq; j += (int64_t)gridDim.x * blockDim.x) {
-        int64_t qi = perm ? (int64_t)__ldg(perm + j) : j;
-        if (qi >= nq) continue;   // unreachable for a valid permutation
-        double px = __ldg(qx + qi), py = __ldg(qy + qi), pz = __ldg(qz + qi);
-        double ha = 0.0;
-        if (STRAT != SCATTER) {
-            int64_t b = nearest_leaf(T, px, py, pz);
-            ha = b < 0 ? __longlong_as_double(0x7ff8000000000000LL) : ldg4(T.leaf + b).w;
-        }
-        double ra = __dmul_rn(K, ha);
-        double r2a = __dmul_rn(ra, ra);
-        ACC<STRAT> acc;
-        acc.init();
-        double4 L;
-        double d2;
-        if (T.root == 0) {
-            if (single_leaf_accepted<STRAT>(T, px, py, pz, K, r2a, L, d2))
-                acc.add(T, C, need_grad, px, py, pz, L, 0, d2, ha, L.w);
-        } else {
-            Walk w{T.root, 1, 0, 0, 4 * n + 64};
-            int64_t b;
-            while ((b = next_accepted<STRAT>(T, w, px, py, pz, K, r2a, L, d2)) >= 0)
-                acc.add(T, C, need_grad, px, py, pz, L, b, d2, ha, L.w);
-        }
-        acc.finalize(C, qi);
-    }
-}
-
-// --------------------------------------------------------------------------------------
-// line-sample kernel (itpScatter): one thread per line
-template <typename R>
-__device__ __forceinline__ R line_lut(const R *__restrict__ I, R qmax, R q)
-{
-    const R dq = qmax / R(PB_LINE_NTAB_DEV - 1);
-    R idxf = q / dq + R(1);
-    int i = (int)idxf;
-    i = i < 1 ? 1 : (i > PB_LINE_NTAB_DEV - 1 ? PB_LINE_NTAB_DEV - 1 : i);
-    R t = idxf - R(i);
-    return __ldg(I + i - 1) * (R(1) - t) + __ldg(I + i) * t;
-}
-
-// FP32 table, index and interpolation fraction formed in FP64 from an FP64 q: near the support
-// edge the line-integrated kernel is small and steep, and an FP32 q / dq would move the
-// fraction by ~4e-4 of a table step
-__device__ __forceinline__ float line_lut_q64(const float *__restrict__ I, double qmax, double q)
-{
-    const double dq = qmax / double(PB_LINE_NTAB_DEV - 1);
-    const double idxf = q / dq + 1.0;
-    int i = (int)idxf;
-    i = i < 1 ? 1 : (i > PB_LINE_NTAB_DEV - 1 ? PB_LINE_NTAB_DEV - 1 : i);
-    const float t = (float)(idxf - (double)i);
-    return __ldg(I + i - 1) * (1.f - t) + __ldg(I + i) * t;
-}
-
-template <typename R>
-__global__ void __launch_bounds__(128) k_lines(DevTree T, DevCatalog C, int64_t nl, const double *__restrict__ ox,
-                                               const double *__restrict__ oy, const double *__restrict__ oz,
-                                               const double *__restrict__ mx, const double *__restrict__ my,
-                                               const double *__restrict__ mz, const uint32_t *__restrict__ perm,
-                                               const R *__restrict__ table)
-{
-    const int64_t n = T.n;
-    const int k = T.kernel;
-    const double K = kernel_valid(k);
-    const R qmax = (R)K;
-    const R *I = table + (int64_t)k * PB_LINE_NTAB_DEV;
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nl; j += (int64_t)gridDim.x * blockDim.x) {
-        int64_t li = perm ? (int64_t)__ldg(perm + j) : j;
-        if (li >= nl) continue;
-        double o[3] = {__ldg(ox + li), __ldg(oy + li), __ldg(oz + li)};
-        double m[3] = {__ldg(mx + li), __ldg(my + li), __ldg(mz + li)};
-        // FP64 mode: plain sums in the reference order; FP32 mode: compensated with offsets
-        double S1 = 0.0, acc[MAXS];
-        CSum cS1, cacc[MAXS];
-        double Ahat[MAXS];
-        bool have = false;
-        cS1.zero();
-#pragma unroll
-        for (int s = 0; s < MAXS; ++s) { acc[s] = 0.0; cacc[s].zero(); Ahat[s] = 0.0; }
-        int node = T.root;
-        int64_t bi = 0, guard = 0, limit = 4 * n + 64;
-        bool brute = (node == 0);
-        while (brute ? (bi < n) : (node != 0)) {
-            if (++guard > limit) { flag(T.status, ST_TRAVERSAL); break; }
-            bool leafnode = brute || node >= n;
-            if (leafnode) {
-                int64_t b = brute ? bi++ : (int64_t)(node - n);
-                double4 L = ldg4(T.leaf + b);
-                int esc = brute ? 0 : __ldg(T.leaf_escape + b);
-                double r = __dmul_rn(K, L.w);
-                double r2 = __dmul_rn(r, r);
-                double d2 = d2_line(L.x, L.y, L.z, o, m);
-                if (d2 <= r2) {
-                    double mb = __ldg(T.m + b), rb = __ldg(T.rho + b);
-                    if (sizeof(R) == 8) {
-                        // line_integrated_kernel_function (line_integrated_kernel.jl:132-137)
-                        double dr = sqrt(d2 > 0.0 ? d2 : 0.0);
-                        double invh = 1.0 / L.w;
-                        double q = dr * invh;
-                        double Iq = (q >= K) ? 0.0 : (double)line_lut<R>(I, qmax, (R)q);
-                        double W = invh * Iq;
-                        double w = mb * W / rb;
-                        S1 += w;
-#pragma unroll
-                        for (int s = 0; s < MAXS; ++s)
-                            if (s < C.n_scalar) acc[s] += __ldg(C.ucol[C.s_u[s]] + b) * w;
-                    } else {
-                        // the line distance and q in FP64 (the pair-distance part), the kernel
-                        // value and the sums in FP32
-                        const double q = sqrt(d2 > 0.0 ? d2 : 0.0) * (1.0 / L.w);
-                        const float invh = (float)(1.0 / L.w);
-                        float Iq = (q >= K) ? 0.f : line_lut_q64(reinterpret_cast<const float *>(I), K, q);
-                        float w = (float)mb * (invh * Iq) / (float)rb;
-                        cS1.add(w);
-#pragma unroll
-                        for (int s = 0; s < MAXS; ++s) {
-                            if (s < C.n_scalar) {
-                                double A = __ldg(C.ucol[C.s_u[s]] + b);
-                                if (!have) Ahat[s] = A;
-                                cacc[s].add((float)(A - Ahat[s]) * w);
-                            }
-                        }
-                        have = true;
-                    }
-                }
-                if (!brute) node = esc;
-            } else {
-                NodeF nd = load_node(T.node + (node - 1));
-                double r = __dmul_rn(K, (double)__ldg(T.node_hmax + (node - 1)));
-                double r2 = __dmul_rn(r, r);
-                node = (d2_line_box_lower(o, m, nd) > r2) ? nd.escape : nd.left;
-            }
-        }
-        double S = (sizeof(R) == 8) ? S1 : cS1.val();
-        int l = 0;
-#pragma unroll
-        for (int s = 0; s < MAXS; ++s) {
-            if (s < C.n_scalar) {
-                double v;
-                if (S == 0.0) v = __longlong_as_double(0x7ff8000000000000LL);
-                else if (sizeof(R) == 8) v = C.s_shep[s] ? acc[s] * (1.0 / S) : acc[s];
-                else v = C.s_shep[s] ? Ahat[s] + cacc[s].val() / S : Ahat[s] * S + cacc[s].val();
-                C.out[l++][li] = v;
-            }
-        }
-    }
-}
 
 }  // namespace pb

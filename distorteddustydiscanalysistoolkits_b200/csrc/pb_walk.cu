@@ -388,9 +388,10 @@ cudaError_t launch_lpt_order(Handle *H, const RunPool &P, int64_t m, uint32_t **
 
 // pair order of a walked slice and the number of heavy queries at its front: heaviest first
 // (LPT) unless `plain`, where it is the stable heavy/light partition of the walk order; the
-// accepted pairs of the heavy and the light queries are added to pairs[0], pairs[1]
+// accepted pairs of the heavy and the light queries are added to pairs[0], pairs[1] (zero before);
+// *light_pairs is the latter's value
 cudaError_t launch_split_order(Handle *H, const RunPool &P, int64_t m, unsigned light_max, bool plain,
-                               uint32_t **order, int64_t *m_heavy, unsigned long long *pairs)
+                               uint32_t **order, int64_t *m_heavy, int64_t *light_pairs, unsigned long long *pairs)
 {
     cudaError_t e;
     if (!plain) {
@@ -415,9 +416,12 @@ cudaError_t launch_split_order(Handle *H, const RunPool &P, int64_t m, unsigned 
     H->launches += 1;
     if ((e = cudaGetLastError())) return e;
     unsigned hcount = 0;
+    unsigned long long lp = 0;
     if ((e = cudaMemcpyAsync(&hcount, cnt, sizeof(unsigned), cudaMemcpyDeviceToHost, H->stream))) return e;
+    if ((e = cudaMemcpyAsync(&lp, pairs + 1, sizeof(lp), cudaMemcpyDeviceToHost, H->stream))) return e;
     if ((e = cudaStreamSynchronize(H->stream))) return e;
     *m_heavy = hcount;
+    *light_pairs = (int64_t)lp;
     return cudaSuccess;
 }
 
