@@ -875,10 +875,9 @@ int do_lines(Handle &H, const pb_catalog *cat, int64_t nl, const double *ox, con
     std::vector<int> is_host;
     if ((rc = stage_outputs(H, L, nl, out, dev, is_host))) return rc;
     DevTree T = make_tree(H);
-    // Both precision modes take the FP64 line kernel.  An FP32-compensated line sum needs its
+    // Both precision modes take the FP64 line kernels: FP32-compensated sums would need their
     // projected distances and table indices in FP64 too (FP32 ones miss the 1e-5 tolerance on
-    // 256^2 images), so only its accumulation would be cheaper, and that did not pay: the whole
-    // C3 image took 433 ms with FP32C accumulation against 388 ms in FP64.
+    // 256^2 images), so only the accumulation would be cheaper.
     std::vector<Launch> launches = plan(items_of(cat, false));
     ev_record(H, 2);   // the line ordering is part of the timed interpolation
     const uint32_t *perm;

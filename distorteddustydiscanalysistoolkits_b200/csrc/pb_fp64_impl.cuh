@@ -15,21 +15,6 @@
 namespace pb {
 
 // ------------------------------------------------------------------------------------
-// a / b, correctly rounded, from y = RN(1/b): Markstein's theorem (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", 1990; Muller et al., Handbook of
-// Floating-Point Arithmetic, on division with a correctly rounded reciprocal): if q is
-// within one ulp of a/b, RN(q + y RN(a - b q)) is RN(a/b).  a y can be off by 1.5 ulp, so one step
-// brings q within an ulp and the second one gives the quotient.  `safe` says that both operands
-// are in the exponent range where no step can under- or overflow (exp_safe); otherwise (zero,
-// infinities and NaN included) they are divided.
-__device__ __forceinline__ double div_by(double a, double b, double y, bool safe)
-{
-    if (!safe) return a / b;
-    double q = a * y;
-    q = fma(fma(-q, b, a), y, q);
-    return fma(fma(-q, b, a), y, q);
-}
-
 // x^N as jl_pow computes it for finite x >= 0, with the steps that only add zeros left out:
 // (p, e) -> (p^2, its low part) is one squaring of the compensated pair.
 __device__ __forceinline__ void jl_sq(double &p, double &e)
@@ -311,23 +296,6 @@ __device__ __forceinline__ void terms64(const DevCatalog &C, const Query64 &Q, c
         put(17, on ? az * qx - ax * qz : 0.0);
         put(18, on ? ax * qy - ay * qx : 0.0);
     }
-}
-
-// adds a row's first `fill` terms to acc in slot order
-__device__ __forceinline__ double add_row(const double *row, int fill, double acc)
-{
-    const double2 *r2 = reinterpret_cast<const double2 *>(row);
-    if (fill == 32) {
-#pragma unroll
-        for (int s = 0; s < 16; ++s) {
-            const double2 v = r2[s];
-            acc += v.x;
-            acc += v.y;
-        }
-        return acc;
-    }
-    for (int s = 0; s < fill; ++s) acc += row[s];
-    return acc;
 }
 
 __device__ __forceinline__ void finalize64(const double *v, const DevCatalog &C, int64_t qi)

@@ -15,7 +15,7 @@
 //     gradient/divergence/curl F - A B cancels as little as possible;
 //   * each lane sums its terms in plain FP32 over chunks of 32 full batches of 32 pairs (32 of
 //     its own pairs) and adds each chunk sum, converted exactly, to an FP64 accumulator.
-// Line integrals are not here: both precision modes use the FP64 line kernel (pb_interp64.cu).
+// Line integrals are not here: both precision modes use the FP64 line kernels (pb_lines.cu).
 // The per-query arithmetic depends only on the query and the tree (chunks are counted over
 // the query's own accepted-neighbour sequence), never on the launch shape or schedule.
 #include "pb_internal.h"

@@ -79,6 +79,22 @@ __device__ __forceinline__ NodeF load_node(const NodeF *p)
     return nd;
 }
 
+// ------------------------------------------------------------------------------------
+// a / b, correctly rounded, from y = RN(1/b): Markstein's theorem (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990; Muller et al., Handbook of
+// Floating-Point Arithmetic, on division with a correctly rounded reciprocal): if q is
+// within one ulp of a/b, RN(q + y RN(a - b q)) is RN(a/b).  a y can be off by 1.5 ulp, so one step
+// brings q within an ulp and the second one gives the quotient.  `safe` says that both operands
+// are in the exponent range where no step can under- or overflow (exp_safe); otherwise (zero,
+// infinities and NaN included) they are divided.
+__device__ __forceinline__ double div_by(double a, double b, double y, bool safe)
+{
+    if (!safe) return a / b;
+    double q = a * y;
+    q = fma(fma(-q, b, a), y, q);
+    return fma(fma(-q, b, a), y, q);
+}
+
 // --------------------------------------------------------------------------------------
 // FP32 box tests with directed rounding.  The query point is kept as round-down/round-up
 // floats; gaps, squares and sums are rounded toward the safe side, so `lower` never exceeds
@@ -550,6 +566,23 @@ __device__ __forceinline__ int deal_runs_part(const RunPool &P, int64_t j, int l
         }
     }
     return turn == w ? fill : 0;
+}
+
+// adds a row's first `fill` terms to acc in slot order
+__device__ __forceinline__ double add_row(const double *row, int fill, double acc)
+{
+    const double2 *r2 = reinterpret_cast<const double2 *>(row);
+    if (fill == 32) {
+#pragma unroll
+        for (int s = 0; s < 16; ++s) {
+            const double2 v = r2[s];
+            acc += v.x;
+            acc += v.y;
+        }
+        return acc;
+    }
+    for (int s = 0; s < fill; ++s) acc += row[s];
+    return acc;
 }
 
 // the n == 1 tree has no internal node: its single leaf is tested directly
