@@ -2,12 +2,10 @@
 // own LBVH, particles, grid and outputs.  The sample points of all discs form one index space
 // (disc after disc, in the processing order the host chose), cut into slices of a fixed size.
 // Per slice, these launches cover every disc:
-//   1. k_batch_nearest, k_batch_filter (count, bucket scan, emit) and k_batch_walk_list: one
-//      thread per sample point finds its disc (binary search over the discs' first indices)
-//      and its nearest particle; every disc's tree is cut into subtrees on the device after
-//      its build, the (point, subtree) items whose subtree root survives the walk's first test
-//      are listed grouped by (disc, subtree), and warps walk that list, appending the
-//      accepted leaves as runs to a shared pool (the single-disc path's prefiltered walk);
+//   1. k_batch_nearest and k_batch_walk: one thread per sample point finds its disc (binary
+//      search over the discs' first indices) and its nearest particle; one warp per point, in
+//      Morton order disc by disc, walks its disc's tree and appends the accepted leaves as runs
+//      to a shared pool (the single-disc path's walk);
 //   2. k_batch_pairs: one warp per sample point sums its runs with the bodies of the single-disc
 //      pair kernels -- FP64 (the reference's arithmetic) for FP64 mode and for FP32C points of at
 //      most light_max accepted neighbours, FP32-compensated for heavier ones -- and a point whose
@@ -79,104 +77,25 @@ __global__ void __launch_bounds__(128) k_batch_nearest(const BatchDisc *__restri
     }
 }
 
-// Prefilter of the walk items (the single-disc k_item_filter for many discs): item (t, s) is
-// walked only if the walk would not prune the root of subtree s of point t's disc at its first
-// step; the others (and every s past the disc's cut) get an empty record here.  Walked items
-// are counted per bucket (disc slot, subtree) and, with EMIT, listed bucket by bucket at
-// off[bucket] + cursor, so that the lanes of a walk warp share a disc and a subtree; points are
-// taken in `order` (the Morton walk order of the slice; NULL: slice order), so a bucket lists
-// neighbouring points next to each other.  The atomics are aggregated over the lanes of a warp
-// with equal buckets.
-template <int STRAT, bool EMIT>
-__global__ void __launch_bounds__(128) k_batch_filter(const BatchDisc *__restrict__ discs,
-                                                      const int64_t *__restrict__ starts,
-                                                      const uint32_t *__restrict__ slot_disc,
-                                                      const int *__restrict__ slot_of, int64_t s0, int64_t m,
-                                                      RunPool P, const uint32_t *__restrict__ order, unsigned *cnt,
-                                                      const unsigned *__restrict__ off, uint2 *list)
-{
-    const int ns = P.ns;
-    const int lane = threadIdx.x & 31;
-    const int64_t mw = (m + 31) & ~int64_t(31);   // whole warps, so every lane reaches the votes
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < mw; p += (int64_t)gridDim.x * blockDim.x) {
-        const bool live = p < m;
-        const int64_t t = live && order ? (int64_t)__ldg(order + p) : p;   // the point at walk position p
-        int lo = 0, nc = 0;
-        const BatchDisc *D = nullptr;
-        QBox q{};
-        float r2a_up = 0.f, Kf = 0.f;
-        if (live) {
-            lo = __ldg(slot_of + t);
-            D = discs + __ldg(slot_disc + lo);
-            nc = min(__ldg(D->ncut), ns);   // the cut holds at most ns subtrees
-            const int64_t qi = s0 + t - __ldg(starts + lo);
-            const double px = __ldg(D->qx + qi), py = __ldg(D->qy + qi), pz = __ldg(D->qz + qi);
-            const double K = kernel_valid(D->T.kernel);
-            double ha = 0.0;
-            if (STRAT != SCATTER) {
-                const int b = P.bnear[t];
-                ha = b < 0 ? __longlong_as_double(0x7ff8000000000000LL) : ldg4(D->T.leaf + b).w;
-            }
-            const double ra = __dmul_rn(K, ha);
-            r2a_up = __double2float_ru(__dmul_rn(ra, ra));
-            Kf = (float)K;
-            q = make_qbox(px, py, pz);
-        }
-        const int smax = __reduce_max_sync(0xffffffffu, nc);
-        for (int s = 0; s < smax; ++s) {
-            bool walk = false;
-            if (s < nc) {
-                const DevTree &T = D->T;
-                const int node = __ldg(&D->cut[s].x);
-                walk = true;
-                if (T.root != 0 && node < T.n)
-                    walk = !node_pruned<STRAT>(T, load_node(T.node + (node - 1)), node, q, Kf, r2a_up);
-                if (!walk && !EMIT) P.items[t * ns + s] = make_int2(-1, 0);
-            }
-            const unsigned key = (unsigned)lo * (unsigned)ns + (unsigned)s;
-            const unsigned act = __ballot_sync(0xffffffffu, walk);
-            if (walk) {
-                const unsigned grp = __match_any_sync(act, key);
-                const int leader = __ffs(grp) - 1;
-                const unsigned rank = __popc(grp & ((1u << lane) - 1u));
-                unsigned base = 0;
-                if (lane == leader) base = atomicAdd(cnt + key, (unsigned)__popc(grp));
-                base = __shfl_sync(grp, base, leader);
-                if (EMIT) list[off[key] + base + rank] = make_uint2((unsigned)t, (unsigned)s);
-            }
-        }
-        if (live && !EMIT)
-            for (int s = nc; s < ns; ++s) P.items[t * ns + s] = make_int2(-1, 0);
-    }
-}
-
-// the walk over the prefiltered list: nlist = off[nb - 1] + cnt[nb - 1], read on the device
+// the walk of the slice's points in walk order (k_walk for many discs)
 template <int STRAT>
-__global__ void __launch_bounds__(128) k_batch_walk_list(const BatchDisc *__restrict__ discs,
-                                                         const int64_t *__restrict__ starts,
-                                                         const uint32_t *__restrict__ slot_disc,
-                                                         const int *__restrict__ slot_of, int64_t s0, RunPool P,
-                                                         const unsigned *__restrict__ cnt,
-                                                         const unsigned *__restrict__ off, int nb,
-                                                         const uint2 *__restrict__ list, unsigned long long *counter)
+__global__ void __launch_bounds__(128, 8) k_batch_walk(const BatchDisc *__restrict__ discs,
+                                                       const int64_t *__restrict__ starts,
+                                                       const uint32_t *__restrict__ slot_disc,
+                                                       const int *__restrict__ slot_of, int64_t s0, int64_t m, RunPool P,
+                                                       const uint32_t *__restrict__ order, unsigned long long *counter)
 {
-    const int lane = threadIdx.x & 31;
-    const int64_t nlist = (int64_t)__ldg(off + nb - 1) + __ldg(cnt + nb - 1);
+    __shared__ int s_walk[BATCH_WARPS][WALK_SMEM];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     for (;;) {
-        unsigned long long wi = 0;
-        if (lane == 0) wi = atomicAdd(counter, 1ULL);
-        wi = __shfl_sync(0xffffffffu, wi, 0);
-        if ((int64_t)wi * 32 >= nlist) break;
-        const int64_t k = (int64_t)wi * 32 + lane;
-        if (k >= nlist) continue;
-        const uint2 it = __ldg(list + k);
-        const int64_t t = it.x;
+        const int64_t p = next_query(counter, lane);
+        if (p >= m) break;
+        const int64_t t = __ldg(order + p);
         const int lo = __ldg(slot_of + t);
         const BatchDisc &D = discs[__ldg(slot_disc + lo)];
-        const DevTree &T = D.T;
         const int64_t qi = s0 + t - __ldg(starts + lo);
-        walk_item_at<STRAT>(T, P, D.cut, t, (int)it.y, (uint32_t)t, __ldg(D.qx + qi), __ldg(D.qy + qi),
-                            __ldg(D.qz + qi), kernel_valid(T.kernel));
+        walk_query<STRAT>(D.T, P, t, (uint32_t)t, __ldg(D.qx + qi), __ldg(D.qy + qi), __ldg(D.qz + qi),
+                          kernel_valid(D.T.kernel), s_walk[wib], lane);
     }
 }
 
@@ -356,24 +275,14 @@ static void launch_slice_pairs(Handle *H, int cat, int cat64, const BatchDisc *d
         discs, starts, slot_disc, ndisc, s0, m, P, O, fp64_only, light_max, leaf_size, ctr + 2);
 }
 
-// nearest particles, the Morton walk order (*worder), prefilter (count, bucket scan, emit) and
-// the walk of a slice
+// nearest particles, the Morton walk order (*worder) and the walk of a slice
 template <int STRAT>
 static cudaError_t launch_walk_batch(Handle *H, const BatchDisc *discs, const int64_t *starts,
                                      const uint32_t *slot_disc, int ndisc, int64_t s0, int64_t m, const RunPool &P,
                                      int *slot_of, int slot_bits, const uint32_t **worder,
                                      unsigned long long *counter)
 {
-    const int64_t nb = (int64_t)ndisc * P.ns;
     cudaError_t e;
-    if ((e = H->batch_bcnt.reserve(sizeof(unsigned) * nb)) || (e = H->batch_boff.reserve(sizeof(unsigned) * nb)) ||
-        (e = H->batch_bcur.reserve(sizeof(unsigned) * nb)) || (e = H->batch_list.reserve(sizeof(uint2) * m * P.ns)))
-        return e;
-    unsigned *cnt = H->batch_bcnt.as<unsigned>(), *off = H->batch_boff.as<unsigned>(), *cur = H->batch_bcur.as<unsigned>();
-    uint2 *list = H->batch_list.as<uint2>();
-    if ((e = cudaMemsetAsync(cnt, 0, sizeof(unsigned) * nb, H->stream)) ||
-        (e = cudaMemsetAsync(cur, 0, sizeof(unsigned) * nb, H->stream)))
-        return e;
     k_batch_nearest<STRAT><<<grid_for(m, 128, 1 << 30), 128, 0, H->stream>>>(discs, starts, slot_disc, ndisc, s0, m, P,
                                                                           slot_of);
     // walk order: disc by disc (processing slot), Morton order of the points inside a disc
@@ -386,14 +295,9 @@ static cudaError_t launch_walk_batch(Handle *H, const BatchDisc *discs, const in
     if ((e = sort_pairs_u64(H, mk, mv, H->batch_mka.as<uint64_t>(), H->batch_mva.as<uint32_t>(), m, 32 + slot_bits)))
         return e;
     *worder = mv;
-    k_batch_filter<STRAT, false><<<grid_for(m, 128, 1 << 30), 128, 0, H->stream>>>(
-        discs, starts, slot_disc, slot_of, s0, m, P, nullptr, cnt, nullptr, nullptr);
-    if ((e = launch_exclusive_scan_u32(H, cnt, off, nb))) return e;
-    k_batch_filter<STRAT, true><<<grid_for(m, 128, 1 << 30), 128, 0, H->stream>>>(discs, starts, slot_disc, slot_of,
-                                                                                s0, m, P, mv, cur, off, list);
-    k_batch_walk_list<STRAT><<<persistent_blocks_of(k_batch_walk_list<STRAT>, 0), 128, 0, H->stream>>>(
-        discs, starts, slot_disc, slot_of, s0, P, cnt, off, (int)nb, list, counter);
-    H->launches += 4;
+    k_batch_walk<STRAT><<<persistent_blocks_of(k_batch_walk<STRAT>, 0), 128, 0, H->stream>>>(
+        discs, starts, slot_disc, slot_of, s0, m, P, mv, counter);
+    H->launches += 2;
     return cudaGetLastError();
 }
 
@@ -417,8 +321,7 @@ static void launch_slice_strat(Handle *H, int kernel, int cat, int cat64, const 
 #undef PB_SLICE
 }
 
-// One slice [s0, s0 + m) of the batch's sample points: nearest particles, the walk over
-// (point, subtree) items, the pair order (by class, then disc, with the FP32C/FP64 split
+// One slice [s0, s0 + m) of the batch's sample points: nearest particles, the walk, the pair order (by class, then disc, with the FP32C/FP64 split
 // counted on the device), then the sums.  slot_of holds m ints.
 // ctr: [0..2] persistent pair-kernel counters, [3..4] pair split sums, [5] heavy count (low
 // word), [6] walk queue.

@@ -24,15 +24,15 @@ pb::Handle::~Handle()
                    &scan_part, &hist, &bbox_part, &qparams, &status, &leaf, &leaf_aux, &odd, &leaf_escape, &node, &node_hmax, &node_child, &node_range, &payload, &counter, &left,
                    &right, &escape, &parent, &bmin64, &bmax64, &hmax64, &counters, &rho_s, &col_ptrs,
                    &q_x, &q_y, &q_z, &q_keys, &q_keys_alt, &q_perm, &q_perm_alt, &q_out, &q_aux,
-                   &pool_runs, &pool_next, &pool_ctr, &items, &wbnear, &qacc, &qflag, &cut, &defer_a, &defer_b,
-                   &lpt_k, &lpt_v, &lpt_ka, &lpt_va, &iota, &grid_ax, &grid_out, &wl_cnt, &wl_off, &wl_s, &wl_j, &wl_sa, &wl_ja, &mlp_w, &mlp_m, &mlp_v, &mlp_g, &mlp_norm,
+                   &pool_runs, &pool_next, &pool_ctr, &items, &wbnear, &qacc, &qflag, &defer_a, &defer_b,
+                   &lpt_k, &lpt_v, &lpt_ka, &lpt_va, &iota, &grid_ax, &grid_out, &mlp_w, &mlp_m, &mlp_v, &mlp_g, &mlp_norm,
                    &mlp_scr, &mlp_idx, &mlp_x, &mlp_y, &mlp_loss, &sched_feat, &sched_pred, &sched_ql, &sched_tmp};
     for (DBuf *b : all) b->release();
     batch_desc.release();
     batch_starts.release();
     batch_slots.release();
     batch_ctr.release();
-    for (DBuf *b : {&batch_slot_of, &batch_bcnt, &batch_boff, &batch_bcur, &batch_list, &batch_mk, &batch_mka, &batch_mv,
+    for (DBuf *b : {&batch_slot_of, &batch_mk, &batch_mka, &batch_mv,
                     &batch_mva})
         b->release();
     if (batch_host) cudaFreeHost(batch_host);
@@ -104,7 +104,6 @@ int check_status(Handle &H)
     if (st & ST_TRAVERSAL) return fail(H, PB_ERR_INTERNAL, "traversal exceeded its iteration bound");
     if (st & ST_POOL)
         return fail(H, PB_ERR_DIMENSION, "neighbour pool offsets too small for a query (DimensionMismatch)");
-    if (st & ST_CUT) return fail(H, PB_ERR_INTERNAL, "walk cut larger than its capacity (raise batch_walk_split)");
     return PB_OK;
 }
 
@@ -480,11 +479,11 @@ int do_build(Handle &H, const pb_input *in, int32_t flags)
 // PB_RUN_POOL_MB, or set exactly in chunks by PB_RUN_POOL_CHUNKS; it never drops below what
 // one query can need (n/2 runs) unless one of the two variables asks for less.  Buffers only
 // grow; the cap of a call is what it may use.
-int reserve_pool(Handle &H, int64_t m, int ns)
+int reserve_pool(Handle &H, int64_t m)
 {
     const unsigned long long per_chunk = sizeof(uint2) * RUN_CHUNK + sizeof(int);
     const unsigned long long min_chunks =
-        (unsigned long long)((H.n / 2 + 1 + RUN_CHUNK - 1) / RUN_CHUNK) + (unsigned long long)ns + 64;
+        (unsigned long long)((H.n / 2 + 1 + RUN_CHUNK - 1) / RUN_CHUNK) + RUN_EXTENT + 64;
     unsigned long long want = (unsigned long long)m * 24ULL;
     if (want < min_chunks) want = min_chunks;
     const char *env = getenv("PB_RUN_POOL_MB");
@@ -522,7 +521,7 @@ int reserve_pool(Handle &H, int64_t m, int ns)
     }
     H.pool_cap = cap;
     CK(H.pool_ctr.reserve(64));   // [0] chunks used, [1] deferred | heavy count, [2] walk queue, [4..5] pair split
-    CK(H.items.reserve(sizeof(int2) * m * ns));
+    CK(H.items.reserve(sizeof(int2) * m));
     CK(H.wbnear.reserve(sizeof(int) * m));
     CK(H.qacc.reserve(sizeof(unsigned) * m));
     CK(H.qflag.reserve(sizeof(int) * m));
@@ -544,8 +543,6 @@ int fused_fallback(Handle &H, const DevTree &T, const std::vector<Launch> &launc
     CK(H.sched_tmp.reserve(sizeof(uint32_t) * 2 * nd));
     lst = H.sched_tmp.as<uint32_t>();
     CK(cudaMemcpyAsync(lst, P.deferred, sizeof(uint32_t) * nd, cudaMemcpyDeviceToDevice, H.stream));
-    CK(cudaMemsetAsync(P.qacc, 0, sizeof(unsigned) * nd, H.stream));
-    CK(cudaMemsetAsync(P.qflag, 0, sizeof(int) * nd, H.stream));
     P.count_only = 1;
     if (strategy != SCATTER) CK(launch_nearest_list(&H, T, nd, lst, dx, dy, dz, P.bnear));
     unsigned long long *ctr = H.pool_ctr.as<unsigned long long>();
@@ -617,16 +614,16 @@ bool grow_pool(Handle &H)
 // at it when the others have finished.
 constexpr int64_t BLOCK64_SHARE = 4096, BLOCK64_MIN = 8192;
 
-// FP32-compensated points in two phases: the walk kernels write every (query, subtree) item's
-// accepted runs, the pair kernel evaluates them (once per catalog launch).  Queries go through
-// in slices of H.slice (Morton order when sorted), which bounds the item and pool memory.
+// FP32-compensated points in two phases: the walk kernel writes every query's accepted runs,
+// the pair kernel evaluates them (once per catalog launch).  Queries go through
+// in slices of H.slice (Morton order when sorted), which bounds the pool memory.
 // Queries that found the pool full are walked again in another round with an emptied pool;
 // if a round completes fewer than 1/8 of its queries, the fused walk-and-sum kernel takes the
 // rest.  Both kernels produce identical bits for a query.
 //
 // Schedule modes (H.sched), all with identical results:
-//   0 plain:   queries in input order, one walk item per query, pairs in walk order;
-//   1 tuned:   Morton order, walk split into ~walk_split subtrees, pairs heaviest first;
+//   0 plain:   queries in input order, pairs in walk order;
+//   1 tuned:   Morton order, pairs heaviest first;
 //   2 learned: as tuned, with the walk order binned by the MLP's predicted work
 //              (heaviest class first, Morton order inside a class).
 int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &launches,
@@ -636,12 +633,8 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
     if (npts > 0x7fffffffLL) return fail(H, PB_ERR_CAPACITY, "more than 2^31-1 sample points in one call");
     const int mode = H.sched;
     if (mode == 2 && !H.mlp_ready) return fail(H, PB_ERR_STATE, "learned schedule requested but no scheduler weights set");
-    int ns = 1;
-    CK(launch_cut(&H, T, mode == 0 ? 1 : H.walk_split, &ns));
-    // a slice holds at most 2^31 - 1 (query, subtree) items: the work-list offsets are 32-bit
-    const int64_t S_items = std::max<int64_t>(1024, (int64_t)0x7fffffff / std::max(ns, 1));
-    const int64_t S = std::min<int64_t>(std::min<int64_t>(H.slice > 0 ? H.slice : npts, npts), S_items);
-    int rc = reserve_pool(H, S, ns);
+    const int64_t S = std::min<int64_t>(H.slice > 0 ? H.slice : npts, npts);
+    int rc = reserve_pool(H, S);
     if (rc) return rc;
     const uint32_t *ql_all = mode == 0 ? nullptr : perm;
     if (!ql_all) {
@@ -677,15 +670,11 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
         for (int round = 0;; ++round) {
             CK(cudaMemsetAsync(ctr, 0, 16, H.stream));
             CK(cudaMemsetAsync(ctr + 4, 0, 16, H.stream));
-            CK(cudaMemsetAsync(H.qacc.p, 0, sizeof(unsigned) * m, H.stream));
-            CK(cudaMemsetAsync(H.qflag.p, 0, sizeof(int) * m, H.stream));
             RunPool P;
             P.runs = H.pool_runs.as<uint2>();
             P.next = H.pool_next.as<int>();
             P.used = ctr;
             P.cap = H.pool_cap;
-            P.ns = ns;
-            P.cut = H.cut.as<int2>() + (4 * (mode == 0 ? 1 : H.walk_split) + 8);
             P.items = H.items.as<int2>();
             P.bnear = H.wbnear.as<int>();
             P.qacc = H.qacc.as<unsigned>();
@@ -693,7 +682,6 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
             P.n_deferred = reinterpret_cast<unsigned *>(ctr + 1);
             P.deferred = lists[round & 1];
             P.count_only = 0;
-            P.leaf_size = H.leaf_size;
             ev_record(H, 4);
             if (strategy != SCATTER || mode == 2) {
                 CK(launch_nearest_list(&H, T, m, ql, dx, dy, dz, P.bnear));
@@ -715,8 +703,7 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
                 H.interp_launches += 4;
             }
             ev_record(H, 5);
-            if (mode == 0 || ns == 1) CK(launch_walk(&H, T, strategy, P, m, ql, dx, dy, dz, ctr + 2));
-            else CK(launch_walk_list(&H, T, strategy, P, m, ql, dx, dy, dz, ctr + 2));
+            CK(launch_walk(&H, T, strategy, P, m, ql, dx, dy, dz, ctr + 2));
             H.interp_launches++;
             uint32_t *order = nullptr;
             int64_t m_heavy = 0;
@@ -1554,8 +1541,6 @@ int32_t pb_batch_points(pb_handle *const *discs, int32_t ndiscs, const pb_catalo
         D.qy = qy[k];
         D.qz = qz[k];
         D.nq = npts[k];
-        // the disc's walk cut, made on the device from the tree just built
-        CK(launch_cut_device(&Hk, D.T, H.batch_walk_split, &D.cut, &D.ncut));
         D.qp = Hk.qparams.as<QuantParams>();
         if (precision == PB_FP32C) {
             float4 *pay = nullptr;
@@ -1572,14 +1557,11 @@ int32_t pb_batch_points(pb_handle *const *discs, int32_t ndiscs, const pb_catalo
     CK(cudaMemcpyAsync(H.batch_slots.p, ho, slot_bytes, cudaMemcpyHostToDevice, H.stream));
     // slices of a fixed size share one run pool, sized once (a call that reuses it allocates
     // nothing, which is what lets a step be captured in a CUDA graph)
-    // (point, subtree) item records per point: the largest cut launch_cut_device can make
-    const int NS = 4 * H.batch_walk_split + 8;
     const int64_t S = std::max<int64_t>(1, std::min<int64_t>(H.slice > 0 ? H.slice : qtotal, qtotal));
-    if (qtotal > 0 && (H.pool_cap == 0 || H.batch_slice < S || H.batch_ns < NS)) {
-        int rc = reserve_pool(H, S, NS);
+    if (qtotal > 0 && (H.pool_cap == 0 || H.batch_slice < S)) {
+        int rc = reserve_pool(H, S);
         if (rc) return rc;
         H.batch_slice = S;
-        H.batch_ns = NS;
     }
     if (qtotal > 0) {
         CK(H.batch_slot_of.reserve(sizeof(int) * H.batch_slice));
@@ -1589,8 +1571,6 @@ int32_t pb_batch_points(pb_handle *const *discs, int32_t ndiscs, const pb_catalo
         P.next = H.pool_next.as<int>();
         P.used = ctr;
         P.cap = H.pool_cap;
-        P.ns = NS;
-        P.cut = nullptr;   // every disc's own cut is in its descriptor
         P.items = H.items.as<int2>();
         P.bnear = H.wbnear.as<int>();
         P.qacc = H.qacc.as<unsigned>();
@@ -1598,12 +1578,9 @@ int32_t pb_batch_points(pb_handle *const *discs, int32_t ndiscs, const pb_catalo
         P.n_deferred = reinterpret_cast<unsigned *>(ctr + 1);
         P.deferred = H.defer_a.as<uint32_t>();
         P.count_only = 0;
-        P.leaf_size = H.leaf_size;
         for (int64_t s0 = 0; s0 < qtotal; s0 += S) {
             const int64_t m = std::min<int64_t>(S, qtotal - s0);
             CK(cudaMemsetAsync(ctr, 0, 16, H.stream));
-            CK(cudaMemsetAsync(P.qacc, 0, sizeof(unsigned) * m, H.stream));
-            CK(cudaMemsetAsync(P.qflag, 0, sizeof(int) * m, H.stream));
             CK(launch_batch_slice(&H, strategy, H.kernel, cat_shape, cat_shape64, H.batch_desc.as<BatchDisc>(),
                                   H.batch_starts.as<int64_t>(), H.batch_slots.as<uint32_t>(), ndiscs, s0, m, P,
                                   precision == PB_FP64 ? 1 : 0, (unsigned)H.light_max, H.leaf_size, H.batch_blocks,

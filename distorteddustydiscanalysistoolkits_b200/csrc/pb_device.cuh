@@ -34,7 +34,6 @@ constexpr int ST_NONFINITE = 1;     // non-finite particle coordinate or smoothi
 constexpr int ST_REFIT = 2;         // an internal node was not combined exactly twice
 constexpr int ST_TRAVERSAL = 4;     // a traversal exceeded its iteration bound (corrupt tree)
 constexpr int ST_POOL = 8;          // neighbour pool too small for a query
-constexpr int ST_CUT = 16;          // a walk cut made on the device had more subtrees than its capacity
 
 struct __align__(16) NodeF {
     float lox, loy, loz;
@@ -58,31 +57,27 @@ struct DevTree {
     int *status;
 };
 
-// Accepted-neighbour run lists written by the walk kernel and read by the pair kernels.
-// The tree is cut into ns disjoint subtrees whose leaf ranges follow one another in DFS
-// order; every (query, subtree) item is walked separately.  A run is a maximal interval of
-// consecutive sorted leaves accepted by one item, stored as (first leaf, length); an item's
-// runs are kept in DFS (= ascending leaf) order in a linked list of fixed-size chunks drawn
-// from one pool, and items[j * ns + s] = (first chunk, number of runs).  Concatenating a
-// query's items in subtree order gives its accepted leaves in the reference's DFS order.
+// Accepted-neighbour run lists written by the walk kernel and read by the pair kernels.  A run
+// is a maximal interval of consecutive sorted leaves accepted by one query, stored as (first leaf,
+// length); a query's runs are kept in DFS (= ascending leaf) order in extents of RUN_EXTENT
+// consecutive chunks of RUN_CHUNK runs drawn from one pool (a query of up to 256 runs reads one
+// contiguous piece), linked by the last chunk's `next`; items[j] = (first chunk, number of runs).
 constexpr int RUN_CHUNK = 32;
+constexpr int RUN_EXTENT = 8;
 constexpr int RUN_DEFERRED = -2;
 
 struct RunPool {
     uint2 *runs;                  // cap * RUN_CHUNK (first leaf, length)
-    int *next;                    // cap chunk links (-1 ends a list)
+    int *next;                    // cap chunk links (of the last chunk of an extent)
     unsigned long long *used;     // chunks handed out (may run past cap)
     unsigned long long cap;       // chunks in the pool
-    int ns;                       // subtrees of the cut
-    const int2 *cut;              // (subtree root, node after the subtree in DFS order) per subtree
-    int2 *items;                  // m * ns item heads
+    int2 *items;                  // m list heads
     int *bnear;                   // nearest sorted leaf per walked query (-1: none / not needed)
     unsigned *qacc;               // accepted leaves per walked query
-    int *qflag;                   // 1: some item of the query found the pool full (deferred)
+    int *qflag;                   // 1: the query found the pool full (deferred)
     unsigned *n_deferred;         // queries deferred in this walk
     uint32_t *deferred;           // their query indices
     int count_only;               // 1: only count accepted leaves (qacc); no runs, no items
-    int leaf_size;                // walk cutoff: subtrees of at most this many leaves are scanned
 };
 
 // Catalog of one launch.  ucol[] are the unique sorted quantity columns read per

@@ -19,8 +19,6 @@ struct BatchDisc {
     DevCatalog C32, C64;
     const float4 *pay;
     const double *qx, *qy, *qz;
-    const int2 *cut;     // the disc's walk cut (subtree root, node after it), in DFS order
-    const int *ncut;     // its number of subtrees (device-resident: the cut is made on the device)
     const QuantParams *qp;   // the disc's quantisation frame (Morton order of its sample points)
     int64_t nq;
     int stride;
@@ -91,10 +89,9 @@ struct Handle {
 
     // run lists of the two-phase point path (walk kernel -> pair kernels)
     DBuf grid_ax, grid_out;   // axes / points of pb_grid_points
-    DBuf wl_cnt, wl_off, wl_s, wl_j, wl_sa, wl_ja;   // (query, subtree) work list of the walk
-    DBuf pool_runs, pool_next, pool_ctr, items, wbnear, qacc, qflag, cut, defer_a, defer_b, lpt_k, lpt_v, lpt_ka,
+    DBuf pool_runs, pool_next, pool_ctr, items, wbnear, qacc, qflag, defer_a, defer_b, lpt_k, lpt_v, lpt_ka,
         lpt_va, iota;
-    int walk_split = 64;   // target number of subtrees each query's walk is split into
+    int walk_split = 64;   // accepted and kept; the walk is not split any more
     int sched = 1;         // 0 plain (input order, one walk per query, no ordering), 1 tuned, 2 learned
     int64_t light_max = 4096;   // FP32C: queries with at most this many neighbours are summed in FP64
     int64_t slice = int64_t(1) << 22;   // queries per two-phase slice
@@ -119,10 +116,8 @@ struct Handle {
     int batch_order = 0;     // 0: discs in the given order, 1: discs with the most work first
     int batch_blocks = 0;    // blocks per SM of the batched pair kernel (0: as many as fit)
     int64_t batch_slice = 0; // sample points per slice the batch's run pool was sized for
-    int batch_ns = 0;        // subtrees per point the batch's item records were sized for
-    int batch_walk_split = 16;   // target number of subtrees per disc of the batched walk
+    int batch_walk_split = 16;   // accepted and kept, as walk_split
     DBuf batch_slot_of;      // processing slot of every point of a slice
-    DBuf batch_bcnt, batch_boff, batch_bcur, batch_list;   // walk prefilter: buckets and item list
     DBuf batch_mk, batch_mka, batch_mv, batch_mva;         // Morton walk order of a slice
 
     // query-side scratch
@@ -163,16 +158,10 @@ cudaError_t launch_query_codes(Handle *H, int64_t nq, const double *qx, const do
 cudaError_t launch_permute_back(Handle *H, int64_t n, const uint32_t *idx, const double *src, double *dst);
 
 // ---- launchers (pb_walk.cu) ----
-cudaError_t launch_cut(Handle *H, const DevTree &T, int target, int *ns_out);
-// launch_cut without the read-back: the ordered cut and its size stay on the device
-cudaError_t launch_cut_device(Handle *H, const DevTree &T, int target, const int2 **cut, const int **count);
 cudaError_t launch_nearest_list(Handle *H, const DevTree &T, int64_t m, const uint32_t *ql, const double *qx,
                                 const double *qy, const double *qz, int *bnear);
 cudaError_t launch_walk(Handle *H, const DevTree &T, int strategy, const RunPool &P, int64_t m, const uint32_t *ql,
                         const double *qx, const double *qy, const double *qz, unsigned long long *counter);
-cudaError_t launch_walk_list(Handle *H, const DevTree &T, int strategy, const RunPool &P, int64_t m,
-                             const uint32_t *ql, const double *qx, const double *qy, const double *qz,
-                             unsigned long long *counter);
 cudaError_t launch_lpt_order(Handle *H, const RunPool &P, int64_t m, uint32_t **order);
 cudaError_t launch_split_order(Handle *H, const RunPool &P, int64_t m, unsigned light_max, bool plain,
                                uint32_t **order, int64_t *m_heavy, int64_t *light_pairs, unsigned long long *pairs);

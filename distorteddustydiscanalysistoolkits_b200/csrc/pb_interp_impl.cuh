@@ -1,8 +1,8 @@
 // pb_interp_impl.cuh -- the traversal building blocks shared by the interpolation units:
 // nearest-h search, the stackless left/escape DFS of the ball query
-// (LinearBVHTraversalMacros.jl:26-371) in its warp-uniform (next_item) and flat per-thread
-// (walk_subtree) forms, the dealing of a query's accepted runs to the lanes of a warp
-// (deal_runs), the FP64 accumulator of the reference's arithmetic and the line kernel.
+// (LinearBVHTraversalMacros.jl:26-371) in its warp-uniform form (next_item), the dealing of a
+// query's accepted runs to the lanes of a warp (deal_runs) and the FP64 accumulator of the
+// reference's arithmetic.
 //
 // Included by pb_interp64.cu (-fmad=false; FP64 terms in the reference's expressions and
 // order, bit-exact with the FP64 oracle), pb_interp32.cu (FP32 per-pair terms with double-float
@@ -302,78 +302,6 @@ __device__ __forceinline__ bool next_item(const DevTree &T, Walk &w, double px, 
     }
 }
 
-// Flat form of the same walk for one thread, over the subtree entered at `start` and left at
-// `stop`: one node step per loop iteration, and every accepted item (a single leaf, or the
-// whole leaf range of a subtree inside the query radius) passed to emit(lo, hi) in DFS order.
-// The decisions are next_item's, step for step (with the same leaf_size cutoff: a small
-// subtree's leaves tested in sorted order); a warp running this loop reconverges once per node
-// step instead of once per accepted item.  Returns false if emit refused an item.
-template <int STRAT, typename EMIT>
-__device__ __forceinline__ bool walk_subtree(const DevTree &T, int start, int stop, double px, double py, double pz,
-                                             double K, double r2a, EMIT &emit, int leaf_size = 1)
-{
-    const int64_t n = T.n;
-    const QBox q = make_qbox(px, py, pz);
-    const float Kf = (float)K;
-    const float r2a_up = __double2float_ru(r2a);
-    const float bulk_lim = __fmul_rd(__double2float_rd(r2a), MARGIN_DN);
-    const int64_t limit = 4 * n + 64;
-    int64_t guard = 0;
-    int node = start;
-    while (node != stop) {
-        if (++guard > limit) {
-            flag(T.status, ST_TRAVERSAL);
-            break;
-        }
-        int64_t lo = -1, hi = -1;
-        if (node >= n) {
-            const int64_t b = node - n;
-            const double4 L = ldg4(T.leaf + b);
-            node = __ldg(T.leaf_escape + b);
-            double r2;
-            if (STRAT == GATHER) r2 = r2a;
-            else {
-                const double r = __dmul_rn(K, L.w);
-                const double rr = __dmul_rn(r, r);
-                r2 = STRAT == SCATTER ? rr : (r2a > rr ? r2a : rr);
-            }
-            if (d2_point(px, py, pz, L) <= r2) lo = hi = b;
-        } else {
-            const NodeF nd = load_node(T.node + (node - 1));
-            if (node_pruned<STRAT>(T, nd, node, q, Kf, r2a_up)) {
-                node = nd.escape;
-            } else if (STRAT != SCATTER && box_upper(q, nd) <= bulk_lim) {
-                const int2 rg = __ldg(T.range + (node - 1));
-                lo = rg.x;
-                hi = rg.y;
-                node = nd.escape;
-            } else if (leaf_size > 1 && __ldg(&T.range[node - 1].y) - __ldg(&T.range[node - 1].x) < leaf_size) {
-                const int2 rg = __ldg(T.range + (node - 1));
-                for (int64_t b = rg.x; b <= rg.y; ++b) {   // the subtree's leaves in sorted order
-                    if (++guard > limit) {
-                        flag(T.status, ST_TRAVERSAL);
-                        return true;
-                    }
-                    const double4 L = ldg4(T.leaf + b);
-                    double r2;
-                    if (STRAT == GATHER) r2 = r2a;
-                    else {
-                        const double r = __dmul_rn(K, L.w);
-                        const double rr = __dmul_rn(r, r);
-                        r2 = STRAT == SCATTER ? rr : (r2a > rr ? r2a : rr);
-                    }
-                    if (d2_point(px, py, pz, L) <= r2 && !emit(b, b)) return false;
-                }
-                node = nd.escape;
-            } else {
-                node = nd.left;
-            }
-        }
-        if (lo >= 0 && !emit(lo, hi)) return false;
-    }
-    return true;
-}
-
 // Slot filler shared by the warp-per-query kernels: accepted leaves, in DFS order, are
 // dealt to the 32 lanes (the k-th accepted leaf goes to lane k mod 32); PROC(fill) is
 // called whenever 32 slots are full and once more for the remainder.
@@ -412,7 +340,7 @@ __device__ __forceinline__ int64_t next_query(unsigned long long *counter, int l
 // One chunk of up to 32 runs of an item, one run per lane (lanes past the last run hold an
 // empty one), with the inclusive prefix sums of the run lengths: leaf position t of the chunk,
 // 0 <= t < tot, lies in the first run r with inc[r] > t.  Leaf indices and counts are 32-bit
-// (n <= 2^30; an item's accepted leaves lie in one subtree).
+// (n <= 2^30).
 struct RunWindow {
     int lo, inc, ex, tot;          // this lane's run: first leaf, inclusive and exclusive prefix
     int r0 = -1, end0 = 0;         // run of the last position looked up, and where it ends
@@ -459,10 +387,16 @@ struct RunWindow {
     }
 };
 
-// Dealing of a walked query's accepted leaves (its items in subtree order, the runs of each
-// item chunk by chunk) to the 32 lanes in DFS order: the k-th accepted leaf goes to lane
-// k mod 32.  first(b) is called with the first leaf of every non-empty item (the callee uses
-// the very first one); one(mine) for every full batch (every lane holds a leaf); two(m1) for
+// the chunk after chunk c of a list with `left` runs from c on
+__device__ __forceinline__ int next_chunk(const RunPool &P, int c, int left)
+{
+    if (left <= RUN_CHUNK) return -1;
+    return (c & (RUN_EXTENT - 1)) != RUN_EXTENT - 1 ? c + 1 : __ldg(P.next + c);
+}
+
+// Dealing of a walked query's accepted leaves (its runs, chunk by chunk) to the 32 lanes in DFS
+// order: the k-th accepted leaf goes to lane k mod 32.  first(b) is called with the first leaf
+// of a non-empty list; one(mine) for every full batch (every lane holds a leaf); two(m1) for
 // two consecutive full batches inside one run (lane leaves m1 and m1 + 32) when cantwo()
 // allows it, and four(m1) for four of them (m1, m1 + 32, m1 + 64, m1 + 96) when canfour()
 // does.  Returns the fill of the last, partial batch, whose leaves are left in `mine` (-1 on
@@ -471,53 +405,43 @@ template <typename FIRST, typename ONE, typename TWO, typename CANTWO, typename 
 __device__ __forceinline__ int deal_runs(const RunPool &P, int64_t j, int lane, FIRST &first, ONE &one, TWO &two,
                                          CANTWO &cantwo, FOUR &four, CANFOUR &canfour, int &mine)
 {
-    const int ns = P.ns;
-    int fill = 0;
+    const int2 itm = __ldg(P.items + j);
+    int fill = 0, c = itm.x, left = itm.y;
     mine = -1;
-    for (int s0 = 0; s0 < ns; s0 += 32) {
-        const int2 itm = s0 + lane < ns ? __ldg(P.items + j * ns + s0 + lane) : make_int2(-1, 0);
-        unsigned nonempty = __ballot_sync(0xffffffffu, itm.y > 0);
-        while (nonempty) {
-            const int l = __ffs(nonempty) - 1;
-            nonempty &= nonempty - 1;
-            int c = __shfl_sync(0xffffffffu, itm.x, l);
-            int left = __shfl_sync(0xffffffffu, itm.y, l);
-            first((int)__ldg(&P.runs[(int64_t)c * RUN_CHUNK].x));
-            while (left > 0) {
-                const int cnt = left < RUN_CHUNK ? left : RUN_CHUNK;
-                const int nextc = left > RUN_CHUNK ? __ldg(P.next + c) : -1;
-                RunWindow R(P, c, cnt, lane);
-                int tb = -fill;
-                for (;;) {
-                    // t0 < tot = inc[cnt - 1], so the cursor stops at a run of this chunk
-                    R.seek(tb <= 0 ? 0 : (tb < R.tot ? tb : R.tot - 1));
-                    if (tb >= 0 && tb + 64 <= R.end0) {
-                        const int m1 = R.lo0 + (tb - R.ex0) + lane;
-                        if (tb + 128 <= R.end0 && canfour()) {   // four full batches inside one run
-                            four(m1);
-                            tb += 128;
-                            continue;
-                        }
-                        if (cantwo()) {   // two full batches inside one run
-                            two(m1);
-                            tb += 64;
-                            continue;   // the next pass assigns or closes what is left of the chunk
-                        }
-                    }
-                    R.leaf_of(tb, lane, mine);
-                    if (tb + 31 < R.tot) {
-                        one(mine);   // full batch
-                        mine = -1;
-                        tb += 32;
-                    } else {
-                        fill = R.tot - tb;
-                        break;
-                    }
+    if (left > 0) first((int)__ldg(&P.runs[(int64_t)c * RUN_CHUNK].x));
+    while (left > 0) {
+        const int cnt = left < RUN_CHUNK ? left : RUN_CHUNK;
+        const int nextc = next_chunk(P, c, left);
+        RunWindow R(P, c, cnt, lane);
+        int tb = -fill;
+        for (;;) {
+            // t0 < tot = inc[cnt - 1], so the cursor stops at a run of this chunk
+            R.seek(tb <= 0 ? 0 : (tb < R.tot ? tb : R.tot - 1));
+            if (tb >= 0 && tb + 64 <= R.end0) {
+                const int m1 = R.lo0 + (tb - R.ex0) + lane;
+                if (tb + 128 <= R.end0 && canfour()) {   // four full batches inside one run
+                    four(m1);
+                    tb += 128;
+                    continue;
                 }
-                left -= cnt;
-                c = nextc;
+                if (cantwo()) {   // two full batches inside one run
+                    two(m1);
+                    tb += 64;
+                    continue;   // the next pass assigns or closes what is left of the chunk
+                }
+            }
+            R.leaf_of(tb, lane, mine);
+            if (tb + 31 < R.tot) {
+                one(mine);   // full batch
+                mine = -1;
+                tb += 32;
+            } else {
+                fill = R.tot - tb;
+                break;
             }
         }
+        left -= cnt;
+        c = nextc;
     }
     return fill;
 }
@@ -528,42 +452,32 @@ __device__ __forceinline__ int deal_runs(const RunPool &P, int64_t j, int lane, 
 template <int W, typename ONE>
 __device__ __forceinline__ int deal_runs_part(const RunPool &P, int64_t j, int lane, int w, ONE &one, int &mine)
 {
-    const int ns = P.ns;
-    int fill = 0, turn = 0;   // turn: the current batch's number mod W
+    const int2 itm = __ldg(P.items + j);
+    int fill = 0, c = itm.x, left = itm.y, turn = 0;   // turn: the current batch's number mod W
     mine = -1;
-    for (int s0 = 0; s0 < ns; s0 += 32) {
-        const int2 itm = s0 + lane < ns ? __ldg(P.items + j * ns + s0 + lane) : make_int2(-1, 0);
-        unsigned nonempty = __ballot_sync(0xffffffffu, itm.y > 0);
-        while (nonempty) {
-            const int l = __ffs(nonempty) - 1;
-            nonempty &= nonempty - 1;
-            int c = __shfl_sync(0xffffffffu, itm.x, l);
-            int left = __shfl_sync(0xffffffffu, itm.y, l);
-            while (left > 0) {
-                const int cnt = left < RUN_CHUNK ? left : RUN_CHUNK;
-                const int nextc = left > RUN_CHUNK ? __ldg(P.next + c) : -1;
-                RunWindow R(P, c, cnt, lane);
-                int tb = -fill;
-                for (;;) {
-                    if (turn == w && tb < R.tot) {
-                        R.seek(tb < 0 ? 0 : tb);
-                        R.leaf_of(tb, lane, mine);
-                    }
-                    if (tb + 31 >= R.tot) {
-                        fill = R.tot - tb;
-                        break;
-                    }
-                    if (turn == w) {
-                        one(mine);
-                        mine = -1;
-                    }
-                    tb += 32;
-                    turn = turn + 1 == W ? 0 : turn + 1;
-                }
-                left -= cnt;
-                c = nextc;
+    while (left > 0) {
+        const int cnt = left < RUN_CHUNK ? left : RUN_CHUNK;
+        const int nextc = next_chunk(P, c, left);
+        RunWindow R(P, c, cnt, lane);
+        int tb = -fill;
+        for (;;) {
+            if (turn == w && tb < R.tot) {
+                R.seek(tb < 0 ? 0 : tb);
+                R.leaf_of(tb, lane, mine);
             }
+            if (tb + 31 >= R.tot) {
+                fill = R.tot - tb;
+                break;
+            }
+            if (turn == w) {
+                one(mine);
+                mine = -1;
+            }
+            tb += 32;
+            turn = turn + 1 == W ? 0 : turn + 1;
         }
+        left -= cnt;
+        c = nextc;
     }
     return turn == w ? fill : 0;
 }
