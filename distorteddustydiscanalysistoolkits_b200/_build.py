@@ -21,7 +21,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", CSRC, "-I", INCLUDE,
-                 "-Xptxas", "-warn-spills", "--split-compile", "0"]
+                 "-Xptxas", "-warn-spills"]
 UNITS = {
     "pb_build.cu": ["-fmad=false"],
     "pb_interp64.cu": ["-fmad=false"],

@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(128, 5) k_batch_pairs32(const BatchDisc *__res
 }
 
 template <int STRAT, int KT, int CAT>
-__global__ void __launch_bounds__(128, minb64<CAT>()) k_batch_pairs64(const BatchDisc *__restrict__ discs,
+__global__ void __launch_bounds__(128, minb64<STRAT, CAT>()) k_batch_pairs64(const BatchDisc *__restrict__ discs,
                                                        const int64_t *__restrict__ starts,
                                                        const uint32_t *__restrict__ slot_disc, int ndisc, int64_t s0,
                                                        int64_t m, RunPool P, SliceOrder O, unsigned long long *counter)

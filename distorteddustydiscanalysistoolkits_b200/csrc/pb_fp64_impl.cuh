@@ -176,15 +176,15 @@ __device__ constexpr int row_of(int a)   // term row of accumulator a, -1 if it 
     return a;
 }
 
-// Blocks of 128 threads per SM of the pair kernels.  They wait on loads and on the chain of
-// dependent additions, so resident warps count for more than registers (the cap of 7 blocks is
-// 72 registers and spills a little): pair sums of 2.8e9 pairs, four columns with gradient,
-// divergence and curl, M4 symmetric, 42.7 / 41.4 / 40.6 / 37.4 / 52.1 ms at 4 / 5 / 6 / 7 / 8 blocks;
-// one scalar (557e6 pairs) 6.1 / 6.6 / 6.7 / 5.8 / 5.4 ms.
-template <int CAT>
+// Blocks of 128 threads per SM of the pair kernels: they wait on loads and on the chain of
+// dependent additions, so resident warps count against the registers (102 at 5 blocks, 85 at 6).
+// 2.8e9 pairs, four columns with gradient, divergence and curl, M4 symmetric: 39.7 / 40.3 / 46.8 /
+// 40.6 / 44.5 ms at 4 / 5 / 6 / 7 / 8 blocks; one scalar (1.2e9 pairs) 8.4 / 7.6 / 8.3 / 9.1 / 9.3; one side
+// (gather, M6, 3.5e9 pairs) needs fewer registers: 50.1 / 43.0 / 38.9 / 39.6 / 40.2.
+template <int STRAT, int CAT>
 __host__ __device__ constexpr int minb64()
 {
-    return CAT == CAT_S1 ? 8 : (CAT == CAT_ANY ? 5 : 7);
+    return STRAT == SYMMETRIC || CAT == CAT_ANY ? 5 : 6;
 }
 
 // Term buffer of a warp: one row per term, one column per lane.  Lanes write their own column

@@ -53,7 +53,7 @@ __device__ __forceinline__ int64_t count_above(const RunPool &P, int64_t m, cons
 }
 
 template <int STRAT, int KT, int CAT>
-__global__ void __launch_bounds__(128, minb64<CAT>()) k_pairs64w(
+__global__ void __launch_bounds__(128, minb64<STRAT, CAT>()) k_pairs64w(
     DevTree T, DevCatalog C, RunPool P, int64_t m, unsigned block_min, const uint32_t *__restrict__ ql,
     const uint32_t *__restrict__ order, const double *__restrict__ qx, const double *__restrict__ qy,
     const double *__restrict__ qz, unsigned long long *counter)

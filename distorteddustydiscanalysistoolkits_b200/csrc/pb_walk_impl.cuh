@@ -3,35 +3,48 @@
 // Shared by the walk kernels (pb_walk.cu) and the batched walk (pb_batch.cu).
 //
 // The warp keeps a stack of tree entries whose top is the next one in DFS order.  Each round its
-// lanes take the top 32: an entry that the query does not reach is dropped, a subtree inside the
-// query's radius or an accepted leaf stays as an accepted range, any other subtree is replaced by
-// its two children.  The accepted ranges before the first subtree still open are the next ones in
-// DFS order and are appended to the runs.  The decisions are those of next_item (node_pruned,
-// box_upper, the exact leaf test), so the accepted set and its order are the reference's.
+// lanes take the top 32: a subtree that the query does not reach is dropped; one inside the
+// query's radius, one of at most WALK_SCAN leaves and a leaf stay; any other is replaced by its two
+// children.  The entries that stay and come before the first one opened are the next ones in DFS
+// order: they collect until there are 32, then their leaves are tested 32 at a time (those of a
+// subtree inside the radius pass as a whole) and what is accepted is appended to the runs.  The node
+// decisions are next_item's (node_pruned, box_upper) and the leaf test is exact, so the accepted set
+// and its order are the reference's.
 //
 // A thread per (query, subtree) item, as before, kept 6.7 of 32 lanes busy (paths of different length,
 // and leaf, prune, accept and emit steps in turn) and needed a cut of the tree, a prefilter, a sorted
-// work list and 64 item records a query; here the 32 lanes test 32 entries of one query.
+// work list and 64 item records a query; here the 32 lanes test 32 entries of one query.  Walk phase
+// before and now: 2.1e6 particles and 4.2e6 points 133 -> 102 ms, 131,072 particles on 64^3 points
+// 3.9 -> 2.5 ms, 1e5 tracers (scatter) 1.43 -> 0.72 ms.
 #pragma once
 #include "pb_interp_impl.cuh"
 
 namespace pb {
 
+// Leaves of a subtree that are tested instead of opening it: a test is a 32-byte load and ten FP64
+// operations, batched over the lanes, an opening two more box tests.  Walk phase at 1 / 4 / 8 / 16 / 32:
+// 2.1e6 particles, 4.2e6 points 147 / 119 / 107 / 102 / 109 ms; 131,072 particles, 64^3 points 3.2 / 2.7 /
+// 2.5 / 2.5 / 2.6; scatter, 1e5 tracers 0.82 / 0.72 / 0.71 / 0.72 / 0.76.
+constexpr int WALK_SCAN = 16;
 constexpr int WSTACK = 512;   // entries; taken one at a time above WSTACK - 160, where a round adds at most one
-constexpr int WALK_SMEM = WSTACK + 128;   // ints of shared memory per warp
+constexpr int WALK_SMEM = WSTACK + 256;   // ints of shared memory per warp
 
 template <int STRAT>
 struct WarpWalk {
     const DevTree &T;
     const RunPool &P;
-    int *stack, *rlo, *rhi;   // WSTACK entries; 64 runs not written yet, the last one still open
+    int *stack;               // WSTACK entries
+    int *clo, *clen;          // 64 candidates in DFS order: first leaf, and the number of leaves to be tested
+                              // or minus the number of leaves accepted as a whole
+    int *rlo, *rhi;           // 64 runs not written yet, the last one still open
     int lane;
-    int cnt = 0;              // runs in rlo/rhi
+    int cand = 0, cnt = 0;    // candidates, runs
     int first = -1, cur = -1, nruns = 0;
     int nacc = 0;             // this lane's share of the accepted leaves
 
     __device__ __forceinline__ WarpWalk(const DevTree &t, const RunPool &p, int *smem, int l)
-        : T(t), P(p), stack(smem), rlo(smem + WSTACK), rhi(smem + WSTACK + 64), lane(l)
+        : T(t), P(p), stack(smem), clo(smem + WSTACK), clen(smem + WSTACK + 64), rlo(smem + WSTACK + 128),
+          rhi(smem + WSTACK + 192), lane(l)
     {
     }
     // writes the first k <= 32 runs as one chunk; false if the pool is full
@@ -82,6 +95,55 @@ struct WarpWalk {
         }
         return true;
     }
+    // tests the leaves of the first k <= 32 candidates, appends what is accepted and removes them;
+    // false if the pool is full
+    __device__ __forceinline__ bool settle(int k, double px, double py, double pz, double K, double r2a)
+    {
+        const int c0 = lane < k ? clo[lane] : 0, len = lane < k ? clen[lane] : 0;
+        const int width = len < 0 ? 1 : len;   // positions: one per leaf to be tested, one per accepted range
+        int inc = width;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += v;
+        }
+        const int tot = __shfl_sync(0xffffffffu, inc, 31), ex = inc - width;
+        for (int tb = 0; tb < tot; tb += 32) {
+            // the candidate of position tb + lane: that of position tb plus the candidates that start
+            // between them
+            const int r0 = __popc(__ballot_sync(0xffffffffu, inc <= tb)), s = ex - tb;
+            const unsigned starts = __reduce_or_sync(0xffffffffu, s > 0 && s < 32 && width > 0 ? 1u << s : 0u);
+            const int r = (r0 + __popc(starts & (0xffffffffu >> (31 - lane)))) & 31;
+            const int l = __shfl_sync(0xffffffffu, c0, r), n = __shfl_sync(0xffffffffu, len, r),
+                      e = __shfl_sync(0xffffffffu, ex, r);
+            bool on = tb + lane < tot;
+            int lo = l, hi = l - n - 1;
+            if (on && n > 0) {
+                lo = hi = l + (tb + lane - e);
+                const double4 L = ldg4(T.leaf + lo);
+                double r2;
+                if (STRAT == GATHER) r2 = r2a;
+                else {
+                    const double rad = __dmul_rn(K, L.w);
+                    const double rr = __dmul_rn(rad, rad);
+                    r2 = STRAT == SCATTER ? rr : (r2a > rr ? r2a : rr);
+                }
+                on = d2_point(px, py, pz, L) <= r2;
+            }
+            const unsigned done = __ballot_sync(0xffffffffu, on);
+            if (done && !append(done, lo, hi)) return false;
+        }
+        __syncwarp();
+        cand -= k;
+        if (cand > 0) {
+            const int a = clo[32 + lane], b = clen[32 + lane];
+            __syncwarp();
+            clo[lane] = a;
+            clen[lane] = b;
+        }
+        __syncwarp();
+        return true;
+    }
     // the walk from the root; false if the pool is full
     __device__ __forceinline__ bool run(double px, double py, double pz, double K, double r2a)
     {
@@ -91,8 +153,8 @@ struct WarpWalk {
         const float r2a_up = __double2float_ru(r2a);
         const float bulk_lim = __fmul_rd(__double2float_rd(r2a), MARGIN_DN);
         const unsigned below = (1u << lane) - 1u;
-        const int64_t limit = 4 * T.n + 64;
-        int64_t guard = 0;
+        const unsigned limit = 2u * (unsigned)n + 64u;   // every round settles or opens at least one entry
+        unsigned guard = 0;
         int size = 1;
         if (lane == 0) stack[0] = T.root;
         __syncwarp();
@@ -102,64 +164,52 @@ struct WarpWalk {
                 break;
             }
             const int k = size > WSTACK - 160 ? 1 : (size < 32 ? size : 32);
-            int c = 0, e0 = 0, e1 = 0, lo = 0, hi = 0;   // c: entries that replace this one
+            int c = 0, e0 = 0, e1 = 0, lo = 0, len = 1;   // c: entries that replace this one
             if (lane < k) {
-                const int e = stack[size - 1 - lane];
-                const int id = e & 0x7fffffff;
-                if (id >= n) {
-                    lo = hi = id - n;
-                    c = 1;
-                    if (e >= 0) {
-                        const double4 L = ldg4(T.leaf + lo);
-                        double r2;
-                        if (STRAT == GATHER) r2 = r2a;
-                        else {
-                            const double r = __dmul_rn(K, L.w);
-                            const double rr = __dmul_rn(r, r);
-                            r2 = STRAT == SCATTER ? rr : (r2a > rr ? r2a : rr);
-                        }
-                        if (!(d2_point(px, py, pz, L) <= r2)) c = 0;
-                    }
-                    e0 = (int)((unsigned)id | 0x80000000u);
-                } else {
+                e0 = stack[size - 1 - lane];
+                c = 1;
+                lo = e0 - n;
+                if (e0 < n) {
+                    const int id = e0;
                     const int2 rg = __ldg(T.range + (id - 1));
+                    const NodeF nd = load_node(T.node + (id - 1));
                     lo = rg.x;
-                    hi = rg.y;
-                    if (e < 0) {   // accepted whole in an earlier round
-                        c = 1;
-                        e0 = e;
-                    } else {
-                        const NodeF nd = load_node(T.node + (id - 1));
-                        if (node_pruned<STRAT>(T, nd, id, q, Kf, r2a_up)) {
-                            c = 0;
-                        } else if (STRAT != SCATTER && box_upper(q, nd) <= bulk_lim) {
-                            c = 1;
-                            e0 = (int)((unsigned)id | 0x80000000u);
-                        } else {
-                            // the children of a Karras node meet at the split, which the left child's
-                            // id gives; a child of one leaf is that leaf
-                            c = 2;
-                            e0 = nd.left;
-                            const int split = nd.left >= n ? nd.left - (n - 1) : nd.left;   // 1-based
-                            e1 = split == hi ? n + hi : split + 1;
-                        }
+                    len = rg.y - rg.x + 1;
+                    if (node_pruned<STRAT>(T, nd, id, q, Kf, r2a_up)) {
+                        c = 0;
+                    } else if (STRAT != SCATTER && box_upper(q, nd) <= bulk_lim) {
+                        len = -len;
+                    } else if (len > WALK_SCAN) {
+                        // the children of a Karras node meet at the split, which the left child's id
+                        // gives; a child of one leaf is that leaf
+                        c = 2;
+                        e0 = nd.left;
+                        const int split = nd.left >= n ? nd.left - (n - 1) : nd.left;   // 1-based
+                        e1 = split == rg.y ? n + rg.y : split + 1;
                     }
                 }
             }
             __syncwarp();
-            const unsigned open = __ballot_sync(0xffffffffu, c == 2);
-            const int firstopen = open ? __ffs(open) - 1 : 32;
-            const unsigned done = __ballot_sync(0xffffffffu, c == 1 && lane < firstopen);
-            const unsigned kept = __ballot_sync(0xffffffffu, c >= 1 && lane >= firstopen);
+            const unsigned open = __ballot_sync(0xffffffffu, c == 2), stay = __ballot_sync(0xffffffffu, c >= 1);
+            const unsigned pre = open ? (open & -open) - 1u : 0xffffffffu;   // lanes before the first open one
+            const unsigned done = stay & pre, kept = stay & ~pre;
             size += __popc(kept) + __popc(open) - k;
-            if (c >= 1 && lane >= firstopen) {
-                const int at = size - 1 - __popc(kept & below) - __popc(open & below);
-                stack[at] = e0;
-                if (c == 2) stack[at - 1] = e1;
+            if (c >= 1) {
+                if ((done >> lane) & 1u) {
+                    const int at = cand + __popc(done & below);
+                    clo[at] = lo;
+                    clen[at] = len;
+                } else {
+                    const int at = size - 1 - __popc(kept & below) - __popc(open & below);
+                    stack[at] = e0;
+                    if (c == 2) stack[at - 1] = e1;
+                }
             }
+            cand += __popc(done);
             __syncwarp();
-            if (done && !append(done, lo, hi)) return false;
+            if (cand >= 32 && !settle(32, px, py, pz, K, r2a)) return false;
         }
+        if (cand > 0 && !settle(cand, px, py, pz, K, r2a)) return false;
         return cnt == 0 || flush(cnt);
     }
 };

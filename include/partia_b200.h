@@ -87,11 +87,11 @@ int32_t pb_last_error(const pb_handle *h, char *buf, int64_t size);
 /* Launch on this stream (a cudaStream_t of the handle's device); NULL = the handle's own. */
 int32_t pb_set_stream(pb_handle *h, void *cuda_stream);
 /* Options: "timing" (record CUDA events around build/traversal), "sort_queries"
-   (Morton-order queries before traversal; schedule only), "block_size", "walk_split" (target
-   number of subtrees each FP32-compensated point walk is split into, 1..4096; schedule only),
-   "schedule" (FP32-compensated points: 0 plain = input order, one walk per query, no
-   ordering; 1 tuned = Morton order, split walks, heaviest first (default); 2 learned = tuned
-   plus binning by predicted work; results are identical), "slice_queries" (queries per
+   (Morton-order queries before traversal; schedule only), "block_size", "walk_split"
+   (1..4096; accepted and without effect: a warp walks a query's whole tree),
+   "schedule" (points: 0 plain = input order, no ordering; 1 tuned = Morton order, heaviest
+   sums first (default); 2 learned = tuned plus binning by predicted work; results are
+   identical), "slice_queries" (queries per
    walk/sum slice, default 2^22). */
 int32_t pb_set_option(pb_handle *h, const char *name, int64_t value);
 
@@ -173,14 +173,13 @@ int32_t pb_line_samples_interpolation(pb_handle *h, const pb_input *in, const pb
    snapshot per call, PointSamples_interpolation.jl:12-29; this batches calls).  discs[k] is a
    handle on which pb_linear_bvh has built disc k (PB_BUILD_ASYNC allowed); npts[k] sample
    points at qx[k], qy[k], qz[k] and the L = n_scalar + 3 n_grad + n_div + 3 n_curl outputs
-   out[k * L + l] are device memory.  Every disc's tree is cut into subtrees on the device; one
-   walk launch covers every disc's (point, subtree) items and persistent kernels sum every
-   disc's points (FP64: the reference's arithmetic; FP32C: queries with at most fp64_light_max
+   out[k * L + l] are device memory.  One walk launch covers every disc's points and persistent
+   kernels sum them (FP64: the reference's arithmetic; FP32C: queries with at most fp64_light_max
    neighbours in FP64, the rest FP32-compensated, decided on the device), with values equal to
    separate pb_interpolate_points calls bit for bit.  Every handle must use the first one's
    device, stream (pb_set_stream) and kernel; the catalog must fit one launch.  Options of
-   discs[0]: "leaf_size" (walk cutoff), "batch_walk_split" (target subtrees per disc, 1..1024,
-   default 16), "batch_order" (0 given, 1 most work first) and "batch_blocks_per_sm" (0 = all
+   discs[0]: "leaf_size" (linear-scan cutoff of the fused walk that takes over from a full pool),
+   "batch_walk_split" (1..1024; accepted and without effect), "batch_order" (0 given, 1 most work first) and "batch_blocks_per_sm" (0 = all
    that fit) change the schedule only.  With device pointers, no
    synchronisation and all buffers already sized by an earlier identical call, the builds with
    PB_BUILD_ASYNC and this call with PB_BATCH_ASYNC can be captured in a CUDA graph. */
@@ -269,8 +268,8 @@ int32_t pb_scheduler_train(pb_handle *h, const float *X, const float *y, int64_t
    walk rounds taken, queries deferred because the accepted-run pool was full (they are walked
    again, or finished by the fused kernel), the pool size in chunks of 32 runs, and (with
    option "timing") the device time in ms of the phases, summed over slices and walk rounds,
-   in phase_ms[3]: nearest search (with the learned binning), walk (with the prefilter and the
-   pair ordering), pair sums.  The pool follows
+   in phase_ms[3]: nearest search (with the learned binning), walk (with the pair
+   ordering), pair sums.  The pool follows
    PB_RUN_POOL_MB (MiB) or PB_RUN_POOL_CHUNKS from the environment when set. */
 int32_t pb_last_schedule(const pb_handle *h, int64_t *walk_rounds, int64_t *deferred, int64_t *pool_chunks,
                          double *phase_ms);
