@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(128, 8) k_batch_walk(const BatchDisc *__restri
                                                        const int *__restrict__ slot_of, int64_t s0, int64_t m, RunPool P,
                                                        const uint32_t *__restrict__ order, unsigned long long *counter)
 {
-    __shared__ int s_walk[BATCH_WARPS][WALK_SMEM];
+    __shared__ int s_walk[BATCH_WARPS][RUN_WALK_SMEM];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     for (;;) {
         const int64_t p = next_query(counter, lane);

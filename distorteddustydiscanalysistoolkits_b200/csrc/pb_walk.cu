@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(128, 8) k_walk(DevTree T, RunPool P, int64_t m
                                                  const double *__restrict__ qx, const double *__restrict__ qy,
                                                  const double *__restrict__ qz, int ticket, unsigned long long *counter)
 {
-    __shared__ int s_walk[4][WALK_SMEM];
+    __shared__ int s_walk[4][RUN_WALK_SMEM];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const double K = kernel_valid(T.kernel);
     for (;;) {

@@ -27,26 +27,20 @@ namespace pb {
 // 2.5 / 2.5 / 2.6; scatter, 1e5 tracers 0.82 / 0.72 / 0.71 / 0.72 / 0.76.
 constexpr int WALK_SCAN = 16;
 constexpr int WSTACK = 512;   // entries; taken one at a time above WSTACK - 160, where a round adds at most one
-constexpr int WALK_SMEM = WSTACK + 256;   // ints of shared memory per warp
+constexpr int WALK_SMEM = WSTACK + 128;       // ints of shared memory per warp of a WarpWalk
+constexpr int RUN_WALK_SMEM = WALK_SMEM + 128;   // and of one into a RunSink
 
-template <int STRAT>
-struct WarpWalk {
-    const DevTree &T;
+// where a walk's accepted ranges go: a query's runs in the shared pool
+struct RunSink {
     const RunPool &P;
-    int *stack;               // WSTACK entries
-    int *clo, *clen;          // 64 candidates in DFS order: first leaf, and the number of leaves to be tested
-                              // or minus the number of leaves accepted as a whole
     int *rlo, *rhi;           // 64 runs not written yet, the last one still open
     int lane;
-    int cand = 0, cnt = 0;    // candidates, runs
+    int cnt = 0;              // runs in rlo/rhi
     int first = -1, cur = -1, nruns = 0;
     int nacc = 0;             // this lane's share of the accepted leaves
 
-    __device__ __forceinline__ WarpWalk(const DevTree &t, const RunPool &p, int *smem, int l)
-        : T(t), P(p), stack(smem), clo(smem + WSTACK), clen(smem + WSTACK + 64), rlo(smem + WSTACK + 128),
-          rhi(smem + WSTACK + 192), lane(l)
-    {
-    }
+    __device__ __forceinline__ RunSink(const RunPool &p, int *smem, int l) : P(p), rlo(smem), rhi(smem + 64), lane(l) {}
+
     // writes the first k <= 32 runs as one chunk; false if the pool is full
     __device__ __forceinline__ bool flush(int k)
     {
@@ -67,7 +61,8 @@ struct WarpWalk {
             P.runs[(int64_t)cur * RUN_CHUNK + lane] = make_uint2((unsigned)rlo[lane], (unsigned)(rhi[lane] - rlo[lane] + 1));
         return true;
     }
-    // appends the ranges [lo, hi] of the lanes of `done`, in lane order; false if the pool is full
+    // appends the ranges [lo, hi] of the lanes of `done` (at least one), in lane order; false if the
+    // pool is full
     __device__ __forceinline__ bool append(unsigned done, int lo, int hi)
     {
         const unsigned self = 1u << lane, below = self - 1u;
@@ -95,8 +90,25 @@ struct WarpWalk {
         }
         return true;
     }
-    // tests the leaves of the first k <= 32 candidates, appends what is accepted and removes them;
-    // false if the pool is full
+    __device__ __forceinline__ bool finish() { return cnt == 0 || flush(cnt); }
+};
+
+template <int STRAT, typename SINK>
+struct WarpWalk {
+    const DevTree &T;
+    SINK &sink;
+    int *stack;               // WSTACK entries
+    int *clo, *clen;          // 64 candidates in DFS order: first leaf, and the number of leaves to be tested
+                              // or minus the number of leaves accepted as a whole
+    int lane;
+    int cand = 0;             // candidates
+
+    __device__ __forceinline__ WarpWalk(const DevTree &t, SINK &s, int *smem, int l)
+        : T(t), sink(s), stack(smem), clo(smem + WSTACK), clen(smem + WSTACK + 64), lane(l)
+    {
+    }
+    // tests the leaves of the first k <= 32 candidates, passes on what is accepted and removes them;
+    // false if the sink refused a range
     __device__ __forceinline__ bool settle(int k, double px, double py, double pz, double K, double r2a)
     {
         const int c0 = lane < k ? clo[lane] : 0, len = lane < k ? clen[lane] : 0;
@@ -131,7 +143,7 @@ struct WarpWalk {
                 on = d2_point(px, py, pz, L) <= r2;
             }
             const unsigned done = __ballot_sync(0xffffffffu, on);
-            if (done && !append(done, lo, hi)) return false;
+            if (done && !sink.append(done, lo, hi)) return false;
         }
         __syncwarp();
         cand -= k;
@@ -144,7 +156,7 @@ struct WarpWalk {
         __syncwarp();
         return true;
     }
-    // the walk from the root; false if the pool is full
+    // the walk from the root; false if the sink refused a range
     __device__ __forceinline__ bool run(double px, double py, double pz, double K, double r2a)
     {
         const int n = (int)T.n;
@@ -209,19 +221,19 @@ struct WarpWalk {
             __syncwarp();
             if (cand >= 32 && !settle(32, px, py, pz, K, r2a)) return false;
         }
-        if (cand > 0 && !settle(cand, px, py, pz, K, r2a)) return false;
-        return cnt == 0 || flush(cnt);
+        return cand == 0 || settle(cand, px, py, pz, K, r2a);
     }
 };
 
 // The walk of the j-th listed query (sample point qi at px, py, pz; nearest sorted leaf P.bnear[j]):
 // its run list, its number of accepted leaves, and whether the pool was full (the query is then
-// listed as deferred).  Every lane of the warp calls it; smem holds WALK_SMEM ints.
+// listed as deferred).  Every lane of the warp calls it; smem holds RUN_WALK_SMEM ints.
 template <int STRAT>
 __device__ __forceinline__ void walk_query(const DevTree &T, const RunPool &P, int64_t j, uint32_t qi, double px,
                                            double py, double pz, double K, int *smem, int lane)
 {
-    WarpWalk<STRAT> W(T, P, smem, lane);
+    RunSink R(P, smem + WALK_SMEM, lane);
+    WarpWalk<STRAT, RunSink> W(T, R, smem, lane);
     bool ok = P.count_only || *(volatile unsigned long long *)P.used < P.cap;   // else the pool is exhausted
     ok = __shfl_sync(0xffffffffu, ok, 0);
     if (ok) {
@@ -234,17 +246,18 @@ __device__ __forceinline__ void walk_query(const DevTree &T, const RunPool &P, i
         if (T.root == 0) {
             double4 L;
             double d2;
-            if (single_leaf_accepted<STRAT>(T, px, py, pz, K, r2a, L, d2)) ok = W.append(1u, 0, 0) && W.flush(1);
+            if (single_leaf_accepted<STRAT>(T, px, py, pz, K, r2a, L, d2)) ok = R.append(1u, 0, 0);
         } else {
             ok = W.run(px, py, pz, K, r2a);
         }
+        ok = ok && R.finish();
     }
-    const int nacc = __reduce_add_sync(0xffffffffu, W.nacc);   // at most n <= 2^30
+    const int nacc = __reduce_add_sync(0xffffffffu, R.nacc);   // at most n <= 2^30
     if (lane == 0) {
         P.qacc[j] = (unsigned)nacc;
         P.qflag[j] = ok ? 0 : 1;
         if (!P.count_only) {
-            P.items[j] = ok ? make_int2(W.first, W.nruns) : make_int2(RUN_DEFERRED, 0);
+            P.items[j] = ok ? make_int2(R.first, R.nruns) : make_int2(RUN_DEFERRED, 0);
             if (!ok) P.deferred[atomicAdd(P.n_deferred, 1u)] = qi;
         }
     }
