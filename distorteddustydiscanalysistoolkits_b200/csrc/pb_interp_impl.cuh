@@ -158,7 +158,9 @@ __device__ __forceinline__ float child_dist(const DevTree &T, const QBox &q, int
         int64_t b = id - n;
         double d2 = d2_point(px, py, pz, ldg4(T.leaf + b));
         if (d2 < best || (d2 == best && b < bi)) { best = d2; bi = b; }
-        return INFINITY;   // a leaf needs no further visit
+        // a leaf needs no further visit: NaN compares false even when the best distance is beyond
+        // FP32 and every finite or infinite bound would pass
+        return __int_as_float(0x7fffffff);
     }
     return box_lower(q, load_node(T.node + (id - 1)));
 }
