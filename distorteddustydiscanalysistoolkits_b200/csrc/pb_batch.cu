@@ -41,6 +41,7 @@ __device__ __forceinline__ int64_t count_accepted(const DevTree &T, double px, d
     return cnt;
 }
 
+constexpr int BATCH_CODE_BITS = 21;   // Morton bits of the walk order inside a disc (7 per axis)
 constexpr int BATCH_WARPS = 4;   // warps per block of the pair kernel (128 threads: the Acc32 slot layout)
 
 // processing slot of global index j: the last slot whose first index is at most j
@@ -100,22 +101,20 @@ __global__ void __launch_bounds__(128, 8) k_batch_walk(const BatchDisc *__restri
 }
 
 // Sort keys of a slice's pair order: class (FP32C points, then FP64 points, then points whose
-// runs overflowed the pool), then the disc's processing slot, then descending accepted count
-// (clipped to the count bits left after the slot's).  Grouping a class by disc keeps the
-// points that run at the same time on one disc's tree and payload, so the L2 holds one disc's
-// working set instead of all of them; heaviest first inside a disc keeps the tail short.
+// runs overflowed the pool), then the disc's processing slot, then descending size class
+// (count_class), laid out in walk order, which the stable sort keeps among equal keys.  Grouping a
+// class by disc keeps the points that run at the same time on one disc's tree and payload, so
+// the L2 holds one disc's working set instead of all of them; heaviest first inside a disc keeps
+// the tail short.
 __global__ void k_batch_keys(int64_t m, const unsigned *__restrict__ qacc, const int *__restrict__ qflag,
                              const int *__restrict__ slot_of, const uint32_t *__restrict__ order, unsigned light_max,
                              int slot_bits, uint32_t *keys, uint32_t *vals)
 {
-    const int cbits = 30 - slot_bits;
-    const unsigned cmask = cbits >= 32 ? 0xffffffffu : ((1u << cbits) - 1u);
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < m; p += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t t = order[p];   // laid out in walk order: the stable sort keeps it among equal keys
+        const int64_t t = order[p];
         const unsigned a = qacc[t];
         const unsigned cls = qflag[t] ? 2u : (a > light_max ? 0u : 1u);
-        const unsigned slot = (unsigned)slot_of[t];
-        keys[p] = (cls << 30) | (slot << cbits) | (cmask - (a > cmask ? cmask : a));
+        keys[p] = (((cls << slot_bits) | (unsigned)slot_of[t]) << 7) | (127u - count_class(a));
         vals[p] = (uint32_t)t;
     }
 }
@@ -291,12 +290,14 @@ static cudaError_t launch_walk_batch(Handle *H, const BatchDisc *discs, const in
         return e;
     uint64_t *mk = H->batch_mk.as<uint64_t>();
     uint32_t *mv = H->batch_mv.as<uint32_t>();
-    if ((e = launch_batch_query_codes(H, m, discs, starts, slot_disc, slot_of, s0, mk, mv))) return e;
-    if ((e = sort_pairs_u64(H, mk, mv, H->batch_mka.as<uint64_t>(), H->batch_mva.as<uint32_t>(), m, 32 + slot_bits)))
+    if ((e = launch_batch_query_codes(H, m, discs, starts, slot_disc, slot_of, s0, BATCH_CODE_BITS, mk, mv))) return e;
+    uint32_t *at = nullptr;
+    if ((e = sort_pairs_u64(H, mk, mv, H->batch_mka.as<uint64_t>(), H->batch_mva.as<uint32_t>(), m,
+                            BATCH_CODE_BITS + slot_bits, &at)))
         return e;
-    *worder = mv;
+    *worder = at;
     k_batch_walk<STRAT><<<persistent_blocks_of(k_batch_walk<STRAT>, 0), 128, 0, H->stream>>>(
-        discs, starts, slot_disc, slot_of, s0, m, P, mv, counter);
+        discs, starts, slot_disc, slot_of, s0, m, P, at, counter);
     H->launches += 2;
     return cudaGetLastError();
 }
@@ -357,10 +358,10 @@ cudaError_t launch_batch_slice(Handle *H, int strategy, int kernel, int cat, int
                                                           fp64_only ? 0xffffffffu : light_max, slot_bits,
                                                           H->lpt_k.as<uint32_t>(), H->lpt_v.as<uint32_t>());
     H->launches += 1;
+    uint32_t *ord = nullptr;
     if ((e = sort_pairs_u32(H, H->lpt_k.as<uint32_t>(), H->lpt_v.as<uint32_t>(), H->lpt_ka.as<uint32_t>(),
-                            H->lpt_va.as<uint32_t>(), m, 32)))
+                            H->lpt_va.as<uint32_t>(), m, 9 + slot_bits, &ord)))
         return e;
-    const uint32_t *ord = H->lpt_v.as<uint32_t>();
     unsigned *nheavy = reinterpret_cast<unsigned *>(ctr + 5);
     if ((e = launch_count_heavy(H, P, m, fp64_only ? 0xffffffffu : light_max, nheavy, ctr + 3))) return e;
     SliceOrder O{ord, slot_of, nheavy, P.n_deferred};

@@ -21,7 +21,7 @@ using namespace pb;
 pb::Handle::~Handle()
 {
     DBuf *all[] = {&in_x, &in_y, &in_z, &in_h, &in_m, &in_rho, &codes, &codes_alt, &idx, &idx_alt, &scan_tmp,
-                   &scan_part, &hist, &bbox_part, &qparams, &status, &leaf, &leaf_aux, &odd, &leaf_escape, &node, &node_hmax, &node_child, &node_range, &payload, &counter, &left,
+                   &hist, &bbox_part, &qparams, &status, &leaf, &leaf_aux, &odd, &leaf_escape, &node, &node_hmax, &node_child, &node_range, &payload, &counter, &left,
                    &right, &escape, &parent, &bmin64, &bmax64, &hmax64, &counters, &rho_s, &col_ptrs,
                    &q_x, &q_y, &q_z, &q_keys, &q_keys_alt, &q_perm, &q_perm_alt, &q_out, &q_aux,
                    &pool_runs, &pool_next, &pool_ctr, &items, &wbnear, &qacc, &qflag, &defer_a, &defer_b,
@@ -102,6 +102,7 @@ int check_status(Handle &H)
     if (st & ST_NONFINITE) return fail(H, PB_ERR_INVALID, "non-finite particle coordinate or smoothing length");
     if (st & ST_REFIT) return fail(H, PB_ERR_INTERNAL, "LBVH refit: an internal node was not combined exactly twice");
     if (st & ST_TRAVERSAL) return fail(H, PB_ERR_INTERNAL, "traversal exceeded its iteration bound");
+    if (st & ST_SORT) return fail(H, PB_ERR_INTERNAL, "radix sort: a tile waited too long for the one before it");
     if (st & ST_POOL)
         return fail(H, PB_ERR_DIMENSION, "neighbour pool offsets too small for a query (DimensionMismatch)");
     return PB_OK;
@@ -368,10 +369,15 @@ int query_order(Handle &H, int64_t nq, const double *dx, const double *dy, const
     CK(H.q_keys_alt.reserve(sizeof(uint32_t) * nq));
     CK(H.q_perm.reserve(sizeof(uint32_t) * nq));
     CK(H.q_perm_alt.reserve(sizeof(uint32_t) * nq));
-    CK(launch_query_codes(&H, nq, dx, dy, dz, H.q_keys.as<uint32_t>(), H.q_perm.as<uint32_t>()));
+    // only an order: enough Morton bits to tell the queries apart
+    int bits = 16;
+    while (bits < 30 && (int64_t(1) << bits) < 4 * nq) bits += 8;
+    if (bits > 30) bits = 30;
+    uint32_t *at = nullptr;
+    CK(launch_query_codes(&H, nq, dx, dy, dz, 30 - bits, H.q_keys.as<uint32_t>(), H.q_perm.as<uint32_t>()));
     CK(sort_pairs_u32(&H, H.q_keys.as<uint32_t>(), H.q_perm.as<uint32_t>(), H.q_keys_alt.as<uint32_t>(),
-                      H.q_perm_alt.as<uint32_t>(), nq, 30));
-    *perm = H.q_perm.as<uint32_t>();
+                      H.q_perm_alt.as<uint32_t>(), nq, bits, &at));
+    *perm = at;
     return PB_OK;
 }
 

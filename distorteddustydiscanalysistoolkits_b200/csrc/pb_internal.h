@@ -76,7 +76,7 @@ struct Handle {
 
     DBuf in_x, in_y, in_z, in_h, in_m, in_rho;    // staging for host inputs
     std::vector<DBuf> in_cols;
-    DBuf codes, codes_alt, idx, idx_alt, scan_tmp, scan_part, hist;
+    DBuf codes, codes_alt, idx, idx_alt, scan_tmp, hist;
     DBuf bbox_part, qparams, status;
     DBuf leaf, leaf_aux, odd, leaf_escape, node, node_hmax, node_child, node_range;
     DBuf payload;       // per-call FP32 particle payload of the FP32-compensated path
@@ -139,21 +139,23 @@ struct Handle {
 // ---- launchers (pb_build.cu) ----
 cudaError_t launch_bbox(Handle *H, int64_t n, const double *x, const double *y, const double *z, const double *h);
 cudaError_t launch_encode(Handle *H, int64_t n, const double *x, const double *y, const double *z);
+// stable sorts by the lowest bits; vals_at: where the sorted values are, instead of in vals (the keys
+// are then left where the last pass put them)
 cudaError_t sort_pairs_u64(Handle *H, uint64_t *keys, uint32_t *vals, uint64_t *kalt, uint32_t *valt, int64_t n,
-                           int bits);
+                           int bits, uint32_t **vals_at = nullptr);
 cudaError_t sort_pairs_u32(Handle *H, uint32_t *keys, uint32_t *vals, uint32_t *kalt, uint32_t *valt, int64_t n,
-                           int bits);
-cudaError_t launch_exclusive_scan_u32(Handle *H, const uint32_t *in, uint32_t *out, int64_t m);
-// per point t of a batch slice: key (processing slot << 32) | Morton code of the point in its
-// disc's quantisation frame, value t
+                           int bits, uint32_t **vals_at = nullptr);
+// per point t of a batch slice: key (processing slot << bits) | the highest `bits` bits of the point's
+// 30-bit Morton code in its disc's quantisation frame, value t
 cudaError_t launch_batch_query_codes(Handle *H, int64_t m, const BatchDisc *discs, const int64_t *starts,
-                                     const uint32_t *slot_disc, const int *slot_of, int64_t s0, uint64_t *keys,
-                                     uint32_t *vals);
+                                     const uint32_t *slot_disc, const int *slot_of, int64_t s0, int bits,
+                                     uint64_t *keys, uint32_t *vals);
 cudaError_t launch_dedupe(Handle *H, uint64_t *codes, int64_t n);
 cudaError_t launch_gather(Handle *H, int64_t n, const double *x, const double *y, const double *z, const double *h,
                           const double *m, const double *rho, const std::vector<const double *> &cols);
 cudaError_t launch_topology(Handle *H, int64_t n);
-cudaError_t launch_query_codes(Handle *H, int64_t nq, const double *qx, const double *qy, const double *qz,
+// 30-bit Morton codes of the sample points without their lowest `drop` bits
+cudaError_t launch_query_codes(Handle *H, int64_t nq, const double *qx, const double *qy, const double *qz, int drop,
                                uint32_t *keys, uint32_t *perm);
 cudaError_t launch_permute_back(Handle *H, int64_t n, const uint32_t *idx, const double *src, double *dst);
 
@@ -162,7 +164,6 @@ cudaError_t launch_nearest_list(Handle *H, const DevTree &T, int64_t m, const ui
                                 const double *qy, const double *qz, int *bnear);
 cudaError_t launch_walk(Handle *H, const DevTree &T, int strategy, const RunPool &P, int64_t m, const uint32_t *ql,
                         const double *qx, const double *qy, const double *qz, unsigned long long *counter);
-cudaError_t launch_lpt_order(Handle *H, const RunPool &P, int64_t m, uint32_t **order);
 cudaError_t launch_split_order(Handle *H, const RunPool &P, int64_t m, unsigned light_max, bool plain,
                                uint32_t **order, int64_t *m_heavy, int64_t *light_pairs, unsigned long long *pairs);
 cudaError_t launch_iota(Handle *H, int64_t m, uint32_t *out);
@@ -190,8 +191,8 @@ cudaError_t launch_pairs_fp32(Handle *H, const DevTree &T, const DevCatalog &C, 
 cudaError_t launch_points_fp64(Handle *H, const DevTree &T, const DevCatalog &C, int strategy, int64_t nq,
                                const double *qx, const double *qy, const double *qz, const uint32_t *perm,
                                int64_t npts);
-// queries of more than block_min accepted leaves (the first of the order, sorted by descending
-// count) are taken by whole blocks; 0xffffffff: none
+// queries of a higher size class than block_min accepted leaves (the first of the order) are taken by
+// whole blocks; 0xffffffff: none
 cudaError_t launch_pairs_fp64(Handle *H, const DevTree &T, const DevCatalog &C, int strategy, const RunPool &P,
                               int64_t m, unsigned block_min, const uint32_t *ql, const uint32_t *order,
                               const double *qx, const double *qy, const double *qz);

@@ -27,11 +27,11 @@ __global__ void __launch_bounds__(128) k_points64w(DevTree T, DevCatalog C, int6
 
 // Two-phase form: the walked queries' runs are read (deal_runs) instead of walking, with the
 // same per-slot terms and the same in-order column sums, so the values are those of k_points64w
-// bit for bit.  The queries of more than block_min leaves, which are the first of the order
-// (sorted by descending count), are taken by whole blocks (pairs64_block), the others by single
+// bit for bit.  The queries of a higher size class than block_min leaves, which are the first of
+// the order, are taken by whole blocks (pairs64_block), the others by single
 // warps once no such query is left.
-// number of queries at the front of the order (descending counts, deferred queries last) with more
-// than `above` accepted leaves: a 32-way search, the same in every warp
+// number of queries at the front of the order (descending size classes, deferred queries last) of a
+// higher class than `above` accepted leaves: a 32-way search, the same in every warp
 __device__ __forceinline__ int64_t count_above(const RunPool &P, int64_t m, const uint32_t *__restrict__ order,
                                                unsigned above, int lane)
 {
@@ -42,7 +42,7 @@ __device__ __forceinline__ int64_t count_above(const RunPool &P, int64_t m, cons
         bool more = false;
         if (t < hi) {
             const uint32_t j = __ldg(order + t);
-            more = !__ldg(P.qflag + j) && __ldg(P.qacc + j) > above;
+            more = !__ldg(P.qflag + j) && count_class(__ldg(P.qacc + j)) > count_class(above);
         }
         const int k = __popc(__ballot_sync(0xffffffffu, more));   // the first k probes are above
         if (k == 0) return lo;

@@ -330,6 +330,16 @@ __device__ __forceinline__ void deal(Slots &S, int lane, int64_t lo, int64_t hi,
     }
 }
 
+// Size class of a query of a accepted leaves, 0..124, ascending with a: the power of two and the next
+// two bits.  The pair kernels take queries by descending class, and within a class in walk (Morton)
+// order, so that queries running at the same time read the same particles.
+__device__ __forceinline__ unsigned count_class(unsigned a)
+{
+    if (a == 0) return 0u;
+    const unsigned e = 31u - (unsigned)__clz((int)a);
+    return 4u * e + (e >= 2 ? (a >> (e - 2)) & 3u : (a << (2 - e)) & 3u) + 1u;
+}
+
 // query scheduling: warps take queries in the given order from a global counter
 __device__ __forceinline__ int64_t next_query(unsigned long long *counter, int lane)
 {

@@ -42,13 +42,14 @@ __global__ void __launch_bounds__(128, 8) k_walk(DevTree T, RunPool P, int64_t m
     }
 }
 
-// descending accepted count first (deferred queries last): the heaviest queries start first
+// 8-bit pair order: the heavy queries (more than light_max accepted leaves), then the others, by
+// descending size class (count_class) in each part; deferred queries last
 __global__ void k_lpt_keys(int64_t m, const unsigned *__restrict__ qacc, const int *__restrict__ qflag,
-                           uint32_t *keys, uint32_t *vals)
+                           unsigned light_max, uint32_t *keys, uint32_t *vals)
 {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m; j += (int64_t)gridDim.x * blockDim.x) {
-        unsigned a = qflag[j] ? 0u : qacc[j];
-        keys[j] = 0x7fffffffu - (a > 0x7fffffffu ? 0x7fffffffu : a);
+        const unsigned a = qacc[j];
+        keys[j] = qflag[j] ? 255u : (a > light_max ? 127u : 255u) - count_class(a);
         vals[j] = (uint32_t)j;
     }
 }
@@ -154,24 +155,6 @@ cudaError_t launch_walk(Handle *H, const DevTree &T, int strategy, const RunPool
     return cudaGetLastError();
 }
 
-cudaError_t launch_lpt_order(Handle *H, const RunPool &P, int64_t m, uint32_t **order)
-{
-    cudaError_t e;
-    if ((e = H->lpt_k.reserve(4 * m))) return e;
-    if ((e = H->lpt_v.reserve(4 * m))) return e;
-    if ((e = H->lpt_ka.reserve(4 * m))) return e;
-    if ((e = H->lpt_va.reserve(4 * m))) return e;
-    k_lpt_keys<<<grid_for(m, 256), 256, 0, H->stream>>>(m, P.qacc, P.qflag, H->lpt_k.as<uint32_t>(),
-                                                        H->lpt_v.as<uint32_t>());
-    H->launches += 1;
-    if ((e = cudaGetLastError())) return e;
-    if ((e = sort_pairs_u32(H, H->lpt_k.as<uint32_t>(), H->lpt_v.as<uint32_t>(), H->lpt_ka.as<uint32_t>(),
-                            H->lpt_va.as<uint32_t>(), m, 31)))
-        return e;
-    *order = H->lpt_v.as<uint32_t>();
-    return cudaSuccess;
-}
-
 // pair order of a walked slice and the number of heavy queries at its front: heaviest first
 // (LPT) unless `plain`, where it is the stable heavy/light partition of the walk order; the
 // accepted pairs of the heavy and the light queries are added to pairs[0], pairs[1] (zero before);
@@ -180,22 +163,15 @@ cudaError_t launch_split_order(Handle *H, const RunPool &P, int64_t m, unsigned 
                                uint32_t **order, int64_t *m_heavy, int64_t *light_pairs, unsigned long long *pairs)
 {
     cudaError_t e;
-    if (!plain) {
-        if ((e = launch_lpt_order(H, P, m, order))) return e;
-    } else {
-        if ((e = H->lpt_k.reserve(4 * m))) return e;
-        if ((e = H->lpt_v.reserve(4 * m))) return e;
-        if ((e = H->lpt_ka.reserve(4 * m))) return e;
-        if ((e = H->lpt_va.reserve(4 * m))) return e;
-        k_heavy_keys<<<grid_for(m, 256), 256, 0, H->stream>>>(m, P.qacc, P.qflag, light_max, H->lpt_k.as<uint32_t>(),
-                                                             H->lpt_v.as<uint32_t>());
-        H->launches += 1;
-        if ((e = cudaGetLastError())) return e;
-        if ((e = sort_pairs_u32(H, H->lpt_k.as<uint32_t>(), H->lpt_v.as<uint32_t>(), H->lpt_ka.as<uint32_t>(),
-                                H->lpt_va.as<uint32_t>(), m, 1)))
-            return e;
-        *order = H->lpt_v.as<uint32_t>();
-    }
+    if ((e = H->lpt_k.reserve(4 * m)) || (e = H->lpt_v.reserve(4 * m)) || (e = H->lpt_ka.reserve(4 * m)) ||
+        (e = H->lpt_va.reserve(4 * m)))
+        return e;
+    uint32_t *k = H->lpt_k.as<uint32_t>(), *v = H->lpt_v.as<uint32_t>();
+    if (plain) k_heavy_keys<<<grid_for(m, 256), 256, 0, H->stream>>>(m, P.qacc, P.qflag, light_max, k, v);
+    else k_lpt_keys<<<grid_for(m, 256), 256, 0, H->stream>>>(m, P.qacc, P.qflag, light_max, k, v);
+    H->launches += 1;
+    if ((e = cudaGetLastError())) return e;
+    if ((e = sort_pairs_u32(H, k, v, H->lpt_ka.as<uint32_t>(), H->lpt_va.as<uint32_t>(), m, 8, order))) return e;
     unsigned *cnt = reinterpret_cast<unsigned *>(P.n_deferred) + 1;
     if ((e = cudaMemsetAsync(cnt, 0, sizeof(unsigned), H->stream))) return e;
     k_count_heavy<<<grid_for(m, 256), 256, 0, H->stream>>>(m, P.qacc, P.qflag, light_max, cnt, pairs);
