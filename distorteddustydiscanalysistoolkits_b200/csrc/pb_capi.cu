@@ -121,6 +121,8 @@ DevTree make_tree(Handle &H)
     T.aux = H.leaf_aux.as<double4>();
     T.odd = H.odd.as<int>();
     T.range = H.node_range.as<int2>();
+    T.codes = H.codes.as<uint64_t>();
+    T.qp = H.qparams.as<QuantParams>();
     T.kernel = H.kernel;
     T.status = H.status.as<int>();
     return T;
@@ -463,17 +465,16 @@ int do_build(Handle &H, const pb_input *in, int32_t flags)
     if (rc) return rc;
     H.t_build_ms = ev_ms(H, 0, 1);
     if (flags & PB_PERMUTE_CALLER) {
-        // the reference permutes the caller's columns in place (InterpolationInput.jl:211-219)
-        CK(H.q_aux.reserve(nb));
-        const double *srcs[6] = {(const double *)x, (const double *)y, (const double *)z,
-                                 (const double *)m, (const double *)h, (const double *)rho};
+        // the reference permutes the caller's columns in place (InterpolationInput.jl:211-219): the
+        // sorted values are written to the arrays the build read, which are the caller's own or, for
+        // host memory, their staged copies
+        double *dev[6] = {(double *)x, (double *)y, (double *)z, (double *)m, (double *)h, (double *)rho};
         const double *dsts[6] = {in->x, in->y, in->z, in->m, in->h, in->rho};
-        for (int a = 0; a < 6 + in->ncolumn; ++a) {
-            const double *s = a < 6 ? srcs[a] : cols[a - 6];
-            double *d = const_cast<double *>(a < 6 ? dsts[a] : in->quant[a - 6]);
-            CK(launch_permute_back(&H, n, H.idx.as<uint32_t>(), s, H.q_aux.as<double>()));
-            CK(cudaMemcpyAsync(d, H.q_aux.p, nb, cudaMemcpyDefault, H.stream));
-        }
+        CK(launch_sorted_columns(&H, n, dev));
+        for (int a = 0; a < 6; ++a)
+            if (dev[a] != dsts[a]) CK(cudaMemcpyAsync(const_cast<double *>(dsts[a]), dev[a], nb, cudaMemcpyDefault, H.stream));
+        for (int c = 0; c < in->ncolumn; ++c)
+            CK(cudaMemcpyAsync(const_cast<double *>(in->quant[c]), H.cols_s[c].p, nb, cudaMemcpyDefault, H.stream));
         CK(cudaStreamSynchronize(H.stream));
     }
     H.built = true;
@@ -617,8 +618,9 @@ bool grow_pool(Handle &H)
 
 // A query of more accepted leaves than an even share of the launch's FP64 pairs over the resident
 // warps (148 x 28), and of at least BLOCK64_MIN, is summed by a whole block: one warp would still be
-// at it when the others have finished.
-constexpr int64_t BLOCK64_SHARE = 4096, BLOCK64_MIN = 8192;
+// at it when the others have finished.  6,000 particles, 2,744 points: 0.07 ms at 1024, 0.11 at 2048, 0.16
+// at 8192.
+constexpr int64_t BLOCK64_SHARE = 4096, BLOCK64_MIN = 1024;
 
 // FP32-compensated points in two phases: the walk kernel writes every query's accepted runs,
 // the pair kernel evaluates them (once per catalog launch).  Queries go through

@@ -43,6 +43,14 @@ struct __align__(16) NodeF {
     int escape;
 };
 
+// quantisation frame of the Morton codes
+struct QuantParams {
+    double vmin[3];
+    double inv[3];
+    int flat[3];   // axis with zero extent: every particle gets f = 0.5
+    int pad;
+};
+
 struct DevTree {
     int64_t n;
     int root;
@@ -54,6 +62,8 @@ struct DevTree {
     const double4 *aux;     // {1/h, 1/rho, m, rho} of each sorted particle (reciprocals correctly rounded)
     const int *odd;         // nonzero: some particle's h or rho is outside aux_regular's range
     const int2 *range;      // 0-based sorted leaf range [lo, hi] of each internal node's subtree
+    const uint64_t *codes;  // sorted 63-bit Morton codes, and their quantisation frame
+    const QuantParams *qp;
     int kernel;
     int *status;
 };
@@ -117,6 +127,16 @@ __device__ __forceinline__ bool exp_safe(double x)
 
 // the particles the pair kernels take their short forms for (DevTree::odd is 0 if all are)
 __device__ __forceinline__ bool aux_regular(double h, double rho) { return h > 0.0 && exp_safe(h) && exp_safe(rho); }
+
+__device__ __forceinline__ uint64_t expand_bits3(uint64_t x)
+{
+    x = (x | (x << 32)) & 0x1f00000000ffffULL;
+    x = (x | (x << 16)) & 0x1f0000ff0000ffULL;
+    x = (x | (x << 8)) & 0x100f00f00f00f00fULL;
+    x = (x | (x << 4)) & 0x10c30c30c30c30c3ULL;
+    x = (x | (x << 2)) & 0x1249249249249249ULL;
+    return x;
+}
 
 __host__ __device__ inline double kernel_valid(int k) { return k == 1 ? 2.5 : (k == 2 ? 3.0 : 2.0); }
 

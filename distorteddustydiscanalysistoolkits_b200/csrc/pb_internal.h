@@ -12,8 +12,6 @@ namespace pb {
 
 // One disc of a batched launch (pb_batch.cu): its tree, the FP32C and FP64 catalogs of its
 // columns and outputs, its FP32C payload, and its sample points.
-struct QuantParams;
-
 struct BatchDisc {
     DevTree T;
     DevCatalog C32, C64;
@@ -53,13 +51,6 @@ struct DBuf {
 constexpr int SCHED_F = 16;
 constexpr int SCHED_H = 64;
 constexpr int SCHED_NPARAM = SCHED_H * SCHED_F + SCHED_H + SCHED_H * SCHED_H + SCHED_H + SCHED_H + 1;
-
-struct QuantParams {
-    double vmin[3];
-    double inv[3];
-    int flat[3];   // axis with zero extent: every particle gets f = 0.5
-    int pad;
-};
 
 struct Handle {
     int device = 0;
@@ -157,7 +148,7 @@ cudaError_t launch_topology(Handle *H, int64_t n);
 // 30-bit Morton codes of the sample points without their lowest `drop` bits
 cudaError_t launch_query_codes(Handle *H, int64_t nq, const double *qx, const double *qy, const double *qz, int drop,
                                uint32_t *keys, uint32_t *perm);
-cudaError_t launch_permute_back(Handle *H, int64_t n, const uint32_t *idx, const double *src, double *dst);
+cudaError_t launch_sorted_columns(Handle *H, int64_t n, double *const dst[6]);   // x, y, z, m, h, rho
 
 // ---- launchers (pb_walk.cu) ----
 cudaError_t launch_nearest_list(Handle *H, const DevTree &T, int64_t m, const uint32_t *ql, const double *qx,
@@ -222,6 +213,11 @@ cudaError_t launch_batch_slice(Handle *H, int strategy, int kernel, int cat, int
 cudaError_t launch_batch_payload(Handle *H, const DevTree &T, const DevCatalog &C, float4 **pay, int *stride);
 cudaError_t launch_line_image(Handle *H, const double *a0, int64_t n0, const double *a1, int64_t n1, const LineFrame &F,
                               double *ox, double *oy, double *oz, double *dx, double *dy, double *dz);
+
+// Nearest searches of at most this many points go a warp each instead of a thread each
+// (2,744 points 131 -> 20 us, 20,000 points 222 -> 95 us; 153,600 points would take 587 us, not 297: a
+// warp reads more nodes than its lanes' own searches, but waits for a quarter of the steps)
+constexpr int64_t NEAREST_WARP_MAX = 32768;
 
 inline int grid_for(int64_t n, int block, int cap = 148 * 32)
 {

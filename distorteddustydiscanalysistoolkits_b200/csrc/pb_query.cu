@@ -20,6 +20,21 @@ __global__ void k_nearest(DevTree T, int64_t nq, const double *__restrict__ qx, 
     }
 }
 
+__global__ void __launch_bounds__(128) k_nearest_warp(DevTree T, int64_t nq, const double *__restrict__ qx,
+                                                      const double *__restrict__ qy, const double *__restrict__ qz,
+                                                      double *h_out, int64_t *idx_out)
+{
+    __shared__ int s_stack[4][WSTACK];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    for (int64_t i = blockIdx.x * (int64_t)4 + wib; i < nq; i += (int64_t)gridDim.x * 4) {
+        const int64_t b = nearest_leaf_warp(T, __ldg(qx + i), __ldg(qy + i), __ldg(qz + i), s_stack[wib], lane);
+        if (lane == 0) {
+            if (h_out) h_out[i] = b < 0 ? __longlong_as_double(0x7ff8000000000000LL) : T.leaf[b].w;
+            if (idx_out) idx_out[i] = b;
+        }
+    }
+}
+
 // A query's accepted leaves, counted and (with a pool) listed in DFS order; a list longer than its
 // `cap` flags ST_POOL and is cut there.
 struct ListSink {
@@ -84,17 +99,36 @@ __global__ void __launch_bounds__(128, 8) k_query(DevTree T, int64_t nq, const d
 // the closest accepted leaf of a query: the nearest leaf of all, if it lies within the radius.  It is the
 // first strictly closer one in DFS order (LinearBVHQueries.jl:33-39,196-203): nearest[i] its index (-1
 // if none), nearest_d2[i] its squared distance (+Inf if none).
+__device__ __forceinline__ void store_closest(const DevTree &T, int64_t i, int64_t b, double px, double py, double pz,
+                                              double r, int64_t *nearest, double *nearest_d2)
+{
+    const double d2 = b < 0 ? INFINITY : d2_point(px, py, pz, ldg4(T.leaf + b));
+    const bool in = d2 <= __dmul_rn(r, r) && d2 < INFINITY;
+    if (nearest) nearest[i] = in ? b : -1;
+    if (nearest_d2) nearest_d2[i] = in ? d2 : INFINITY;
+}
+
 __global__ void __launch_bounds__(128) k_closest(DevTree T, int64_t nq, const double *__restrict__ qx,
                                                  const double *__restrict__ qy, const double *__restrict__ qz,
                                                  const double *__restrict__ radius, int64_t *nearest, double *nearest_d2)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nq; i += (int64_t)gridDim.x * blockDim.x) {
-        const double px = __ldg(qx + i), py = __ldg(qy + i), pz = __ldg(qz + i), r = __ldg(radius + i);
-        const int64_t b = nearest_leaf(T, px, py, pz);
-        const double d2 = b < 0 ? INFINITY : d2_point(px, py, pz, ldg4(T.leaf + b));
-        const bool in = d2 <= __dmul_rn(r, r) && d2 < INFINITY;
-        if (nearest) nearest[i] = in ? b : -1;
-        if (nearest_d2) nearest_d2[i] = in ? d2 : INFINITY;
+        const double px = __ldg(qx + i), py = __ldg(qy + i), pz = __ldg(qz + i);
+        store_closest(T, i, nearest_leaf(T, px, py, pz), px, py, pz, __ldg(radius + i), nearest, nearest_d2);
+    }
+}
+
+__global__ void __launch_bounds__(128) k_closest_warp(DevTree T, int64_t nq, const double *__restrict__ qx,
+                                                      const double *__restrict__ qy, const double *__restrict__ qz,
+                                                      const double *__restrict__ radius, int64_t *nearest,
+                                                      double *nearest_d2)
+{
+    __shared__ int s_stack[4][WSTACK];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    for (int64_t i = blockIdx.x * (int64_t)4 + wib; i < nq; i += (int64_t)gridDim.x * 4) {
+        const double px = __ldg(qx + i), py = __ldg(qy + i), pz = __ldg(qz + i);
+        const int64_t b = nearest_leaf_warp(T, px, py, pz, s_stack[wib], lane);
+        if (lane == 0) store_closest(T, i, b, px, py, pz, __ldg(radius + i), nearest, nearest_d2);
     }
 }
 
@@ -197,7 +231,9 @@ cudaError_t launch_stats(Handle *H, const DevTree &T, int strategy, int64_t nq, 
 cudaError_t launch_nearest(Handle *H, const DevTree &T, int64_t nq, const double *qx, const double *qy,
                            const double *qz, double *h_out, int64_t *idx_out)
 {
-    k_nearest<<<grid_for(nq, 128, 1 << 30), 128, 0, H->stream>>>(T, nq, qx, qy, qz, h_out, idx_out);
+    if (nq <= NEAREST_WARP_MAX)
+        k_nearest_warp<<<grid_for(nq, 4, 1 << 30), 128, 0, H->stream>>>(T, nq, qx, qy, qz, h_out, idx_out);
+    else k_nearest<<<grid_for(nq, 128, 1 << 30), 128, 0, H->stream>>>(T, nq, qx, qy, qz, h_out, idx_out);
     H->launches += 1;
     return cudaGetLastError();
 }
@@ -215,7 +251,9 @@ cudaError_t launch_query(Handle *H, const DevTree &T, int64_t nq, const double *
         H->launches += 1;
     }
     if (nearest || nearest_d2) {
-        k_closest<<<grid_for(nq, 128, 1 << 30), 128, 0, H->stream>>>(T, nq, qx, qy, qz, radius, nearest, nearest_d2);
+        if (nq <= NEAREST_WARP_MAX)
+            k_closest_warp<<<grid_for(nq, 4, 1 << 30), 128, 0, H->stream>>>(T, nq, qx, qy, qz, radius, nearest, nearest_d2);
+        else k_closest<<<grid_for(nq, 128, 1 << 30), 128, 0, H->stream>>>(T, nq, qx, qy, qz, radius, nearest, nearest_d2);
         H->launches += 1;
     }
     return cudaGetLastError();

@@ -19,6 +19,20 @@ __global__ void __launch_bounds__(128) k_nearest_list(DevTree T, int64_t m, cons
     }
 }
 
+// few queries: a warp each (nearest_leaf_warp)
+__global__ void __launch_bounds__(128) k_nearest_list_warp(DevTree T, int64_t m, const uint32_t *__restrict__ ql,
+                                                           const double *__restrict__ qx, const double *__restrict__ qy,
+                                                           const double *__restrict__ qz, int *bnear)
+{
+    __shared__ int s_stack[4][WSTACK];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    for (int64_t j = blockIdx.x * (int64_t)4 + wib; j < m; j += (int64_t)gridDim.x * 4) {
+        const uint32_t qi = __ldg(ql + j);
+        const int64_t b = nearest_leaf_warp(T, __ldg(qx + qi), __ldg(qy + qi), __ldg(qz + qi), s_stack[wib], lane);
+        if (lane == 0) bnear[j] = (int)b;
+    }
+}
+
 // A warp takes WALK_TICKET queries at a time from the queue (one counter for millions of short
 // walks would be the bottleneck).
 constexpr int WALK_TICKET = 4;
@@ -125,7 +139,9 @@ static int persistent_blocks(const void *kern, int bs)
 cudaError_t launch_nearest_list(Handle *H, const DevTree &T, int64_t m, const uint32_t *ql, const double *qx,
                                 const double *qy, const double *qz, int *bnear)
 {
-    k_nearest_list<<<grid_for(m, 128, 1 << 30), 128, 0, H->stream>>>(T, m, ql, qx, qy, qz, bnear);
+    if (m <= NEAREST_WARP_MAX)
+        k_nearest_list_warp<<<grid_for(m, 4, 1 << 30), 128, 0, H->stream>>>(T, m, ql, qx, qy, qz, bnear);
+    else k_nearest_list<<<grid_for(m, 128, 1 << 30), 128, 0, H->stream>>>(T, m, ql, qx, qy, qz, bnear);
     H->launches += 1;
     return cudaGetLastError();
 }

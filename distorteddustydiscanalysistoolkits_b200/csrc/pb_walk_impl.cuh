@@ -225,6 +225,98 @@ struct WarpWalk {
     }
 };
 
+// nearest_leaf by a warp: the 32 leaves around the point's place in the Morton order give a first
+// distance, then the lanes take 32 tree entries a round and keep those that may hold a leaf at most
+// that far.  The result is nearest_leaf's: the least squared distance and, among equal ones, the
+// smallest sorted index.  Every lane of the warp calls it; smem holds WSTACK ints.
+__device__ __forceinline__ int64_t nearest_leaf_warp(const DevTree &T, double px, double py, double pz, int *stack,
+                                                     int lane)
+{
+    const int n = (int)T.n;
+    double best = INFINITY;
+    int bi = -1;
+    // the warp's least (d2, index) over its lanes' candidates and the best so far
+    auto take = [&](double d2, int b) {
+        if (!__any_sync(0xffffffffu, d2 < best || (d2 == best && b < bi))) return;
+        if (!(d2 < best || (d2 == best && b < bi))) { d2 = best; b = bi; }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double v = __shfl_xor_sync(0xffffffffu, d2, o);
+            const int vb = __shfl_xor_sync(0xffffffffu, b, o);
+            if (v < d2 || (v == d2 && vb < b)) { d2 = v; b = vb; }
+        }
+        best = d2;
+        bi = b;
+    };
+    if (T.root == 0) {
+        take(lane == 0 ? d2_point(px, py, pz, ldg4(T.leaf)) : INFINITY, 0);
+        return bi;
+    }
+    uint64_t code = 0;
+    {
+        const double p[3] = {px, py, pz};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double f = T.qp->flat[d] ? 0.5 : (p[d] - T.qp->vmin[d]) * T.qp->inv[d];
+            const uint64_t c = f > 0.0 ? (uint64_t)(fmin(f, 1.0) * 2097151.0) : 0;   // NaN: 0
+            code |= expand_bits3(c) << (2 - d);
+        }
+    }
+    int lo = 0, hi = n;
+    while (hi - lo > 32) {
+        const int step = (hi - lo + 31) / 32, t = lo + lane * step;
+        const int k = __popc(__ballot_sync(0xffffffffu, t < hi && __ldg(T.codes + t) < code));
+        hi = min(hi, lo + max(k, 1) * step);
+        lo = lo + (k > 0 ? (k - 1) * step : 0);
+    }
+    {
+        const int b = max(0, min((lo + hi) / 2 - 16, n - 32)) + lane;
+        take(b < n ? d2_point(px, py, pz, ldg4(T.leaf + b)) : INFINITY, b);
+    }
+    const QBox q = make_qbox(px, py, pz);
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned limit = 2u * (unsigned)n + 64u;
+    unsigned guard = 0;
+    int size = 1;
+    __syncwarp();
+    if (lane == 0) stack[0] = T.root;
+    __syncwarp();
+    while (size > 0) {
+        if (++guard > limit || size > WSTACK - 2) {
+            flag(T.status, ST_TRAVERSAL);
+            break;
+        }
+        const int k = size > WSTACK - 160 ? 1 : (size < 32 ? size : 32);
+        // a subtree is skipped only when its lower bound exceeds the best distance by the margin
+        const float lim = __fmul_ru(__double2float_ru(best), MARGIN_UP);
+        int e0 = 0, e1 = 0, b = -1;
+        bool open = false;
+        if (lane < k) {
+            const int e = stack[size - 1 - lane];
+            if (e >= n) {
+                b = e - n;
+            } else {
+                const NodeF nd = load_node(T.node + (e - 1));
+                open = !(box_lower(q, nd) > lim);
+                const int2 rg = __ldg(T.range + (e - 1));
+                e0 = nd.left;
+                const int split = nd.left >= n ? nd.left - (n - 1) : nd.left;   // 1-based
+                e1 = split == rg.y ? n + rg.y : split + 1;
+            }
+        }
+        take(b >= 0 ? d2_point(px, py, pz, ldg4(T.leaf + b)) : INFINITY, b >= 0 ? b : n);
+        const unsigned o = __ballot_sync(0xffffffffu, open);
+        size += 2 * __popc(o) - k;
+        if (open) {
+            const int at = size - 1 - 2 * __popc(o & below);
+            stack[at] = e0;
+            stack[at - 1] = e1;
+        }
+        __syncwarp();
+    }
+    return bi;
+}
+
 // The walk of the j-th listed query (sample point qi at px, py, pz; nearest sorted leaf P.bnear[j]):
 // its run list, its number of accepted leaves, and whether the pool was full (the query is then
 // listed as deferred).  Every lane of the warp calls it; smem holds RUN_WALK_SMEM ints.
