@@ -540,9 +540,10 @@ cudaError_t launch_gather(Handle *H, int64_t n, const double *x, const double *y
     return cudaGetLastError();
 }
 
-// the sorted x, y, z, m, h, rho as six columns (the caller's arrays are put into Morton order)
+// the sorted x, y, z, m, h, rho as six columns, and the sorted quantity columns (the caller's arrays are
+// put into Morton order)
 __global__ void k_sorted_columns(int64_t n, const double4 *__restrict__ leaf, const double4 *__restrict__ aux, double *x,
-                                 double *y, double *z, double *m, double *h, double *rho)
+                                 double *y, double *z, double *m, double *h, double *rho, GatherCols cols)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double4 L = ldg4(leaf + i), X = ldg4(aux + i);
@@ -552,13 +553,25 @@ __global__ void k_sorted_columns(int64_t n, const double4 *__restrict__ leaf, co
         m[i] = X.z;
         h[i] = L.w;
         rho[i] = X.w;
+        for (int c = 0; c < cols.n; ++c) cols.dst[c][i] = cols.src[c][i];
     }
 }
 
-cudaError_t launch_sorted_columns(Handle *H, int64_t n, double *const dst[6])
+cudaError_t launch_sorted_columns(Handle *H, int64_t n, double *const dst[6], const std::vector<double *> &cols)
 {
+    GatherCols G{};
+    for (size_t c = 0; c < cols.size(); ++c) {
+        if (c >= GATHER_COLS) {
+            cudaError_t e = cudaMemcpyAsync(cols[c], H->cols_s[c].p, sizeof(double) * n, cudaMemcpyDeviceToDevice, H->stream);
+            if (e) return e;
+            continue;
+        }
+        G.src[c] = H->cols_s[c].as<double>();
+        G.dst[c] = cols[c];
+        G.n = (int)c + 1;
+    }
     k_sorted_columns<<<grid_for(n, 256), 256, 0, H->stream>>>(n, H->leaf.as<double4>(), H->leaf_aux.as<double4>(), dst[0],
-                                                              dst[1], dst[2], dst[3], dst[4], dst[5]);
+                                                              dst[1], dst[2], dst[3], dst[4], dst[5], G);
     H->launches += 1;
     return cudaGetLastError();
 }

@@ -36,6 +36,8 @@ pb::Handle::~Handle()
                     &batch_mva})
         b->release();
     if (batch_host) cudaFreeHost(batch_host);
+    if (pin) cudaFreeHost(pin);
+    for (DBuf *b : {&in_pack, &q_pack, &out_pack}) b->release();
     for (auto &b : in_cols) b.release();
     for (auto &b : cols_s) b.release();
     for (auto &b : q_outs) b.release();
@@ -94,11 +96,46 @@ cudaError_t stage_in(Handle &H, DBuf &buf, const void *p, size_t bytes, const vo
     return e;
 }
 
+// Page-locked staging of a handle: PIN_WORDS bytes for words that the host reads back, then PIN_MAX
+// bytes through which small host arrays travel packed, in one copy instead of one per array (a copy
+// from or to pageable memory costs 5 to 12 us of host time each: 39 of them were 1 ms of a call on
+// 6,000 particles and 2,744 points).  Every use ends in the call's own synchronisation, and calls on a
+// handle do not overlap.
+constexpr size_t PIN_WORDS = 256, PIN_MAX = size_t(2) << 20;
+
+cudaError_t pin_reserve(Handle &H)
+{
+    return H.pin ? cudaSuccess : cudaMallocHost(reinterpret_cast<void **>(&H.pin), PIN_WORDS + PIN_MAX);
+}
+
+// whether k arrays of `bytes` each go packed: all in host memory, and small
+bool packs(const Handle &H, const void *const *p, int k, size_t bytes)
+{
+    if (bytes * (size_t)k > PIN_MAX) return false;
+    for (int i = 0; i < k; ++i)
+        if (!p[i] || ptr_place(H, p[i]) != 0) return false;
+    return true;
+}
+
+// device views of k host arrays through one packed copy
+cudaError_t pack_in(Handle &H, DBuf &buf, const void *const *p, int k, size_t bytes, const void **out)
+{
+    cudaError_t e;
+    if ((e = pin_reserve(H)) || (e = buf.reserve(bytes * k))) return e;
+    for (int i = 0; i < k; ++i) {
+        memcpy(H.pin + PIN_WORDS + i * bytes, p[i], bytes);
+        out[i] = buf.as<unsigned char>() + i * bytes;
+    }
+    return cudaMemcpyAsync(buf.p, H.pin + PIN_WORDS, bytes * k, cudaMemcpyHostToDevice, H.stream);
+}
+
 int check_status(Handle &H)
 {
-    int st = 0;
-    CK(cudaMemcpyAsync(&st, H.status.p, sizeof(int), cudaMemcpyDeviceToHost, H.stream));
+    CK(pin_reserve(H));
+    volatile int *word = reinterpret_cast<volatile int *>(H.pin);
+    CK(cudaMemcpyAsync(H.pin, H.status.p, sizeof(int), cudaMemcpyDeviceToHost, H.stream));
     CK(cudaStreamSynchronize(H.stream));
+    const int st = *word;
     if (st & ST_NONFINITE) return fail(H, PB_ERR_INVALID, "non-finite particle coordinate or smoothing length");
     if (st & ST_REFIT) return fail(H, PB_ERR_INTERNAL, "LBVH refit: an internal node was not combined exactly twice");
     if (st & ST_TRAVERSAL) return fail(H, PB_ERR_INTERNAL, "traversal exceeded its iteration bound");
@@ -321,19 +358,28 @@ DevCatalog dev_catalog(Handle &H, const Launch &L, double *const *outs)
 
 int64_t catalog_L(const pb_catalog *c) { return c->n_scalar + 3 * c->n_grad + c->n_div + 3 * c->n_curl; }
 
-// stage output pointers: device outputs are written in place, host outputs via staging
+// stage output pointers: device outputs are written in place, host outputs via staging (contiguous if
+// they are small and all in host memory: they then come back in one copy)
 int stage_outputs(Handle &H, int64_t L, int64_t npts, double *const *out, std::vector<double *> &dev,
                   std::vector<int> &is_host)
 {
     dev.assign(L, nullptr);
     is_host.assign(L, 0);
     if ((int64_t)H.q_outs.size() < L) H.q_outs.resize(L);
+    const size_t nb = sizeof(double) * npts;
+    if (out && L <= 1024 && packs(H, reinterpret_cast<const void *const *>(out), (int)L, nb)) {
+        CK(pin_reserve(H));
+        CK(H.out_pack.reserve(nb * L));
+        for (int64_t l = 0; l < L; ++l) dev[l] = H.out_pack.as<double>() + l * npts;
+        is_host.assign(L, 2);
+        return PB_OK;
+    }
     for (int64_t l = 0; l < L; ++l) {
         if (!out || !out[l]) return fail(H, PB_ERR_INVALID, "output pointer is NULL");
         if (ptr_place(H, out[l]) == 2) return fail(H, PB_ERR_INVALID, "output is device memory of another GPU");
         if (is_device_ptr(H, out[l])) dev[l] = out[l];
         else {
-            CK(H.q_outs[l].reserve(sizeof(double) * npts));
+            CK(H.q_outs[l].reserve(nb));
             dev[l] = H.q_outs[l].as<double>();
             is_host[l] = 1;
         }
@@ -344,21 +390,32 @@ int stage_outputs(Handle &H, int64_t L, int64_t npts, double *const *out, std::v
 int finish_outputs(Handle &H, int64_t L, int64_t npts, double *const *out, const std::vector<double *> &dev,
                    const std::vector<int> &is_host)
 {
+    const size_t nb = sizeof(double) * npts;
+    if (is_host[0] == 2) {
+        CK(cudaMemcpyAsync(H.pin + PIN_WORDS, H.out_pack.p, nb * L, cudaMemcpyDeviceToHost, H.stream));
+        const int rc = check_status(H);   // waits
+        for (int64_t l = 0; l < L; ++l) memcpy(out[l], H.pin + PIN_WORDS + l * nb, nb);
+        return rc;
+    }
     for (int64_t l = 0; l < L; ++l)
-        if (is_host[l]) CK(cudaMemcpyAsync(out[l], dev[l], sizeof(double) * npts, cudaMemcpyDeviceToHost, H.stream));
+        if (is_host[l]) CK(cudaMemcpyAsync(out[l], dev[l], nb, cudaMemcpyDeviceToHost, H.stream));
     return check_status(H);
 }
 
 int stage_queries(Handle &H, int64_t nq, const double *qx, const double *qy, const double *qz, const double **dx,
                   const double **dy, const double **dz)
 {
-    const void *a, *b, *c;
-    CK(stage_in(H, H.q_x, qx, sizeof(double) * nq, &a));
-    CK(stage_in(H, H.q_y, qy, sizeof(double) * nq, &b));
-    CK(stage_in(H, H.q_z, qz, sizeof(double) * nq, &c));
-    *dx = (const double *)a;
-    *dy = (const double *)b;
-    *dz = (const double *)c;
+    const void *src[3] = {qx, qy, qz}, *d[3];
+    if (packs(H, src, 3, sizeof(double) * nq)) {
+        CK(pack_in(H, H.q_pack, src, 3, sizeof(double) * nq, d));
+    } else {
+        CK(stage_in(H, H.q_x, qx, sizeof(double) * nq, &d[0]));
+        CK(stage_in(H, H.q_y, qy, sizeof(double) * nq, &d[1]));
+        CK(stage_in(H, H.q_z, qz, sizeof(double) * nq, &d[2]));
+    }
+    *dx = (const double *)d[0];
+    *dy = (const double *)d[1];
+    *dz = (const double *)d[2];
     return PB_OK;
 }
 
@@ -400,20 +457,24 @@ int do_build(Handle &H, const pb_input *in, int32_t flags)
     CK(cudaSetDevice(H.device));
     H.built = false;
     const size_t nb = sizeof(double) * n;
-    const void *x, *y, *z, *h, *m, *rho;
-    CK(stage_in(H, H.in_x, in->x, nb, &x));
-    CK(stage_in(H, H.in_y, in->y, nb, &y));
-    CK(stage_in(H, H.in_z, in->z, nb, &z));
-    CK(stage_in(H, H.in_h, in->h, nb, &h));
-    CK(stage_in(H, H.in_m, in->m, nb, &m));
-    CK(stage_in(H, H.in_rho, in->rho, nb, &rho));
-    if ((int)H.in_cols.size() < in->ncolumn) H.in_cols.resize(in->ncolumn);
-    if ((int)H.cols_s.size() < in->ncolumn) H.cols_s.resize(in->ncolumn);
-    std::vector<const double *> cols(in->ncolumn);
-    for (int c = 0; c < in->ncolumn; ++c) {
-        const void *p;
-        CK(stage_in(H, H.in_cols[c], in->quant[c], nb, &p));
-        cols[c] = (const double *)p;
+    const int ncol = in->ncolumn;
+    if ((int)H.in_cols.size() < ncol) H.in_cols.resize(ncol);
+    if ((int)H.cols_s.size() < ncol) H.cols_s.resize(ncol);
+    // x, y, z, h, m, rho and the quantity columns
+    std::vector<const void *> src = {in->x, in->y, in->z, in->h, in->m, in->rho}, at(6 + ncol);
+    for (int c = 0; c < ncol; ++c) src.push_back(in->quant[c]);
+    // an asynchronous build returns before its copies are done: no packing then
+    const bool packed = !(flags & PB_BUILD_ASYNC) && packs(H, src.data(), 6 + ncol, nb);
+    if (packed) {
+        CK(pack_in(H, H.in_pack, src.data(), 6 + ncol, nb, at.data()));
+    } else {
+        DBuf *bufs[6] = {&H.in_x, &H.in_y, &H.in_z, &H.in_h, &H.in_m, &H.in_rho};
+        for (int a = 0; a < 6 + ncol; ++a) CK(stage_in(H, a < 6 ? *bufs[a] : H.in_cols[a - 6], src[a], nb, &at[a]));
+    }
+    const void *x = at[0], *y = at[1], *z = at[2], *h = at[3], *m = at[4], *rho = at[5];
+    std::vector<const double *> cols(ncol);
+    for (int c = 0; c < ncol; ++c) {
+        cols[c] = (const double *)at[6 + c];
         CK(H.cols_s[c].reserve(nb));
     }
     int64_t nin = n > 1 ? n - 1 : 1, ntot = 2 * n - 1;
@@ -461,20 +522,26 @@ int do_build(Handle &H, const pb_input *in, int32_t flags)
         H.built = true;
         return PB_OK;
     }
+    // the reference permutes the caller's columns in place (InterpolationInput.jl:211-219): the sorted
+    // values are written to the arrays the build read, which are the caller's own or, for host
+    // memory, their staged copies
+    double *dev[6] = {(double *)x, (double *)y, (double *)z, (double *)m, (double *)h, (double *)rho};
+    std::vector<double *> dcol(ncol);
+    for (int c = 0; c < ncol; ++c) dcol[c] = const_cast<double *>(cols[c]);
+    const bool permute = flags & PB_PERMUTE_CALLER;
+    if (permute && packed) {   // back in one copy; the caller's arrays are written if the build succeeded
+        CK(launch_sorted_columns(&H, n, dev, dcol));
+        CK(cudaMemcpyAsync(H.pin + PIN_WORDS, H.in_pack.p, nb * (6 + ncol), cudaMemcpyDeviceToHost, H.stream));
+    }
     int rc = check_status(H);
     if (rc) return rc;
     H.t_build_ms = ev_ms(H, 0, 1);
-    if (flags & PB_PERMUTE_CALLER) {
-        // the reference permutes the caller's columns in place (InterpolationInput.jl:211-219): the
-        // sorted values are written to the arrays the build read, which are the caller's own or, for
-        // host memory, their staged copies
-        double *dev[6] = {(double *)x, (double *)y, (double *)z, (double *)m, (double *)h, (double *)rho};
-        const double *dsts[6] = {in->x, in->y, in->z, in->m, in->h, in->rho};
-        CK(launch_sorted_columns(&H, n, dev));
-        for (int a = 0; a < 6; ++a)
-            if (dev[a] != dsts[a]) CK(cudaMemcpyAsync(const_cast<double *>(dsts[a]), dev[a], nb, cudaMemcpyDefault, H.stream));
-        for (int c = 0; c < in->ncolumn; ++c)
-            CK(cudaMemcpyAsync(const_cast<double *>(in->quant[c]), H.cols_s[c].p, nb, cudaMemcpyDefault, H.stream));
+    if (permute && packed) {
+        for (int a = 0; a < 6 + ncol; ++a) memcpy(const_cast<void *>(src[a]), H.pin + PIN_WORDS + a * nb, nb);
+    } else if (permute) {
+        CK(launch_sorted_columns(&H, n, dev, dcol));
+        for (int a = 0; a < 6 + ncol; ++a)
+            if (at[a] != src[a]) CK(cudaMemcpyAsync(const_cast<void *>(src[a]), at[a], nb, cudaMemcpyDefault, H.stream));
         CK(cudaStreamSynchronize(H.stream));
     }
     H.built = true;
@@ -496,8 +563,12 @@ int reserve_pool(Handle &H, int64_t m)
     const char *env = getenv("PB_RUN_POOL_MB");
     const char *envc = getenv("PB_RUN_POOL_CHUNKS");
     long long env_mb = env ? atoll(env) : 0, env_chunks = envc ? atoll(envc) : 0;
+    // a pool an earlier call grew (grow_pool) is kept: its memory is already held
+    const unsigned long long held = std::min<unsigned long long>(H.pool_runs.bytes / (sizeof(uint2) * RUN_CHUNK),
+                                                                 H.pool_next.bytes / sizeof(int));
     unsigned long long budget;
     if (env_mb > 0) budget = (unsigned long long)env_mb << 20;
+    else if (held >= want) budget = held * per_chunk;   // enough: no need to ask for the free memory
     else {
         // half of the free memory plus what the pool already holds, at most 64 GiB
         size_t fr = 0, tot = 0;
@@ -508,9 +579,6 @@ int reserve_pool(Handle &H, int64_t m)
     unsigned long long cap = budget / per_chunk;
     if (cap > want) cap = want;
     if (env_mb <= 0 && cap < min_chunks) cap = min_chunks;
-    // a pool an earlier call grew (grow_pool) is kept: its memory is already held
-    const unsigned long long held = std::min<unsigned long long>(H.pool_runs.bytes / (sizeof(uint2) * RUN_CHUNK),
-                                                                 H.pool_next.bytes / sizeof(int));
     if (env_mb <= 0 && held > cap) cap = held;
     if (env_chunks > 0) cap = (unsigned long long)env_chunks;
     if (cap < 1) cap = 1;
@@ -714,9 +782,15 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
             CK(launch_walk(&H, T, strategy, P, m, ql, dx, dy, dz, ctr + 2));
             H.interp_launches++;
             uint32_t *order = nullptr;
-            int64_t m_heavy = 0;
-            int64_t light_pairs = 0;
-            CK(launch_split_order(&H, P, m, (unsigned)H.light_max, mode == 0, &order, &m_heavy, &light_pairs, ctr + 4));
+            CK(launch_split_order(&H, P, m, (unsigned)H.light_max, mode == 0, &order, ctr + 4));
+            // the pool use, the deferred and the heavy queries and the pairs are final here
+            CK(pin_reserve(H));
+            CK(cudaMemcpyAsync(H.pin, ctr, 6 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, H.stream));
+            CK(cudaStreamSynchronize(H.stream));
+            unsigned long long used_nd[6];
+            memcpy(used_nd, H.pin, sizeof(used_nd));
+            const unsigned nd = (unsigned)(used_nd[1] & 0xffffffffULL);
+            const int64_t m_heavy = (int64_t)(used_nd[1] >> 32), light_pairs = (int64_t)used_nd[5];
             // the plain order is not sorted: no block queries there
             const unsigned block_min =
                 mode == 0 ? 0xffffffffu
@@ -735,10 +809,9 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
                     H.interp_launches++;
                 }
             ev_record(H, 7);
-            unsigned long long used_nd[6] = {0, 0, 0, 0, 0, 0};
-            CK(cudaMemcpyAsync(used_nd, ctr, 6 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, H.stream));
-            CK(cudaStreamSynchronize(H.stream));
-            const unsigned nd = (unsigned)(used_nd[1] & 0xffffffffULL);
+            // the sums are waited for only where the host needs them done: to time the phases, or before
+            // the pool may be given back
+            if (H.timing || nd > 0) CK(cudaStreamSynchronize(H.stream));
             H.split_hq += m_heavy;
             H.split_lq += m - (int64_t)nd - m_heavy;
             H.split_hp += (int64_t)used_nd[4];
@@ -849,23 +922,27 @@ int do_lines(Handle &H, const pb_catalog *cat, int64_t nl, const double *ox, con
     if (!ox || !oy || !oz || !mx || !my || !mz) return fail(H, PB_ERR_INVALID, "line pointer is NULL");
     CK(cudaSetDevice(H.device));
     CK(cudaMemsetAsync(H.status.p, 0, sizeof(int), H.stream));
-    const double *dox, *doy, *doz;
-    if ((rc = stage_queries(H, nl, ox, oy, oz, &dox, &doy, &doz))) return rc;
-    const void *a, *b, *c;
-    CK(H.q_out.reserve(sizeof(double) * 3 * nl));
-    // directions: device views or staged into q_out (3 * nl doubles)
-    double *stage = H.q_out.as<double>();
-    const double *dirs[3] = {mx, my, mz};
-    const void *dv[3];
-    for (int d = 0; d < 3; ++d) {
-        if (ptr_place(H, dirs[d]) == 2) return fail(H, PB_ERR_INVALID, "direction is device memory of another GPU");
-        if (is_device_ptr(H, dirs[d])) dv[d] = dirs[d];
-        else {
-            CK(cudaMemcpyAsync(stage + d * nl, dirs[d], sizeof(double) * nl, cudaMemcpyHostToDevice, H.stream));
-            dv[d] = stage + d * nl;
+    // origins and directions: device views, one packed copy, or staged (directions in q_out)
+    const void *src[6] = {ox, oy, oz, mx, my, mz}, *at[6];
+    if (packs(H, src, 6, sizeof(double) * nl)) {
+        CK(pack_in(H, H.q_pack, src, 6, sizeof(double) * nl, at));
+    } else {
+        const double *d[3];
+        if ((rc = stage_queries(H, nl, ox, oy, oz, &d[0], &d[1], &d[2]))) return rc;
+        CK(H.q_out.reserve(sizeof(double) * 3 * nl));
+        double *stage = H.q_out.as<double>();
+        for (int k = 0; k < 3; ++k) {
+            at[k] = d[k];
+            if (ptr_place(H, src[3 + k]) == 2) return fail(H, PB_ERR_INVALID, "direction is device memory of another GPU");
+            if (is_device_ptr(H, src[3 + k])) at[3 + k] = src[3 + k];
+            else {
+                CK(cudaMemcpyAsync(stage + k * nl, src[3 + k], sizeof(double) * nl, cudaMemcpyHostToDevice, H.stream));
+                at[3 + k] = stage + k * nl;
+            }
         }
     }
-    a = dv[0]; b = dv[1]; c = dv[2];
+    const double *dox = (const double *)at[0], *doy = (const double *)at[1], *doz = (const double *)at[2];
+    const void *a = at[3], *b = at[4], *c = at[5];
     std::vector<double *> dev;
     std::vector<int> is_host;
     if ((rc = stage_outputs(H, L, nl, out, dev, is_host))) return rc;

@@ -111,6 +111,10 @@ struct Handle {
     DBuf batch_slot_of;      // processing slot of every point of a slice
     DBuf batch_mk, batch_mka, batch_mv, batch_mva;         // Morton walk order of a slice
 
+    // page-locked staging: words the host reads back, and small host arrays packed into one copy
+    unsigned char *pin = nullptr;
+    DBuf in_pack, q_pack, out_pack;
+
     // query-side scratch
     DBuf q_x, q_y, q_z, q_keys, q_keys_alt, q_perm, q_perm_alt, q_out, q_aux;
     std::vector<DBuf> q_outs;
@@ -148,7 +152,8 @@ cudaError_t launch_topology(Handle *H, int64_t n);
 // 30-bit Morton codes of the sample points without their lowest `drop` bits
 cudaError_t launch_query_codes(Handle *H, int64_t nq, const double *qx, const double *qy, const double *qz, int drop,
                                uint32_t *keys, uint32_t *perm);
-cudaError_t launch_sorted_columns(Handle *H, int64_t n, double *const dst[6]);   // x, y, z, m, h, rho
+// the sorted x, y, z, m, h, rho and quantity columns to device arrays
+cudaError_t launch_sorted_columns(Handle *H, int64_t n, double *const dst[6], const std::vector<double *> &cols);
 
 // ---- launchers (pb_walk.cu) ----
 cudaError_t launch_nearest_list(Handle *H, const DevTree &T, int64_t m, const uint32_t *ql, const double *qx,
@@ -156,7 +161,7 @@ cudaError_t launch_nearest_list(Handle *H, const DevTree &T, int64_t m, const ui
 cudaError_t launch_walk(Handle *H, const DevTree &T, int strategy, const RunPool &P, int64_t m, const uint32_t *ql,
                         const double *qx, const double *qy, const double *qz, unsigned long long *counter);
 cudaError_t launch_split_order(Handle *H, const RunPool &P, int64_t m, unsigned light_max, bool plain,
-                               uint32_t **order, int64_t *m_heavy, int64_t *light_pairs, unsigned long long *pairs);
+                               uint32_t **order, unsigned long long *pairs);
 cudaError_t launch_iota(Handle *H, int64_t m, uint32_t *out);
 cudaError_t launch_count_heavy(Handle *H, const RunPool &P, int64_t m, unsigned light_max, unsigned *count,
                                unsigned long long *pairs);

@@ -171,12 +171,11 @@ cudaError_t launch_walk(Handle *H, const DevTree &T, int strategy, const RunPool
     return cudaGetLastError();
 }
 
-// pair order of a walked slice and the number of heavy queries at its front: heaviest first
-// (LPT) unless `plain`, where it is the stable heavy/light partition of the walk order; the
-// accepted pairs of the heavy and the light queries are added to pairs[0], pairs[1] (zero before);
-// *light_pairs is the latter's value
+// pair order of a walked slice, heavy queries first, by descending size class unless `plain` (then the
+// stable heavy/light partition of the walk order); the word after *P.n_deferred counts the heavy
+// queries, and the accepted pairs of the heavy and the light queries are added to pairs[0], pairs[1]
 cudaError_t launch_split_order(Handle *H, const RunPool &P, int64_t m, unsigned light_max, bool plain,
-                               uint32_t **order, int64_t *m_heavy, int64_t *light_pairs, unsigned long long *pairs)
+                               uint32_t **order, unsigned long long *pairs)
 {
     cudaError_t e;
     if ((e = H->lpt_k.reserve(4 * m)) || (e = H->lpt_v.reserve(4 * m)) || (e = H->lpt_ka.reserve(4 * m)) ||
@@ -192,15 +191,7 @@ cudaError_t launch_split_order(Handle *H, const RunPool &P, int64_t m, unsigned 
     if ((e = cudaMemsetAsync(cnt, 0, sizeof(unsigned), H->stream))) return e;
     k_count_heavy<<<grid_for(m, 256), 256, 0, H->stream>>>(m, P.qacc, P.qflag, light_max, cnt, pairs);
     H->launches += 1;
-    if ((e = cudaGetLastError())) return e;
-    unsigned hcount = 0;
-    unsigned long long lp = 0;
-    if ((e = cudaMemcpyAsync(&hcount, cnt, sizeof(unsigned), cudaMemcpyDeviceToHost, H->stream))) return e;
-    if ((e = cudaMemcpyAsync(&lp, pairs + 1, sizeof(lp), cudaMemcpyDeviceToHost, H->stream))) return e;
-    if ((e = cudaStreamSynchronize(H->stream))) return e;
-    *m_heavy = hcount;
-    *light_pairs = (int64_t)lp;
-    return cudaSuccess;
+    return cudaGetLastError();
 }
 
 // the FP32C/FP64 split of a walked slice, left on the device: *count (zeroed here) = queries
