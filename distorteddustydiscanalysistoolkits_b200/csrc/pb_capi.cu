@@ -25,7 +25,7 @@ pb::Handle::~Handle()
                    &right, &escape, &parent, &bmin64, &bmax64, &hmax64, &counters, &rho_s, &col_ptrs,
                    &q_x, &q_y, &q_z, &q_keys, &q_keys_alt, &q_perm, &q_perm_alt, &q_out, &q_aux,
                    &pool_runs, &pool_next, &pool_ctr, &items, &wbnear, &qacc, &qflag, &defer_a, &defer_b,
-                   &lpt_k, &lpt_v, &lpt_ka, &lpt_va, &iota, &grid_ax, &grid_out, &mlp_w, &mlp_m, &mlp_v, &mlp_g, &mlp_norm,
+                   &lpt_k, &lpt_v, &lpt_ka, &lpt_va, &iota, &long_list, &long_count, &grid_ax, &grid_out, &mlp_w, &mlp_m, &mlp_v, &mlp_g, &mlp_norm,
                    &mlp_scr, &mlp_idx, &mlp_x, &mlp_y, &mlp_loss, &sched_feat, &sched_pred, &sched_ql, &sched_tmp};
     for (DBuf *b : all) b->release();
     batch_desc.release();
@@ -619,9 +619,9 @@ int fused_fallback(Handle &H, const DevTree &T, const std::vector<Launch> &launc
     lst = H.sched_tmp.as<uint32_t>();
     CK(cudaMemcpyAsync(lst, P.deferred, sizeof(uint32_t) * nd, cudaMemcpyDeviceToDevice, H.stream));
     P.count_only = 1;
-    if (strategy != SCATTER) CK(launch_nearest_list(&H, T, nd, lst, dx, dy, dz, P.bnear));
+    if (strategy != SCATTER) CK(launch_nearest_list(&H, T, nd, lst, dx, dy, dz, P.bnear, false));
     unsigned long long *ctr = H.pool_ctr.as<unsigned long long>();
-    CK(launch_walk(&H, T, strategy, P, nd, lst, dx, dy, dz, ctr + 2));
+    CK(launch_walk(&H, T, strategy, P, nd, lst, dx, dy, dz, false, ctr + 2));
     CK(cudaMemcpyAsync(list.data(), lst, sizeof(uint32_t) * nd, cudaMemcpyDeviceToHost, H.stream));
     CK(cudaMemcpyAsync(acc.data(), P.qacc, sizeof(unsigned) * nd, cudaMemcpyDeviceToHost, H.stream));
     CK(cudaStreamSynchronize(H.stream));
@@ -759,8 +759,10 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
             P.deferred = lists[round & 1];
             P.count_only = 0;
             ev_record(H, 4);
+            // longest walks first; the plain schedule keeps the input order, the learned one its own
+            const bool listed = strategy != SCATTER && mode == 1;
             if (strategy != SCATTER || mode == 2) {
-                CK(launch_nearest_list(&H, T, m, ql, dx, dy, dz, P.bnear));
+                CK(launch_nearest_list(&H, T, m, ql, dx, dy, dz, P.bnear, listed));
                 H.interp_launches++;
             }
             if (mode == 2) {
@@ -779,7 +781,7 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
                 H.interp_launches += 4;
             }
             ev_record(H, 5);
-            CK(launch_walk(&H, T, strategy, P, m, ql, dx, dy, dz, ctr + 2));
+            CK(launch_walk(&H, T, strategy, P, m, ql, dx, dy, dz, listed, ctr + 2));
             H.interp_launches++;
             uint32_t *order = nullptr;
             CK(launch_split_order(&H, P, m, (unsigned)H.light_max, mode == 0, &order, ctr + 4));

@@ -81,7 +81,7 @@ struct Handle {
     // run lists of the two-phase point path (walk kernel -> pair kernels)
     DBuf grid_ax, grid_out;   // axes / points of pb_grid_points
     DBuf pool_runs, pool_next, pool_ctr, items, wbnear, qacc, qflag, defer_a, defer_b, lpt_k, lpt_v, lpt_ka,
-        lpt_va, iota;
+        lpt_va, iota, long_list, long_count;
     int walk_split = 64;   // accepted and kept; the walk is not split any more
     int sched = 1;         // 0 plain (input order, one walk per query, no ordering), 1 tuned, 2 learned
     int64_t light_max = 4096;   // FP32C: queries with at most this many neighbours are summed in FP64
@@ -157,9 +157,10 @@ cudaError_t launch_sorted_columns(Handle *H, int64_t n, double *const dst[6], co
 
 // ---- launchers (pb_walk.cu) ----
 cudaError_t launch_nearest_list(Handle *H, const DevTree &T, int64_t m, const uint32_t *ql, const double *qx,
-                                const double *qy, const double *qz, int *bnear);
+                                const double *qy, const double *qz, int *bnear, bool listed);
+// listed: the nearest search of the same queries has listed those with the longest walks
 cudaError_t launch_walk(Handle *H, const DevTree &T, int strategy, const RunPool &P, int64_t m, const uint32_t *ql,
-                        const double *qx, const double *qy, const double *qz, unsigned long long *counter);
+                        const double *qx, const double *qy, const double *qz, bool listed, unsigned long long *counter);
 cudaError_t launch_split_order(Handle *H, const RunPool &P, int64_t m, unsigned light_max, bool plain,
                                uint32_t **order, unsigned long long *pairs);
 cudaError_t launch_iota(Handle *H, int64_t m, uint32_t *out);

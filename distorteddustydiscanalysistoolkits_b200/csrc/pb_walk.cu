@@ -9,27 +9,51 @@
 
 namespace pb {
 
+// Queries whose nearest particle's h is within a factor 8 of the largest have the longest walks (the
+// walk's work grows with the surface of the support).  The nearest search lists them, and the walk
+// takes them first: in Morton order they come last where a grid's corner lies far from the particles,
+// and the launch waited for them (SMs busy 72 % of the walk of 131,072 particles on 64^3 points).
+__device__ __forceinline__ bool long_walk(const DevTree &T, int b)
+{
+    if (T.root == 0 || b < 0) return false;
+    return 8.f * (float)ldg4(T.leaf + b).w >= __ldg(T.node_hmax + (T.root - 1));
+}
+
+struct LongList {
+    uint32_t *list;    // NULL: none
+    unsigned *count;
+    __device__ __forceinline__ void add(const DevTree &T, int64_t j, int b) const
+    {
+        if (list && long_walk(T, b)) list[atomicAdd(count, 1u)] = (uint32_t)j;
+    }
+};
+
 __global__ void __launch_bounds__(128) k_nearest_list(DevTree T, int64_t m, const uint32_t *__restrict__ ql,
                                                       const double *__restrict__ qx, const double *__restrict__ qy,
-                                                      const double *__restrict__ qz, int *bnear)
+                                                      const double *__restrict__ qz, int *bnear, LongList longs)
 {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m; j += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t qi = __ldg(ql + j);
-        bnear[j] = (int)nearest_leaf(T, __ldg(qx + qi), __ldg(qy + qi), __ldg(qz + qi));
+        const int b = (int)nearest_leaf(T, __ldg(qx + qi), __ldg(qy + qi), __ldg(qz + qi));
+        bnear[j] = b;
+        longs.add(T, j, b);
     }
 }
 
 // few queries: a warp each (nearest_leaf_warp)
 __global__ void __launch_bounds__(128) k_nearest_list_warp(DevTree T, int64_t m, const uint32_t *__restrict__ ql,
                                                            const double *__restrict__ qx, const double *__restrict__ qy,
-                                                           const double *__restrict__ qz, int *bnear)
+                                                           const double *__restrict__ qz, int *bnear, LongList longs)
 {
     __shared__ int s_stack[4][WSTACK];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     for (int64_t j = blockIdx.x * (int64_t)4 + wib; j < m; j += (int64_t)gridDim.x * 4) {
         const uint32_t qi = __ldg(ql + j);
-        const int64_t b = nearest_leaf_warp(T, __ldg(qx + qi), __ldg(qy + qi), __ldg(qz + qi), s_stack[wib], lane);
-        if (lane == 0) bnear[j] = (int)b;
+        const int b = (int)nearest_leaf_warp(T, __ldg(qx + qi), __ldg(qy + qi), __ldg(qz + qi), s_stack[wib], lane);
+        if (lane == 0) {
+            bnear[j] = b;
+            longs.add(T, j, b);
+        }
     }
 }
 
@@ -40,16 +64,22 @@ constexpr int WALK_TICKET = 4;
 template <int STRAT>
 __global__ void __launch_bounds__(128, 8) k_walk(DevTree T, RunPool P, int64_t m, const uint32_t *__restrict__ ql,
                                                  const double *__restrict__ qx, const double *__restrict__ qy,
-                                                 const double *__restrict__ qz, int ticket, unsigned long long *counter)
+                                                 const double *__restrict__ qz, int ticket, LongList longs,
+                                                 unsigned long long *counter)
 {
     __shared__ int s_walk[4][RUN_WALK_SMEM];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const double K = kernel_valid(T.kernel);
+    const int64_t nlong = longs.list ? min((int64_t)*longs.count, m) : 0;
+    // tickets: the listed queries one by one, then all others, `ticket` at a time
     for (;;) {
-        const int64_t t = next_query(counter, lane) * ticket;
-        if (t >= m) break;
-        const int64_t end = min(t + ticket, m);
-        for (int64_t j = t; j < end; ++j) {
+        const int64_t t = next_query(counter, lane);
+        const int64_t first = (t - nlong) * ticket;
+        if (t >= nlong && first >= m) break;
+        const int64_t end = t < nlong ? first + 1 : min(first + ticket, m);
+        for (int64_t k = first; k < end; ++k) {
+            const int64_t j = t < nlong ? (int64_t)longs.list[t] : k;
+            if (nlong > 0 && t >= nlong && long_walk(T, P.bnear[j])) continue;   // walked already
             const uint32_t qi = __ldg(ql + j);
             walk_query<STRAT>(T, P, j, qi, __ldg(qx + qi), __ldg(qy + qi), __ldg(qz + qi), K, s_walk[wib], lane);
         }
@@ -137,35 +167,41 @@ static int persistent_blocks(const void *kern, int bs)
 }
 
 cudaError_t launch_nearest_list(Handle *H, const DevTree &T, int64_t m, const uint32_t *ql, const double *qx,
-                                const double *qy, const double *qz, int *bnear)
+                                const double *qy, const double *qz, int *bnear, bool listed)
 {
+    cudaError_t e;
+    if (listed && ((e = H->long_list.reserve(sizeof(uint32_t) * m)) || (e = H->long_count.reserve(sizeof(unsigned))) ||
+                   (e = cudaMemsetAsync(H->long_count.p, 0, sizeof(unsigned), H->stream))))
+        return e;
+    const LongList L{listed ? H->long_list.as<uint32_t>() : nullptr, H->long_count.as<unsigned>()};
     if (m <= NEAREST_WARP_MAX)
-        k_nearest_list_warp<<<grid_for(m, 4, 1 << 30), 128, 0, H->stream>>>(T, m, ql, qx, qy, qz, bnear);
-    else k_nearest_list<<<grid_for(m, 128, 1 << 30), 128, 0, H->stream>>>(T, m, ql, qx, qy, qz, bnear);
+        k_nearest_list_warp<<<grid_for(m, 4, 1 << 30), 128, 0, H->stream>>>(T, m, ql, qx, qy, qz, bnear, L);
+    else k_nearest_list<<<grid_for(m, 128, 1 << 30), 128, 0, H->stream>>>(T, m, ql, qx, qy, qz, bnear, L);
     H->launches += 1;
     return cudaGetLastError();
 }
 
 template <int STRAT>
 static void launch_walk_strat(Handle *H, const DevTree &T, const RunPool &P, int64_t m, const uint32_t *ql,
-                              const double *qx, const double *qy, const double *qz, unsigned long long *counter)
+                              const double *qx, const double *qy, const double *qz, const LongList &longs,
+                              unsigned long long *counter)
 {
     const int warps = 4 * persistent_blocks((const void *)k_walk<STRAT>, 128);
     const int ticket = m >= (int64_t)warps * 16 ? WALK_TICKET : 1;
-    k_walk<STRAT><<<grid_for((m + ticket - 1) / ticket, 4, warps / 4), 128, 0, H->stream>>>(T, P, m, ql, qx, qy, qz, ticket,
-                                                                                          counter);
+    k_walk<STRAT><<<grid_for(m, 4, warps / 4), 128, 0, H->stream>>>(T, P, m, ql, qx, qy, qz, ticket, longs, counter);
 }
 
 cudaError_t launch_walk(Handle *H, const DevTree &T, int strategy, const RunPool &P, int64_t m, const uint32_t *ql,
-                        const double *qx, const double *qy, const double *qz, unsigned long long *counter)
+                        const double *qx, const double *qy, const double *qz, bool listed, unsigned long long *counter)
 {
     if (m <= 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), H->stream);
     if (e) return e;
+    const LongList L{listed ? H->long_list.as<uint32_t>() : nullptr, H->long_count.as<unsigned>()};
     switch (strategy) {
-    case GATHER: launch_walk_strat<GATHER>(H, T, P, m, ql, qx, qy, qz, counter); break;
-    case SCATTER: launch_walk_strat<SCATTER>(H, T, P, m, ql, qx, qy, qz, counter); break;
-    default: launch_walk_strat<SYMMETRIC>(H, T, P, m, ql, qx, qy, qz, counter); break;
+    case GATHER: launch_walk_strat<GATHER>(H, T, P, m, ql, qx, qy, qz, L, counter); break;
+    case SCATTER: launch_walk_strat<SCATTER>(H, T, P, m, ql, qx, qy, qz, L, counter); break;
+    default: launch_walk_strat<SYMMETRIC>(H, T, P, m, ql, qx, qy, qz, L, counter); break;
     }
     H->launches += 1;
     return cudaGetLastError();
