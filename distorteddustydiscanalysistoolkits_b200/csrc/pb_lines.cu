@@ -2,7 +2,7 @@
 // One thread per line walking the tree with an FP64 node bound was bound by that bound (six
 // divisions, two square roots a node) and by latency (5 % of the warp slots for a small image):
 // 1.5e6 particles on 1024^2 lines 54.6 ms, 20,011 particles on 97 x 61 oblique lines 3.18 ms.  Now
-// 12.7 ms (FP64 pipe 32 % active; the sums of 6e8 accepted pairs are most of it) and 0.29 ms.
+// 11.7 ms (FP64 pipe 32 % active; the sums of 6e8 accepted pairs are most of it) and 0.29 ms.
 // Compiled with -fmad=false: every expression is the IEEE result of the reference's operation
 // order.
 #include "line_tables.h"
@@ -285,18 +285,23 @@ __global__ void __launch_bounds__(128) k_lines_warp(DevTree T, DevCatalog C, int
 // pierce in the plane normal to them and stages 32 of the leaves so found at a time.  Every lane marks
 // the staged leaves near its own line (an FP32 test in the plane that errs on the safe side), then
 // takes its marked ones in DFS order: the exact test, the term, the sums.  Two leaves are in flight
-// per lane: a term is a chain of a square root, two table loads and two quotients.  Lines of different directions, and tiles whose lines share few of
-// their leaves (fewer than 1 in 16 tests passed after LTILE_PROBE leaves), go line by line through
-// line_by_warp.  4 blocks of 128 per SM (128 registers): 12.7 ms against 16.1 / 13.0 / 13.0 / 14.8 at
+// per lane: a term is a chain of a square root, two table loads and two quotients.  Lines of different
+// directions, and tiles whose lines share few of their leaves (fewer than 1 in 16 tests passed after
+// LTILE_PROBE leaves), go line by line through line_by_warp.  4 blocks of 128 per SM (128 registers): 12.7 ms against 16.1 / 13.0 / 13.0 / 14.8 at
 // 3 / 5 / 6 / 8 for 1.5e6 particles on 1024^2 lines.
 constexpr int LTILE_PROBE = 512;
 constexpr int LREC = 14;   // doubles per staged leaf: x, y, z, (K h)^2, the aux record, four columns; two of padding
 
+// WEIGH estimates the tiles' work instead, for the order they are taken in: the leaves of the subtrees of
+// at most `cut` leaves that the tile's rectangle reaches (keys: 8 bits, heaviest first; vals: the tile).
+template <bool WEIGH>
 __global__ void __launch_bounds__(128, 4) k_lines_tile(DevTree T, DevCatalog C, int64_t nl, const double *__restrict__ ox,
                                                     const double *__restrict__ oy, const double *__restrict__ oz,
                                                     const double *__restrict__ mx, const double *__restrict__ my,
                                                     const double *__restrict__ mz, const uint32_t *__restrict__ perm,
-                                                    const double *__restrict__ table, unsigned long long *counter)
+                                                    const double *__restrict__ table, unsigned long long *counter,
+                                                    const uint32_t *__restrict__ order, int cut, uint32_t *keys,
+                                                    uint32_t *vals)
 {
     __shared__ int s_stack[4][LSTACK], s_next[4][64];
     __shared__ __align__(16) double s_rec[4][32 * LREC];
@@ -313,9 +318,10 @@ __global__ void __launch_bounds__(128, 4) k_lines_tile(DevTree T, DevCatalog C, 
     unsigned long long nxt = 0;
     if (lane == 0) nxt = atomicAdd(counter, 1ULL);
     for (;;) {
-        const int64_t t = (int64_t)__shfl_sync(0xffffffffu, nxt, 0);
-        if (t >= ntile) break;
+        const int64_t k = (int64_t)__shfl_sync(0xffffffffu, nxt, 0);
+        if (k >= ntile) break;
         if (lane == 0) nxt = atomicAdd(counter, 1ULL);
+        const int64_t t = !WEIGH && order ? (int64_t)__ldg(order + k) : k;
         // lanes past the last line repeat it and store nothing
         const bool live = t * 32 + lane < nl;
         const int64_t j = live ? t * 32 + lane : nl - 1;
@@ -330,6 +336,7 @@ __global__ void __launch_bounds__(128, 4) k_lines_tile(DevTree T, DevCatalog C, 
             same = same && m[d] == m0;
         }
         bool tiled = __all_sync(0xffffffffu, same);
+        unsigned weight = 0;
         if (tiled) {
             LineBound B = make_line_bound(T, o, m);   // u, v are the same in every lane
             tiled = __all_sync(0xffffffffu, B.unit);
@@ -356,101 +363,131 @@ __global__ void __launch_bounds__(128, 4) k_lines_tile(DevTree T, DevCatalog C, 
             B.eu0 = fmaf(0.5f, amax - amin, 4.f * eps);
             B.ev0 = fmaf(0.5f, bmax - bmin, 4.f * eps);
             B.slack = slack;
-            double S1 = 0.0, acc[MAXS];
-#pragma unroll
-            for (int s = 0; s < MAXS; ++s) acc[s] = 0.0;
-            int tested = 0, passed = 0;
-            // this line's position relative to the rectangle's centre
-            const float al = a - ac, bl = b - bc;
-            auto sum = [&](int f) {   // the first f leaves of next[]
-                if (lane < f) {
-                    const int64_t b = Wk.next[lane];
-                    const double4 L = ldg4(T.leaf + b), X = ldg4(T.aux + b);
-                    double *r = rec + lane * LREC;
-                    r[0] = L.x; r[1] = L.y; r[2] = L.z; r[3] = leaf_radius2(lt.K, L.w);
-                    r[4] = X.x; r[5] = X.y; r[6] = X.z; r[7] = X.w;
-#pragma unroll
-                    for (int s = 0; s < MAXS; ++s) r[8 + s] = s < C.n_scalar ? __ldg(C.ucol[C.s_u[s]] + b) : 0.0;
-                    const float cx = (float)L.x - B.ox, cy = (float)L.y - B.oy, cz = (float)L.z - B.oz;
-                    const float rr = fmaf(Kf, __double2float_ru(fabs(L.w)), 8.f * eps);
-                    pos[lane] = make_float4(fmaf(B.uz, cz, fmaf(B.uy, cy, B.ux * cx)),
-                                            fmaf(B.vz, cz, fmaf(B.vy, cy, B.vx * cx)), fmaf(rr * rr, 1.000002f, slack), 0.f);
-                }
-                __syncwarp();
-                unsigned near = 0;
-                for (int i = 0; i < f; ++i) {
-                    const float4 p = pos[i];
-                    const float da = p.x - al, db = p.y - bl;
-                    near |= (!(fmaf(db, db, da * da) > p.z) ? 1u : 0u) << i;
-                }
-                passed += __popc(near);
-                auto term = [&](int i, double *A) {   // w (0 if the exact test fails) and the columns
-                    const double2 *r = reinterpret_cast<const double2 *>(rec + i * LREC);
-                    const double2 xy = r[0], zr = r[1], p = r[2], q = r[3];
-                    const double d2 = d2_line(xy.x, xy.y, zr.x, o, m);
-                    const bool in = d2 <= zr.y;
-                    const double w = line_weight(make_double4(p.x, p.y, q.x, q.y), lt, regular, d2);
-#pragma unroll
-                    for (int s = 0; s < MAXS; ++s) A[s] = in && s < C.n_scalar ? rec[i * LREC + 8 + s] * w : 0.0;
-                    return in ? w : 0.0;   // adding zero leaves a sum as it is
-                };
-                while (near) {
-                    const int i0 = __ffs(near) - 1;
-                    near &= near - 1;
-                    const int i1 = near ? __ffs(near) - 1 : -1;
-                    near &= near - 1;
-                    double A0[MAXS], A1[MAXS];
-                    const double w0 = term(i0, A0), w1 = term(i1 >= 0 ? i1 : i0, A1);
-                    S1 += w0;
-                    if (i1 >= 0) S1 += w1;
-#pragma unroll
-                    for (int s = 0; s < MAXS; ++s) {
-                        acc[s] += A0[s];
-                        if (i1 >= 0) acc[s] += A1[s];
+            if (WEIGH) {
+                auto weigh = [&](int e, int &e0, int &e1) {
+                    if (e >= n) {
+                        weight += 1u;
+                        return 0;
                     }
+                    if (line_pruned(B, load_node(T.node + (e - 1)), Kf, __ldg(T.node_hmax + (e - 1)))) return 0;
+                    const int2 r = __ldg(T.range + (e - 1)), ch = __ldg(T.child + (e - 1));
+                    if (r.y - r.x < cut) {
+                        weight += (unsigned)(r.y - r.x + 1);
+                        return 0;
+                    }
+                    e0 = ch.x;
+                    e1 = ch.y;
+                    return 2;
+                };
+                if (tiled) {
+                    Wk.start(T);
+                    while (Wk.round(T, weigh)) {}
                 }
-                tested += f;
-                __syncwarp();
-            };
-            auto visit = [&](int e, int &e0, int &e1) {
-                if (e >= n) {
-                    const double4 L = ldg4(T.leaf + (e - n));
-                    e0 = (int)((unsigned)(e - n) | 0x80000000u);
-                    NodeF nd;   // the leaf's position as an empty box (its rounding is within eu0, ev0)
-                    nd.lox = nd.hix = (float)L.x;
-                    nd.loy = nd.hiy = (float)L.y;
-                    nd.loz = nd.hiz = (float)L.z;
-                    return line_pruned(B, nd, Kf, __double2float_ru(fabs(L.w))) ? 0 : 1;
-                }
-                const NodeF nd = load_node(T.node + (e - 1));
-                const float hm = __ldg(T.node_hmax + (e - 1));
-                const int2 ch = __ldg(T.child + (e - 1));
-                e0 = ch.x;
-                e1 = ch.y;
-                return line_pruned(B, nd, Kf, hm) ? 0 : 2;
-            };
-            if (tiled) {
-                Wk.start(T);
-                while (Wk.round(T, visit))
-                    if (Wk.fill >= 32) {
-                        sum(32);
-                        Wk.advance();
-                        if (tested == LTILE_PROBE && __reduce_add_sync(0xffffffffu, passed) < 2 * LTILE_PROBE) {
-                            tiled = false;
-                            break;
+                weight = __reduce_add_sync(0xffffffffu, weight);
+            } else {
+                double S1 = 0.0, acc[MAXS];
+#pragma unroll
+                for (int s = 0; s < MAXS; ++s) acc[s] = 0.0;
+                int tested = 0, passed = 0;
+                // this line's position relative to the rectangle's centre
+                const float al = a - ac, bl = b - bc;
+                auto sum = [&](int f) {   // the first f leaves of next[]
+                    if (lane < f) {
+                        const int64_t b = Wk.next[lane];
+                        const double4 L = ldg4(T.leaf + b), X = ldg4(T.aux + b);
+                        double *r = rec + lane * LREC;
+                        r[0] = L.x; r[1] = L.y; r[2] = L.z; r[3] = leaf_radius2(lt.K, L.w);
+                        r[4] = X.x; r[5] = X.y; r[6] = X.z; r[7] = X.w;
+#pragma unroll
+                        for (int s = 0; s < MAXS; ++s) r[8 + s] = s < C.n_scalar ? __ldg(C.ucol[C.s_u[s]] + b) : 0.0;
+                        const float cx = (float)L.x - B.ox, cy = (float)L.y - B.oy, cz = (float)L.z - B.oz;
+                        const float rr = fmaf(Kf, __double2float_ru(fabs(L.w)), 8.f * eps);
+                        pos[lane] = make_float4(fmaf(B.uz, cz, fmaf(B.uy, cy, B.ux * cx)),
+                                                fmaf(B.vz, cz, fmaf(B.vy, cy, B.vx * cx)), fmaf(rr * rr, 1.000002f, slack), 0.f);
+                    }
+                    __syncwarp();
+                    unsigned near = 0;
+                    for (int i = 0; i < f; ++i) {
+                        const float4 p = pos[i];
+                        const float da = p.x - al, db = p.y - bl;
+                        near |= (!(fmaf(db, db, da * da) > p.z) ? 1u : 0u) << i;
+                    }
+                    passed += __popc(near);
+                    auto term = [&](int i, double *A) {   // w (0 if the exact test fails) and the columns
+                        const double2 *r = reinterpret_cast<const double2 *>(rec + i * LREC);
+                        const double2 xy = r[0], zr = r[1], p = r[2], q = r[3];
+                        const double d2 = d2_line(xy.x, xy.y, zr.x, o, m);
+                        const bool in = d2 <= zr.y;
+                        const double w = line_weight(make_double4(p.x, p.y, q.x, q.y), lt, regular, d2);
+#pragma unroll
+                        for (int s = 0; s < MAXS; ++s) A[s] = in && s < C.n_scalar ? rec[i * LREC + 8 + s] * w : 0.0;
+                        return in ? w : 0.0;   // adding zero leaves a sum as it is
+                    };
+                    while (near) {
+                        const int i0 = __ffs(near) - 1;
+                        near &= near - 1;
+                        const int i1 = near ? __ffs(near) - 1 : -1;
+                        near &= near - 1;
+                        double A0[MAXS], A1[MAXS];
+                        const double w0 = term(i0, A0), w1 = term(i1 >= 0 ? i1 : i0, A1);
+                        S1 += w0;
+                        if (i1 >= 0) S1 += w1;
+#pragma unroll
+                        for (int s = 0; s < MAXS; ++s) {
+                            acc[s] += A0[s];
+                            if (i1 >= 0) acc[s] += A1[s];
                         }
                     }
-            }
-            if (tiled) {
-                if (Wk.fill > 0) sum(Wk.fill);
-                if (live) {
+                    tested += f;
+                    __syncwarp();
+                };
+                auto visit = [&](int e, int &e0, int &e1) {
+                    if (e >= n) {
+                        const double4 L = ldg4(T.leaf + (e - n));
+                        e0 = (int)((unsigned)(e - n) | 0x80000000u);
+                        NodeF nd;   // the leaf's position as an empty box (its rounding is within eu0, ev0)
+                        nd.lox = nd.hix = (float)L.x;
+                        nd.loy = nd.hiy = (float)L.y;
+                        nd.loz = nd.hiz = (float)L.z;
+                        return line_pruned(B, nd, Kf, __double2float_ru(fabs(L.w))) ? 0 : 1;
+                    }
+                    const NodeF nd = load_node(T.node + (e - 1));
+                    const float hm = __ldg(T.node_hmax + (e - 1));
+                    const int2 ch = __ldg(T.child + (e - 1));
+                    e0 = ch.x;
+                    e1 = ch.y;
+                    return line_pruned(B, nd, Kf, hm) ? 0 : 2;
+                };
+                if (tiled) {
+                    Wk.start(T);
+                    while (Wk.round(T, visit))
+                        if (Wk.fill >= 32) {
+                            sum(32);
+                            Wk.advance();
+                            if (tested == LTILE_PROBE && __reduce_add_sync(0xffffffffu, passed) < 2 * LTILE_PROBE) {
+                                tiled = false;
+                                break;
+                            }
+                        }
+                }
+                if (tiled) {
+                    if (Wk.fill > 0) sum(Wk.fill);
+                    if (live) {
 #pragma unroll
-                    for (int s = 0; s < MAXS; ++s)
-                        if (s < C.n_scalar)
-                            C.out[s][li] = S1 == 0.0 ? __longlong_as_double(0x7ff8000000000000LL)
-                                                     : (C.s_shep[s] ? acc[s] * (1.0 / S1) : acc[s]);
+                        for (int s = 0; s < MAXS; ++s)
+                            if (s < C.n_scalar)
+                                C.out[s][li] = S1 == 0.0 ? __longlong_as_double(0x7ff8000000000000LL)
+                                                         : (C.s_shep[s] ? acc[s] * (1.0 / S1) : acc[s]);
+                    }
                 }
             }
+        }
+        if (WEIGH) {
+            if (lane == 0) {
+                keys[t] = 255u - count_class(tiled ? weight : 0x7fffffffu);   // line by line: the most work
+                vals[t] = (uint32_t)t;
+            }
+            continue;
         }
         if (!tiled) {
             const int lines = (int)(nl - t * 32 < 32 ? nl - t * 32 : 32);
@@ -472,6 +509,13 @@ __global__ void __launch_bounds__(128, 4) k_lines_tile(DevTree T, DevCatalog C, 
 // particles, 512^2 2.3 / 4.5 ms; 20,011 particles, 512^2 1.6 / 2.6 ms; 256^2 lines go by warps (2.3 ms,
 // one thread per line 8.9 ms).
 constexpr int64_t LINE_TILES_MIN = 131072;
+// Particles from which on the tiles are taken by descending estimated work: in Morton order the tiles of
+// the densest part, met late, run on alone (SMs active 70 % of the time).  Subtrees of at most
+// n / 2^13 leaves are counted whole; n / 2^9 .. n / 2^15 are within 6 %.  Morton order / by work, 1024^2
+// lines of 1.5e6 particles: face-on 12.3 / 11.7 ms, oblique 16.2 / 12.8; 512^2 lines of 2e5 2.02 / 1.98,
+// of 20,011 1.34 / 1.55 (the estimate costs more than it gives).
+constexpr int64_t LINE_ORDER_MIN = 262144;
+constexpr int LINE_CUT_SHIFT = 13;
 
 cudaError_t launch_lines_fp64(Handle *H, const DevTree &T, const DevCatalog &C, int64_t nl, const double *ox,
                               const double *oy, const double *oz, const double *dx, const double *dy,
@@ -484,13 +528,29 @@ cudaError_t launch_lines_fp64(Handle *H, const DevTree &T, const DevCatalog &C, 
     unsigned long long *ctr = H->counter.as<unsigned long long>();
     if ((e = cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), H->stream))) return e;
     const bool tiles = nl >= LINE_TILES_MIN && perm;
-    const void *kern = tiles ? (const void *)k_lines_tile : (const void *)k_lines_warp;
+    const void *kern = tiles ? (const void *)k_lines_tile<false> : (const void *)k_lines_warp;
     int sms = 148, per = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, H->device);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 128, 0);
     const int grid = grid_for(tiles ? (nl + 31) / 32 : nl, 4, sms * (per > 0 ? per : 1));
-    if (tiles) k_lines_tile<<<grid, 128, 0, H->stream>>>(T, C, nl, ox, oy, oz, dx, dy, dz, perm, tab, ctr);
-    else k_lines_warp<<<grid, 128, 0, H->stream>>>(T, C, nl, ox, oy, oz, dx, dy, dz, perm, tab, ctr);
+    if (tiles) {
+        uint32_t *order = nullptr;
+        const int64_t nt = (nl + 31) / 32;
+        if (T.n >= LINE_ORDER_MIN) {
+            if ((e = H->lpt_k.reserve(4 * nt)) || (e = H->lpt_v.reserve(4 * nt)) || (e = H->lpt_ka.reserve(4 * nt)) ||
+                (e = H->lpt_va.reserve(4 * nt)))
+                return e;
+            uint32_t *k = H->lpt_k.as<uint32_t>(), *v = H->lpt_v.as<uint32_t>();
+            k_lines_tile<true><<<grid, 128, 0, H->stream>>>(T, C, nl, ox, oy, oz, dx, dy, dz, perm, tab, ctr, nullptr,
+                                                            (int)(T.n >> LINE_CUT_SHIFT), k, v);
+            if ((e = cudaGetLastError())) return e;
+            if ((e = sort_pairs_u32(H, k, v, H->lpt_ka.as<uint32_t>(), H->lpt_va.as<uint32_t>(), nt, 8, &order))) return e;
+            if ((e = cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), H->stream))) return e;
+            H->launches += 1;
+        }
+        k_lines_tile<false><<<grid, 128, 0, H->stream>>>(T, C, nl, ox, oy, oz, dx, dy, dz, perm, tab, ctr, order, 0, nullptr,
+                                                         nullptr);
+    } else k_lines_warp<<<grid, 128, 0, H->stream>>>(T, C, nl, ox, oy, oz, dx, dy, dz, perm, tab, ctr);
     H->launches += 1;
     return cudaGetLastError();
 }
