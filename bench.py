@@ -50,7 +50,7 @@ UNIT = "grid pts/s"
 L2_FLUSH_BYTES = 256 << 20
 # thread instructions per pair of k_pairs32w<itpSymmetric, M4, grad+div+curl> measured by ncu
 # (smsp__inst_executed.sum x 32 / pairs; profiles/k_pairs32w_c2disc_96x96x24.md)
-PAIRS32_THREAD_INST_PER_PAIR = 113.7
+PAIRS32_THREAD_INST_PER_PAIR = 112.6
 
 
 def parse():
@@ -642,14 +642,14 @@ def main():
         kname = {"M4_spline": "M4", "C4_Wendland": "C4"}.get(config["kernel"], config["kernel"])
         pk = "k_pairs32w<itpSymmetric,%s> (+ k_pairs64w for light queries)" % kname if prec == pb.FP32C \
             else "k_pairs64w<itpSymmetric>"
-        kern = {"walk": ("k_nearest_list + k_item_filter + k_walk_list<itpSymmetric>", ph[0] + ph[1]), "pairs": (pk, ph[2])}
+        kern = {"walk": ("k_nearest_list + k_walk<itpSymmetric>", ph[0] + ph[1]), "pairs": (pk, ph[2])}
         per = {}
         for key, (name, ms) in kern.items():
             a = alg[key] / (ms / 1e3) / 1e9 if ms > 0 else None
             per[key] = {"kernel": name, "ms": float(ms), "algorithmic_bytes": alg[key], "achieved_gbs": a}
         dom = max(per, key=lambda k: per[k]["ms"])
         traffic = None
-        prof = os.path.join(REPO, "profiles", {"pairs": "k_pairs32w", "walk": "k_walk_items"}[dom] + "_c2_traffic.json")
+        prof = os.path.join(REPO, "profiles", {"pairs": "k_pairs32w", "walk": "k_walk"}[dom] + "_c2_traffic.json")
         if os.path.exists(prof) and args.precision == "fp32c" and args.config == "c2" and \
                 args.particles in (None, 1 << 21) and args.grid in (None, "256,256,64"):
             traffic = json.load(open(prof)).get("dram_bytes_per_launch")

@@ -8,15 +8,16 @@ its size class.  The options change only the schedule, so a batch gives the same
 separate calls (tests/test_gpu_batch.py).
 
 The autotuner times the interpolation of a representative job of each size class (particles
-and points rounded to powers of 4) under every candidate setting of the walk split, the slice
-size and the scheduler bin width, and keeps the fastest.
+and points rounded to powers of 4) under every candidate setting of the slice size and the
+scheduler bin width (the walk split, still a candidate, no longer has an effect), and keeps the
+fastest.
 
 ``DeviceBatch`` is the one-launch form: every disc's particles, sample points and outputs stay
 on the device, each disc has its own handle (its tree), all handles share one stream, and a
 step enqueues every disc's LBVH build (PB_BUILD_ASYNC) and one pb_batch_points launch that
 interpolates the sample points of all discs.  The step can be captured in a CUDA graph and
-replayed.  ``BatchAutotuner`` picks its schedule options -- the walk's leaf size (subtrees of at
-most that many leaves scanned linearly), the disc order (given or most work first) and the
+replayed.  ``BatchAutotuner`` picks its schedule options -- the fused
+fallback's leaf size (subtrees of at most that many leaves scanned linearly), the disc order (given or most work first) and the
 blocks per SM -- by timing graph replays; outputs do not depend on them.
 """
 import ctypes

@@ -45,8 +45,8 @@ __global__ void __launch_bounds__(128) k_points32w(DevTree T, DevCatalog C, cons
     }
 }
 
-// Pair kernel of the two-phase path: a warp takes a walked query (heaviest first), reads the
-// runs of its (query, subtree) items in subtree order, chunk by chunk, and deals the accepted
+// Pair kernel of the two-phase path: a warp takes a walked query (heaviest first), reads its
+// runs chunk by chunk, and deals the accepted
 // leaves to its lanes in DFS order -- the k-th accepted leaf to lane k mod 32, exactly as the
 // fused kernel does, so both produce the same bits.  A block takes four queries that follow each other
 // in the order (one size class, Morton order): its warps read the same particles at about the same
