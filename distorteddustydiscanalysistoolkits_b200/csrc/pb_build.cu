@@ -497,7 +497,7 @@ __global__ void k_gather(int64_t n, const uint32_t *__restrict__ idx, const doub
                          const double *__restrict__ m, const double *__restrict__ rho, double4 *leaf, double4 *aux,
                          double *rhos, int *odd, GatherCols cols)
 {
-    bool bad = false;
+    int bits = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         uint32_t o = idx[i];
         if (o >= (uint64_t)n) o = 0;   // unreachable for a valid permutation; keeps reads in bounds
@@ -506,9 +506,9 @@ __global__ void k_gather(int64_t n, const uint32_t *__restrict__ idx, const doub
         aux[i] = make_double4(1.0 / ho, 1.0 / ro, m[o], ro);
         rhos[i] = ro;
         for (int c = 0; c < cols.n; ++c) cols.dst[c][i] = cols.src[c][o];
-        bad |= !aux_regular(ho, ro);
+        if (!aux_regular(ho, ro)) bits |= ho < 0.0 ? ODD_RANGE | ODD_NEGATIVE_H : ODD_RANGE;
     }
-    if (bad) atomicOr(odd, 1);
+    if (bits) atomicOr(odd, bits);
 }
 
 __global__ void k_gather_cols(int64_t n, const uint32_t *__restrict__ idx, GatherCols cols)

@@ -60,7 +60,7 @@ struct DevTree {
     const float *node_hmax;
     const int2 *child;      // (left, right) unified ids of each internal node
     const double4 *aux;     // {1/h, 1/rho, m, rho} of each sorted particle (reciprocals correctly rounded)
-    const int *odd;         // nonzero: some particle's h or rho is outside aux_regular's range
+    const int *odd;         // ODD_* bits of the particles, 0 for an ordinary set
     const int2 *range;      // 0-based sorted leaf range [lo, hi] of each internal node's subtree
     const uint64_t *codes;  // sorted 63-bit Morton codes, and their quantisation frame
     const QuantParams *qp;
@@ -124,6 +124,10 @@ __device__ __forceinline__ bool exp_safe(double x)
 {
     return (unsigned)((__double2hiint(x) & 0x7ff00000) - ((1023 - 250) << 20)) < (unsigned)(500 << 20);
 }
+
+// DevTree::odd
+constexpr int ODD_RANGE = 1;        // some particle's h or rho is outside aux_regular's range
+constexpr int ODD_NEGATIVE_H = 2;   // some h is negative: a leaf's radius |K h| may exceed its nodes' K hmax
 
 // the particles the pair kernels take their short forms for (DevTree::odd is 0 if all are)
 __device__ __forceinline__ bool aux_regular(double h, double rho) { return h > 0.0 && exp_safe(h) && exp_safe(rho); }

@@ -22,17 +22,18 @@ __device__ const double g_line_inorm64[6][PB_LINE_NTAB] = PB_LINE_INORM_INIT;
 // in d2_line's difference (measured from the caller's origin), so a node is pruned only if
 // d2_line exceeds the radius of every leaf in it.  29 FP32 operations a node; the FP64 slab and
 // sphere bound (d2_line_box_lower) took six divisions and two square roots.  Directions
-// that are not unit vectors to 1e-12 keep that one: d2_line is not their distance.
+// that are not unit vectors to 1e-12 keep that one, as d2_line is not their distance, and so do trees with
+// a negative h, where a leaf's radius may exceed its nodes' and the bound decides which leaves are reached.
 struct LineBound {
     float ox, oy, oz, ux, uy, uz, vx, vy, vz, eu0, ev0, slack;   // eu0, ev0: added to the half extents
-    bool unit;
+    bool plane;   // the FP32 bound holds; else d2_line_box_lower is taken
 };
 
 __device__ __forceinline__ LineBound make_line_bound(const DevTree &T, const double o[3], const double m[3])
 {
     LineBound B;
     const double m2 = m[0] * m[0] + m[1] * m[1] + m[2] * m[2];
-    B.unit = fabs(m2 - 1.0) <= 1e-12;
+    B.plane = fabs(m2 - 1.0) <= 1e-12 && !(__ldg(T.odd) & ODD_NEGATIVE_H);
     const NodeF nd = load_node(T.node + (T.root - 1));
     const double lo[3] = {(double)nd.lox, (double)nd.loy, (double)nd.loz}, hi[3] = {(double)nd.hix, (double)nd.hiy, (double)nd.hiz};
     double c[3], t = 0.0, far2 = 0.0, rad2 = 0.0;
@@ -235,7 +236,7 @@ __device__ __forceinline__ void line_by_warp(const DevTree &T, const DevCatalog 
             const int2 ch = __ldg(T.child + (e - 1));
             e0 = ch.x;
             e1 = ch.y;
-            const bool prune = B.unit ? line_pruned(B, nd, Kf, hm) : d2_line_box_lower(o, m, nd) > leaf_radius2(lt.K, (double)hm);
+            const bool prune = B.plane ? line_pruned(B, nd, Kf, hm) : d2_line_box_lower(o, m, nd) > leaf_radius2(lt.K, (double)hm);
             return prune ? 0 : 2;
         };
         Wk.start(T);
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(128, 4) k_lines_tile(DevTree T, DevCatalog C, 
         unsigned weight = 0;
         if (tiled) {
             LineBound B = make_line_bound(T, o, m);   // u, v are the same in every lane
-            tiled = __all_sync(0xffffffffu, B.unit);
+            tiled = __all_sync(0xffffffffu, B.plane);
             // the lines' positions in the plane, relative to the first one's, and their rectangle
             const float px = __shfl_sync(0xffffffffu, B.ox, 0), py = __shfl_sync(0xffffffffu, B.oy, 0),
                         pz = __shfl_sync(0xffffffffu, B.oz, 0);

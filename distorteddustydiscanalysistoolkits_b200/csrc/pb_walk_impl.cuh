@@ -4,7 +4,7 @@
 //
 // The warp keeps a stack of tree entries whose top is the next one in DFS order.  Each round its
 // lanes take the top 32: a subtree that the query does not reach is dropped; one inside the
-// query's radius, one of at most WALK_SCAN leaves and a leaf stay; any other is replaced by its two
+// query's radius, one of few leaves (WALK_SCAN) and a leaf stay; any other is replaced by its two
 // children.  The entries that stay and come before the first one opened are the next ones in DFS
 // order: they collect until there are 32, then their leaves are tested 32 at a time (those of a
 // subtree inside the radius pass as a whole) and what is accepted is appended to the runs.  The node
@@ -25,6 +25,8 @@ namespace pb {
 // operations, batched over the lanes, an opening two more box tests.  Walk phase at 1 / 4 / 8 / 16 / 32:
 // 2.1e6 particles, 4.2e6 points 147 / 119 / 107 / 102 / 109 ms; 131,072 particles, 64^3 points 3.2 / 2.7 /
 // 2.5 / 2.5 / 2.6; scatter, 1e5 tracers 0.82 / 0.72 / 0.71 / 0.72 / 0.76.
+// A scanned leaf skips the tests of the nodes between it and the subtree; they could only have cut it
+// off where its radius exceeds theirs, that is where an h is negative: such trees are opened to the leaves.
 constexpr int WALK_SCAN = 16;
 constexpr int WSTACK = 512;   // entries; taken one at a time above WSTACK - 160, where a round adds at most one
 constexpr int WALK_SMEM = WSTACK + 128;       // ints of shared memory per warp of a WarpWalk
@@ -166,6 +168,7 @@ struct WarpWalk {
         const float bulk_lim = __fmul_rd(__double2float_rd(r2a), MARGIN_DN);
         const unsigned below = (1u << lane) - 1u;
         const unsigned limit = 2u * (unsigned)n + 64u;   // every round settles or opens at least one entry
+        const int scan = STRAT != GATHER && (__ldg(T.odd) & ODD_NEGATIVE_H) ? 1 : WALK_SCAN;
         unsigned guard = 0;
         int size = 1;
         if (lane == 0) stack[0] = T.root;
@@ -191,7 +194,7 @@ struct WarpWalk {
                         c = 0;
                     } else if (STRAT != SCATTER && box_upper(q, nd) <= bulk_lim) {
                         len = -len;
-                    } else if (len > WALK_SCAN) {
+                    } else if (len > scan) {
                         // the children of a Karras node meet at the split, which the left child's id
                         // gives; a child of one leaf is that leaf
                         c = 2;
