@@ -81,7 +81,7 @@ struct Handle {
     // run lists of the two-phase point path (walk kernel -> pair kernels)
     DBuf grid_ax, grid_out;   // axes / points of pb_grid_points
     DBuf pool_runs, pool_next, pool_ctr, items, wbnear, qacc, qflag, defer_a, defer_b, lpt_k, lpt_v, lpt_ka,
-        lpt_va, iota, long_list, long_count;
+        lpt_va, iota, long_list, long_count, line_rest;
     int walk_split = 64;   // accepted and kept; the walk is not split any more
     int sched = 1;         // 0 plain (input order, one walk per query, no ordering), 1 tuned, 2 learned
     int64_t light_max = 4096;   // FP32C: queries with at most this many neighbours are summed in FP64

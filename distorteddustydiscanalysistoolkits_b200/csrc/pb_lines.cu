@@ -256,11 +256,13 @@ __device__ __forceinline__ void line_by_warp(const DevTree &T, const DevCatalog 
     }
 }
 
+// rest: the number of tiles and the tiles (of k_lines_tile) whose lines are taken; NULL: all lines
 __global__ void __launch_bounds__(128) k_lines_warp(DevTree T, DevCatalog C, int64_t nl, const double *__restrict__ ox,
                                                     const double *__restrict__ oy, const double *__restrict__ oz,
                                                     const double *__restrict__ mx, const double *__restrict__ my,
                                                     const double *__restrict__ mz, const uint32_t *__restrict__ perm,
-                                                    const double *__restrict__ table, unsigned long long *counter)
+                                                    const double *__restrict__ table, unsigned long long *counter,
+                                                    const uint32_t *__restrict__ rest)
 {
     __shared__ int s_stack[4][LSTACK], s_next[4][64];
     __shared__ __align__(16) double s_term[4][LROWS * LROW];
@@ -268,12 +270,17 @@ __global__ void __launch_bounds__(128) k_lines_warp(DevTree T, DevCatalog C, int
     LineWalk Wk{s_stack[wib], s_next[wib], lane};
     const LineTable lt = make_line_table(table, T.kernel);
     const bool regular = __ldg(T.odd) == 0;
+    const int64_t todo = rest ? 32 * (int64_t)__ldg(rest) : nl;
     unsigned long long nxt = 0;
     if (lane == 0) nxt = atomicAdd(counter, 1ULL);
     for (;;) {
-        const int64_t j = (int64_t)__shfl_sync(0xffffffffu, nxt, 0);
-        if (j >= nl) break;
+        int64_t j = (int64_t)__shfl_sync(0xffffffffu, nxt, 0);
+        if (j >= todo) break;
         if (lane == 0) nxt = atomicAdd(counter, 1ULL);
+        if (rest) {
+            j = (int64_t)__ldg(rest + 1 + (j >> 5)) * 32 + (j & 31);
+            if (j >= nl) continue;   // past the last line of the last tile
+        }
         const int64_t li = perm ? (int64_t)__ldg(perm + j) : j;
         if (li >= nl) continue;   // unreachable for a valid permutation
         const double o[3] = {__ldg(ox + li), __ldg(oy + li), __ldg(oz + li)};
@@ -287,10 +294,15 @@ __global__ void __launch_bounds__(128) k_lines_warp(DevTree T, DevCatalog C, int
 // the staged leaves near its own line (an FP32 test in the plane that errs on the safe side), then
 // takes its marked ones in DFS order: the exact test, the term, the sums.  Two leaves are in flight
 // per lane: a term is a chain of a square root, two table loads and two quotients.  Lines of different
-// directions, and tiles whose lines share few of their leaves (fewer than 1 in 16 tests passed after
-// LTILE_PROBE leaves), go line by line through line_by_warp.  4 blocks of 128 per SM (128 registers): 12.7 ms against 16.1 / 13.0 / 13.0 / 14.8 at
+// directions, and tiles whose lines share few of their leaves (fewer than 1 in LTILE_SHARE tests passed after
+// LTILE_PROBE leaves, and after twice as many, and so on: a tile that lies across a jump of the Morton
+// order, or lines in no order at all), are left to k_lines_warp, tile by tile in `rest`.  Taking them here,
+// 32 lines one after the other, made one warp the end of the launch: 363^2 lines of 1.5e6 particles 36.3 ms,
+// now 6.3; 400^2 with origins at scattered depths 50.2, now 12.6.  Shares of 4 / 8 / 16 / 32: 6.9 / 6.3 / 7.3 / 8.2
+// and 12.9 / 12.6 / 14.3 / 18.3 ms; images in order are within 5 % (1024^2 17.3 / 16.6 / 16.6 / 16.6).
+// 4 blocks of 128 per SM (128 registers): 12.7 ms against 16.1 / 13.0 / 13.0 / 14.8 at
 // 3 / 5 / 6 / 8 for 1.5e6 particles on 1024^2 lines.
-constexpr int LTILE_PROBE = 512;
+constexpr int LTILE_PROBE = 512, LTILE_SHARE = 8;
 constexpr int LREC = 14;   // doubles per staged leaf: x, y, z, (K h)^2, the aux record, four columns; two of padding
 
 // WEIGH estimates the tiles' work instead, for the order they are taken in: the leaves of the subtrees of
@@ -302,12 +314,11 @@ __global__ void __launch_bounds__(128, 4) k_lines_tile(DevTree T, DevCatalog C, 
                                                     const double *__restrict__ mz, const uint32_t *__restrict__ perm,
                                                     const double *__restrict__ table, unsigned long long *counter,
                                                     const uint32_t *__restrict__ order, int cut, uint32_t *keys,
-                                                    uint32_t *vals)
+                                                    uint32_t *vals, uint32_t *rest)
 {
     __shared__ int s_stack[4][LSTACK], s_next[4][64];
     __shared__ __align__(16) double s_rec[4][32 * LREC];
     __shared__ __align__(16) float4 s_pos[4][32];
-    static_assert(32 * LREC >= LROWS * LROW, "the staged leaves share their space with line_by_warp's terms");
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, n = (int)T.n;
     LineWalk Wk{s_stack[wib], s_next[wib], lane};
     double *rec = s_rec[wib];
@@ -465,7 +476,8 @@ __global__ void __launch_bounds__(128, 4) k_lines_tile(DevTree T, DevCatalog C, 
                         if (Wk.fill >= 32) {
                             sum(32);
                             Wk.advance();
-                            if (tested == LTILE_PROBE && __reduce_add_sync(0xffffffffu, passed) < 2 * LTILE_PROBE) {
+                            if (tested >= LTILE_PROBE && (tested & (tested - 1)) == 0 &&
+                                (int64_t)__reduce_add_sync(0xffffffffu, (unsigned)passed) * LTILE_SHARE < (int64_t)tested * 32) {
                                 tiled = false;
                                 break;
                             }
@@ -490,25 +502,14 @@ __global__ void __launch_bounds__(128, 4) k_lines_tile(DevTree T, DevCatalog C, 
             }
             continue;
         }
-        if (!tiled) {
-            const int lines = (int)(nl - t * 32 < 32 ? nl - t * 32 : 32);
-            for (int l = 0; l < lines; ++l) {
-                double ol[3], ml[3];
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    ol[d] = __shfl_sync(0xffffffffu, o[d], l);
-                    ml[d] = __shfl_sync(0xffffffffu, m[d], l);
-                }
-                line_by_warp(T, C, lt, regular, ol, ml, __shfl_sync(0xffffffffu, li, l), Wk, rec);
-            }
-        }
+        if (!tiled && lane == 0) rest[1 + atomicAdd(rest, 1u)] = (uint32_t)t;
     }
 }
 
 // Lines from which on the tiles of 32 (in Morton order) fill the chip's warps twice; below, a warp per
-// line has more in flight.  Tiles / a warp per line: 1.5e6 particles, 1024^2 lines 12.7 / 29.7 ms; 2e5
-// particles, 512^2 2.3 / 4.5 ms; 20,011 particles, 512^2 1.6 / 2.6 ms; 256^2 lines go by warps (2.3 ms,
-// one thread per line 8.9 ms).
+// line has more in flight.  Tiles / a warp per line (M5), 256^2, 300^2, 363^2 (131,769) and 512^2 lines: 1.5e6
+// particles 6.3 / 4.2, 6.6 / 5.7, 6.3 / 8.3, 6.7 / 16.2 ms; 2e5 2.0 / 2.2, 2.1 / 3.0, 2.2 / 4.4, 2.9 / 8.5;
+// 20,011 0.69 / 1.10, 0.76 / 1.47, 0.79 / 2.07, 1.03 / 3.93: one line for all sets, where none is slower by tiles.
 constexpr int64_t LINE_TILES_MIN = 131072;
 // Particles from which on the tiles are taken by descending estimated work: in Morton order the tiles of
 // the densest part, met late, run on alone (SMs active 70 % of the time).  Subtrees of at most
@@ -525,33 +526,42 @@ cudaError_t launch_lines_fp64(Handle *H, const DevTree &T, const DevCatalog &C, 
     const double *tab = nullptr;
     cudaError_t e = cudaGetSymbolAddress((void **)&tab, g_line_inorm64);
     if (e) return e;
-    if ((e = H->counter.reserve(sizeof(unsigned long long)))) return e;
+    if ((e = H->counter.reserve(2 * sizeof(unsigned long long)))) return e;
     unsigned long long *ctr = H->counter.as<unsigned long long>();
-    if ((e = cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), H->stream))) return e;
+    if ((e = cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned long long), H->stream))) return e;
     const bool tiles = nl >= LINE_TILES_MIN && perm;
-    const void *kern = tiles ? (const void *)k_lines_tile<false> : (const void *)k_lines_warp;
-    int sms = 148, per = 1;
+    int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, H->device);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 128, 0);
-    const int grid = grid_for(tiles ? (nl + 31) / 32 : nl, 4, sms * (per > 0 ? per : 1));
+    auto grid_of = [&](const void *kern, int64_t warps) {
+        int per = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 128, 0);
+        return grid_for(warps, 4, sms * (per > 0 ? per : 1));
+    };
+    const int wgrid = grid_of((const void *)k_lines_warp, nl);
     if (tiles) {
         uint32_t *order = nullptr;
         const int64_t nt = (nl + 31) / 32;
+        const int grid = grid_of((const void *)k_lines_tile<false>, nt);
+        if ((e = H->line_rest.reserve(4 * (nt + 1)))) return e;
+        uint32_t *rest = H->line_rest.as<uint32_t>();
+        if ((e = cudaMemsetAsync(rest, 0, 4, H->stream))) return e;
         if (T.n >= LINE_ORDER_MIN) {
             if ((e = H->lpt_k.reserve(4 * nt)) || (e = H->lpt_v.reserve(4 * nt)) || (e = H->lpt_ka.reserve(4 * nt)) ||
                 (e = H->lpt_va.reserve(4 * nt)))
                 return e;
             uint32_t *k = H->lpt_k.as<uint32_t>(), *v = H->lpt_v.as<uint32_t>();
             k_lines_tile<true><<<grid, 128, 0, H->stream>>>(T, C, nl, ox, oy, oz, dx, dy, dz, perm, tab, ctr, nullptr,
-                                                            (int)(T.n >> LINE_CUT_SHIFT), k, v);
+                                                            (int)(T.n >> LINE_CUT_SHIFT), k, v, nullptr);
             if ((e = cudaGetLastError())) return e;
             if ((e = sort_pairs_u32(H, k, v, H->lpt_ka.as<uint32_t>(), H->lpt_va.as<uint32_t>(), nt, 8, &order))) return e;
             if ((e = cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), H->stream))) return e;
             H->launches += 1;
         }
         k_lines_tile<false><<<grid, 128, 0, H->stream>>>(T, C, nl, ox, oy, oz, dx, dy, dz, perm, tab, ctr, order, 0, nullptr,
-                                                         nullptr);
-    } else k_lines_warp<<<grid, 128, 0, H->stream>>>(T, C, nl, ox, oy, oz, dx, dy, dz, perm, tab, ctr);
+                                                         nullptr, rest);
+        k_lines_warp<<<wgrid, 128, 0, H->stream>>>(T, C, nl, ox, oy, oz, dx, dy, dz, perm, tab, ctr + 1, rest);
+        H->launches += 1;
+    } else k_lines_warp<<<wgrid, 128, 0, H->stream>>>(T, C, nl, ox, oy, oz, dx, dy, dz, perm, tab, ctr, nullptr);
     H->launches += 1;
     return cudaGetLastError();
 }
