@@ -165,13 +165,23 @@ __device__ __forceinline__ float child_dist(const DevTree &T, const QBox &q, int
     return box_lower(q, load_node(T.node + (id - 1)));
 }
 
-__device__ __forceinline__ int64_t nearest_leaf(const DevTree &T, double px, double py, double pz)
+// WITHIN: of the leaves with d2 <= within only (-1 if there is none).  The bound also ends the search
+// early: a point far from all particles else visits the whole tree, as the FP32 boxes do not tell its
+// distances apart (probes of radius 1 at 40,000 points some 1e9 from 2e5 particles: 332 ms, 0.29 ms with it).
+template <bool WITHIN = false>
+__device__ __forceinline__ int64_t nearest_leaf(const DevTree &T, double px, double py, double pz,
+                                                double within = INFINITY)
 {
     double best = INFINITY;
     int64_t bi = -1;
+    if (WITHIN && within < INFINITY) {   // the index of a leaf at exactly that distance is below T.n
+        best = within;
+        bi = T.n;
+    }
+    if (WITHIN && !(within >= 0.0)) return -1;   // NaN
     if (T.root == 0) {
         double d2 = d2_point(px, py, pz, ldg4(T.leaf));
-        return d2 < best ? 0 : -1;
+        return d2 < best || (WITHIN && d2 == best && bi > 0) ? 0 : -1;
     }
     const QBox q = make_qbox(px, py, pz);
     int sn[NN_STACK];
@@ -205,7 +215,7 @@ __device__ __forceinline__ int64_t nearest_leaf(const DevTree &T, double px, dou
         }
         if (node == 0) break;
     }
-    return bi;
+    return !WITHIN || bi < T.n ? bi : -1;
 }
 
 // --------------------------------------------------------------------------------------

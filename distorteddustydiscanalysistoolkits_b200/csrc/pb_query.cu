@@ -96,16 +96,14 @@ __global__ void __launch_bounds__(128, 8) k_query(DevTree T, int64_t nq, const d
     }
 }
 
-// the closest accepted leaf of a query: the nearest leaf of all, if it lies within the radius.  It is the
+// the closest accepted leaf of a query: the nearest leaf of all within the radius.  It is the
 // first strictly closer one in DFS order (LinearBVHQueries.jl:33-39,196-203): nearest[i] its index (-1
 // if none), nearest_d2[i] its squared distance (+Inf if none).
 __device__ __forceinline__ void store_closest(const DevTree &T, int64_t i, int64_t b, double px, double py, double pz,
-                                              double r, int64_t *nearest, double *nearest_d2)
+                                              int64_t *nearest, double *nearest_d2)
 {
-    const double d2 = b < 0 ? INFINITY : d2_point(px, py, pz, ldg4(T.leaf + b));
-    const bool in = d2 <= __dmul_rn(r, r) && d2 < INFINITY;
-    if (nearest) nearest[i] = in ? b : -1;
-    if (nearest_d2) nearest_d2[i] = in ? d2 : INFINITY;
+    if (nearest) nearest[i] = b;
+    if (nearest_d2) nearest_d2[i] = b < 0 ? INFINITY : d2_point(px, py, pz, ldg4(T.leaf + b));
 }
 
 __global__ void __launch_bounds__(128) k_closest(DevTree T, int64_t nq, const double *__restrict__ qx,
@@ -113,8 +111,8 @@ __global__ void __launch_bounds__(128) k_closest(DevTree T, int64_t nq, const do
                                                  const double *__restrict__ radius, int64_t *nearest, double *nearest_d2)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nq; i += (int64_t)gridDim.x * blockDim.x) {
-        const double px = __ldg(qx + i), py = __ldg(qy + i), pz = __ldg(qz + i);
-        store_closest(T, i, nearest_leaf(T, px, py, pz), px, py, pz, __ldg(radius + i), nearest, nearest_d2);
+        const double px = __ldg(qx + i), py = __ldg(qy + i), pz = __ldg(qz + i), r = __ldg(radius + i);
+        store_closest(T, i, nearest_leaf<true>(T, px, py, pz, __dmul_rn(r, r)), px, py, pz, nearest, nearest_d2);
     }
 }
 
@@ -126,9 +124,9 @@ __global__ void __launch_bounds__(128) k_closest_warp(DevTree T, int64_t nq, con
     __shared__ int s_stack[4][WSTACK];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     for (int64_t i = blockIdx.x * (int64_t)4 + wib; i < nq; i += (int64_t)gridDim.x * 4) {
-        const double px = __ldg(qx + i), py = __ldg(qy + i), pz = __ldg(qz + i);
-        const int64_t b = nearest_leaf_warp(T, px, py, pz, s_stack[wib], lane);
-        if (lane == 0) store_closest(T, i, b, px, py, pz, __ldg(radius + i), nearest, nearest_d2);
+        const double px = __ldg(qx + i), py = __ldg(qy + i), pz = __ldg(qz + i), r = __ldg(radius + i);
+        const int64_t b = nearest_leaf_warp<true>(T, px, py, pz, s_stack[wib], lane, __dmul_rn(r, r));
+        if (lane == 0) store_closest(T, i, b, px, py, pz, nearest, nearest_d2);
     }
 }
 

@@ -231,13 +231,19 @@ struct WarpWalk {
 // nearest_leaf by a warp: the 32 leaves around the point's place in the Morton order give a first
 // distance, then the lanes take 32 tree entries a round and keep those that may hold a leaf at most
 // that far.  The result is nearest_leaf's: the least squared distance and, among equal ones, the
-// smallest sorted index.  Every lane of the warp calls it; smem holds WSTACK ints.
+// smallest sorted index; WITHIN as there.  Every lane of the warp calls it; smem holds WSTACK ints.
+template <bool WITHIN = false>
 __device__ __forceinline__ int64_t nearest_leaf_warp(const DevTree &T, double px, double py, double pz, int *stack,
-                                                     int lane)
+                                                     int lane, double within = INFINITY)
 {
     const int n = (int)T.n;
     double best = INFINITY;
     int bi = -1;
+    if (WITHIN && within < INFINITY) {
+        best = within;
+        bi = n;
+    }
+    if (WITHIN && !(within >= 0.0)) return -1;   // NaN
     // the warp's least (d2, index) over its lanes' candidates and the best so far
     auto take = [&](double d2, int b) {
         if (!__any_sync(0xffffffffu, d2 < best || (d2 == best && b < bi))) return;
@@ -253,7 +259,7 @@ __device__ __forceinline__ int64_t nearest_leaf_warp(const DevTree &T, double px
     };
     if (T.root == 0) {
         take(lane == 0 ? d2_point(px, py, pz, ldg4(T.leaf)) : INFINITY, 0);
-        return bi;
+        return !WITHIN || bi < n ? bi : -1;
     }
     uint64_t code = 0;
     {
@@ -317,7 +323,7 @@ __device__ __forceinline__ int64_t nearest_leaf_warp(const DevTree &T, double px
         }
         __syncwarp();
     }
-    return bi;
+    return !WITHIN || bi < n ? bi : -1;
 }
 
 // The walk of the j-th listed query (sample point qi at px, py, pz; nearest sorted leaf P.bnear[j]):
