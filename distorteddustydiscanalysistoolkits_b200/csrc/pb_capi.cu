@@ -23,7 +23,7 @@ pb::Handle::~Handle()
     DBuf *all[] = {&in_x, &in_y, &in_z, &in_h, &in_m, &in_rho, &codes, &codes_alt, &idx, &idx_alt, &scan_tmp,
                    &hist, &bbox_part, &qparams, &status, &leaf, &leaf_aux, &odd, &leaf_escape, &node, &node_hmax, &node_child, &node_range, &payload, &counter, &left,
                    &right, &escape, &parent, &bmin64, &bmax64, &hmax64, &counters, &rho_s, &col_ptrs,
-                   &q_x, &q_y, &q_z, &q_keys, &q_keys_alt, &q_perm, &q_perm_alt, &q_out, &q_aux,
+                   &q_x, &q_y, &q_z, &q_keys, &q_keys_alt, &q_perm, &q_perm_alt, &q_out, &q_aux, &q_rest,
                    &pool_runs, &pool_next, &pool_ctr, &items, &wbnear, &qacc, &qflag, &defer_a, &defer_b,
                    &lpt_k, &lpt_v, &lpt_ka, &lpt_va, &iota, &long_list, &long_count, &line_rest, &grid_ax, &grid_out, &mlp_w, &mlp_m, &mlp_v, &mlp_g, &mlp_norm,
                    &mlp_scr, &mlp_idx, &mlp_x, &mlp_y, &mlp_loss, &sched_feat, &sched_pred, &sched_ql, &sched_tmp};

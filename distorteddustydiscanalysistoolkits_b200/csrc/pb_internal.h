@@ -116,7 +116,7 @@ struct Handle {
     DBuf in_pack, q_pack, out_pack;
 
     // query-side scratch
-    DBuf q_x, q_y, q_z, q_keys, q_keys_alt, q_perm, q_perm_alt, q_out, q_aux;
+    DBuf q_x, q_y, q_z, q_keys, q_keys_alt, q_perm, q_perm_alt, q_out, q_aux, q_rest;
     std::vector<DBuf> q_outs;
 
     // timing (CUDA events around the build and the traversal launches)

@@ -73,15 +73,18 @@ struct ListSink {
 };
 
 // gather predicate d2 <= radius^2 (LinearBVHTraversalMacros.jl:26-108), one warp per query (WarpWalk);
-// pool == nullptr counts only
+// pool == nullptr counts only.  rest: the number of queries and the queries to take; NULL: all
 __global__ void __launch_bounds__(128, 8) k_query(DevTree T, int64_t nq, const double *__restrict__ qx,
                                                   const double *__restrict__ qy, const double *__restrict__ qz,
                                                   const double *__restrict__ radius,
-                                                  const int64_t *__restrict__ offsets, int64_t *counts, int64_t *pool)
+                                                  const int64_t *__restrict__ offsets, int64_t *counts, int64_t *pool,
+                                                  const uint32_t *__restrict__ rest)
 {
     __shared__ int s_walk[4][WALK_SMEM];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    for (int64_t i = blockIdx.x * (int64_t)4 + wib; i < nq; i += (int64_t)gridDim.x * 4) {
+    const int64_t todo = rest ? (int64_t)__ldg(rest) : nq;
+    for (int64_t k = blockIdx.x * (int64_t)4 + wib; k < todo; k += (int64_t)gridDim.x * 4) {
+        const int64_t i = rest ? (int64_t)__ldg(rest + 1 + k) : k;
         const double px = __ldg(qx + i), py = __ldg(qy + i), pz = __ldg(qz + i), r = __ldg(radius + i);
         const double r2 = __dmul_rn(r, r);
         const int64_t base = pool ? __ldg(offsets + i) : 0;
@@ -96,6 +99,62 @@ __global__ void __launch_bounds__(128, 8) k_query(DevTree T, int64_t nq, const d
     }
 }
 
+// From QUERY_SHORT_MIN queries on a thread takes up to QUERY_STEPS nodes and leaves of its query's
+// depth-first walk first; a query that is not done then is listed in `rest` and taken by a warp (k_query,
+// which writes the same leaves again, and k_closest_rest).  A query of few leaves needs no more, and a warp's
+// rounds would be mostly idle on it; for others the thread's steps come on top.  Counts on 1e6 particles, a
+// thread for the whole walk / a warp / this: 100,000 points of 0.4 leaves each 0.45 / 0.63 / 0.36 ms, of 15 leaves
+// 1.31 / 0.67 / 0.48, of 339 leaves 8.7 / 0.91 / 0.98; 40,000 points 0.30 / 0.31 / 0.23, 1.09 / 0.33 / 0.28 and
+// 8.2 / 0.46 / 0.53; 20,000 points 0.24 / 0.17 / 0.16, 0.98 / 0.18 / 0.19 and 8.0 / 0.25 / 0.35.  Steps of 64 / 96 /
+// 128 / 192 at 100,000 points: 0.38 / 0.37 / 0.41 / 0.43 (0.4 leaves) and 0.54 / 0.48 / 0.49 / 0.50 (15 leaves).
+constexpr int QUERY_STEPS = 96;
+constexpr int64_t QUERY_SHORT_MIN = 24576;
+
+__global__ void __launch_bounds__(128) k_query_short(DevTree T, int64_t nq, const double *__restrict__ qx,
+                                                     const double *__restrict__ qy, const double *__restrict__ qz,
+                                                     const double *__restrict__ radius,
+                                                     const int64_t *__restrict__ offsets, int64_t *counts, int64_t *pool,
+                                                     int64_t *nearest, double *nearest_d2, uint32_t *rest)
+{
+    const int n = (int)T.n;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nq; i += (int64_t)gridDim.x * blockDim.x) {
+        const double px = __ldg(qx + i), py = __ldg(qy + i), pz = __ldg(qz + i), r = __ldg(radius + i);
+        const double r2 = __dmul_rn(r, r);
+        const QBox q = make_qbox(px, py, pz);
+        const float r2_up = __double2float_ru(r2);
+        const int64_t base = pool ? __ldg(offsets + i) : 0, cap = pool ? __ldg(offsets + i + 1) - base : 0;
+        int node = T.root, ci = -1;
+        int64_t cnt = 0;
+        double cd = INFINITY;
+        for (int s = 0; s < QUERY_STEPS && node != 0; ++s) {
+            if (node >= n) {
+                const int b = node - n;
+                const double d2 = d2_point(px, py, pz, ldg4(T.leaf + b));
+                node = __ldg(T.leaf_escape + b);
+                if (d2 <= r2) {
+                    if (cnt < cap) pool[base + cnt] = b;
+                    ++cnt;
+                    if (d2 < cd) {
+                        cd = d2;
+                        ci = b;
+                    }
+                }
+            } else {
+                const NodeF nd = load_node(T.node + (node - 1));
+                node = node_pruned<GATHER>(T, nd, node, q, 0.f, r2_up) ? nd.escape : nd.left;
+            }
+        }
+        if (node != 0 || T.root == 0) {
+            rest[1 + atomicAdd(rest, 1u)] = (uint32_t)i;
+            continue;
+        }
+        if (pool && cnt > cap) flag(T.status, ST_POOL);
+        if (counts) counts[i] = cnt;
+        if (nearest) nearest[i] = ci;
+        if (nearest_d2) nearest_d2[i] = cd;
+    }
+}
+
 // the closest accepted leaf of a query: the nearest leaf of all within the radius.  It is the
 // first strictly closer one in DFS order (LinearBVHQueries.jl:33-39,196-203): nearest[i] its index (-1
 // if none), nearest_d2[i] its squared distance (+Inf if none).
@@ -106,13 +165,19 @@ __device__ __forceinline__ void store_closest(const DevTree &T, int64_t i, int64
     if (nearest_d2) nearest_d2[i] = b < 0 ? INFINITY : d2_point(px, py, pz, ldg4(T.leaf + b));
 }
 
-__global__ void __launch_bounds__(128) k_closest(DevTree T, int64_t nq, const double *__restrict__ qx,
+template <typename REST>
+__device__ __forceinline__ void closest_by_warps(const DevTree &T, int64_t todo, const double *__restrict__ qx,
                                                  const double *__restrict__ qy, const double *__restrict__ qz,
-                                                 const double *__restrict__ radius, int64_t *nearest, double *nearest_d2)
+                                                 const double *__restrict__ radius, int64_t *nearest, double *nearest_d2,
+                                                 REST query)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nq; i += (int64_t)gridDim.x * blockDim.x) {
+    __shared__ int s_stack[4][WSTACK];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    for (int64_t k = blockIdx.x * (int64_t)4 + wib; k < todo; k += (int64_t)gridDim.x * 4) {
+        const int64_t i = query(k);
         const double px = __ldg(qx + i), py = __ldg(qy + i), pz = __ldg(qz + i), r = __ldg(radius + i);
-        store_closest(T, i, nearest_leaf<true>(T, px, py, pz, __dmul_rn(r, r)), px, py, pz, nearest, nearest_d2);
+        const int64_t b = nearest_leaf_warp<true>(T, px, py, pz, s_stack[wib], lane, __dmul_rn(r, r));
+        if (lane == 0) store_closest(T, i, b, px, py, pz, nearest, nearest_d2);
     }
 }
 
@@ -121,12 +186,24 @@ __global__ void __launch_bounds__(128) k_closest_warp(DevTree T, int64_t nq, con
                                                       const double *__restrict__ radius, int64_t *nearest,
                                                       double *nearest_d2)
 {
-    __shared__ int s_stack[4][WSTACK];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    for (int64_t i = blockIdx.x * (int64_t)4 + wib; i < nq; i += (int64_t)gridDim.x * 4) {
+    closest_by_warps(T, nq, qx, qy, qz, radius, nearest, nearest_d2, [](int64_t k) { return k; });
+}
+
+// the queries that k_query_short left: a warp each for up to NEAREST_WARP_MAX of them, a thread each for more
+__global__ void __launch_bounds__(128) k_closest_rest(DevTree T, const double *__restrict__ qx,
+                                                      const double *__restrict__ qy, const double *__restrict__ qz,
+                                                      const double *__restrict__ radius, int64_t *nearest,
+                                                      double *nearest_d2, const uint32_t *__restrict__ rest)
+{
+    const int64_t todo = __ldg(rest);
+    if (todo <= NEAREST_WARP_MAX) {
+        closest_by_warps(T, todo, qx, qy, qz, radius, nearest, nearest_d2, [&](int64_t k) { return (int64_t)__ldg(rest + 1 + k); });
+        return;
+    }
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < todo; k += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = __ldg(rest + 1 + k);
         const double px = __ldg(qx + i), py = __ldg(qy + i), pz = __ldg(qz + i), r = __ldg(radius + i);
-        const int64_t b = nearest_leaf_warp<true>(T, px, py, pz, s_stack[wib], lane, __dmul_rn(r, r));
-        if (lane == 0) store_closest(T, i, b, px, py, pz, nearest, nearest_d2);
+        store_closest(T, i, nearest_leaf<true>(T, px, py, pz, __dmul_rn(r, r)), px, py, pz, nearest, nearest_d2);
     }
 }
 
@@ -240,18 +317,31 @@ cudaError_t launch_query(Handle *H, const DevTree &T, int64_t nq, const double *
                          const double *qz, const double *radius, const int64_t *offsets, int64_t *counts,
                          int64_t *pool, int64_t *nearest, double *nearest_d2)
 {
+    uint32_t *rest = nullptr;   // what is left after the short queries, if there are many
+    if (nq >= QUERY_SHORT_MIN && nq < 0xffffffffLL) {
+        cudaError_t e = H->q_rest.reserve(sizeof(uint32_t) * (nq + 1));
+        if (!e) e = cudaMemsetAsync(H->q_rest.p, 0, sizeof(uint32_t), H->stream);
+        if (e) return e;
+        rest = H->q_rest.as<uint32_t>();
+        k_query_short<<<grid_for(nq, 128, 1 << 30), 128, 0, H->stream>>>(T, nq, qx, qy, qz, radius, offsets, counts, pool,
+                                                                         nearest, nearest_d2, rest);
+        H->launches += 1;
+    }
     int sms = 148, per = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, H->device);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_query, 128, 0);
     if (counts || pool) {
-        k_query<<<grid_for(nq, 4, 4 * sms * (per > 0 ? per : 1)), 128, 0, H->stream>>>(T, nq, qx, qy, qz, radius, offsets,
-                                                                                       counts, pool);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_query, 128, 0);
+        k_query<<<grid_for(nq, 4, (rest ? 1 : 4) * sms * (per > 0 ? per : 1)), 128, 0, H->stream>>>(
+            T, nq, qx, qy, qz, radius, offsets, counts, pool, rest);
         H->launches += 1;
     }
     if (nearest || nearest_d2) {
-        if (nq <= NEAREST_WARP_MAX)
+        if (rest) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_closest_rest, 128, 0);
+            k_closest_rest<<<sms * (per > 0 ? per : 1), 128, 0, H->stream>>>(T, qx, qy, qz, radius, nearest, nearest_d2, rest);
+        } else {
             k_closest_warp<<<grid_for(nq, 4, 1 << 30), 128, 0, H->stream>>>(T, nq, qx, qy, qz, radius, nearest, nearest_d2);
-        else k_closest<<<grid_for(nq, 128, 1 << 30), 128, 0, H->stream>>>(T, nq, qx, qy, qz, radius, nearest, nearest_d2);
+        }
         H->launches += 1;
     }
     return cudaGetLastError();
