@@ -801,7 +801,7 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
             if (m_heavy > 0)
                 for (const Launch &Lc : launches) {
                     DevCatalog C = dev_catalog(H, Lc, dev.data());
-                    CK(launch_pairs_fp32(&H, T, C, strategy, P, m_heavy, ql, order, dx, dy, dz));
+                    CK(launch_pairs_fp32(&H, T, C, strategy, P, m_heavy, ql, order, dx, dy, dz, mode != 0));
                     H.interp_launches++;
                 }
             if (m_heavy < m)

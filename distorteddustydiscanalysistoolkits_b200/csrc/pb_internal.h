@@ -182,9 +182,10 @@ cudaError_t launch_gather_u32(Handle *H, int64_t m, const uint32_t *order, const
 cudaError_t launch_gather_i32(Handle *H, int64_t m, const uint32_t *order, const int *src, int *dst);
 
 // ---- launchers (pb_interp64.cu / pb_interp32.cu / pb_query.cu) ----
+// classes: the order is by descending size class
 cudaError_t launch_pairs_fp32(Handle *H, const DevTree &T, const DevCatalog &C, int strategy, const RunPool &P,
                               int64_t m, const uint32_t *ql, const uint32_t *order, const double *qx,
-                              const double *qy, const double *qz);
+                              const double *qy, const double *qz, bool classes);
 cudaError_t launch_points_fp64(Handle *H, const DevTree &T, const DevCatalog &C, int strategy, int64_t nq,
                                const double *qx, const double *qy, const double *qz, const uint32_t *perm,
                                int64_t npts);

@@ -48,10 +48,17 @@ __global__ void __launch_bounds__(128) k_points32w(DevTree T, DevCatalog C, cons
 // Pair kernel of the two-phase path: a warp takes a walked query (heaviest first), reads its
 // runs chunk by chunk, and deals the accepted
 // leaves to its lanes in DFS order -- the k-th accepted leaf to lane k mod 32, exactly as the
-// fused kernel does, so both produce the same bits.  A block takes four queries that follow each other
-// in the order (one size class, Morton order): its warps read the same particles at about the same
-// time (L1 hits 7 -> 19 % on 221,184 points of the 2^21-particle disc, 26.7 -> 25.0 ms).
-template <int STRAT, int KT, int CAT>
+// fused kernel does, so both produce the same bits.  TOGETHER: a block takes four queries that follow
+// each other in the order (one size class, Morton order), so that its warps read the same particles at
+// about the same time (L1 hits 7 -> 19 % on 221,184 points of the 2^21-particle disc, 26.7 -> 25.0 ms).
+// The block waits for the slowest of the four, which costs more than it gives where there are few
+// queries a warp, or no size classes to make the four alike (the plain order): a warp each then.
+// Together / a warp each, 2^20 particles: 269,000 queries 223.6 / 227.2 ms, 81,407 67.8 / 68.6, 32,946 28.6 / 28.8,
+// 9,910 14.4 / 13.6, 4,237 14.2 / 10.9, 1,329 13.9 / 9.5; plain order 269,000 237.0 / 230.3, 1,329 9.2 / 8.6.
+// (A choice at run time inside one kernel spoils the code of the single warps: 4,237 queries 12.4 ms.)
+constexpr int TOGETHER_MIN = 8;   // queries a resident warp
+
+template <int STRAT, int KT, int CAT, bool TOGETHER>
 __global__ void __launch_bounds__(128, 5) k_pairs32w(DevTree T, DevCatalog C, const float4 *__restrict__ pay, int stride,
                                                   RunPool P, int64_t m, const uint32_t *__restrict__ ql,
                                                   const uint32_t *__restrict__ order, const double *__restrict__ qx,
@@ -60,14 +67,20 @@ __global__ void __launch_bounds__(128, 5) k_pairs32w(DevTree T, DevCatalog C, co
 {
     __shared__ double s_acc[ACC_SLOTS * ACC_STRIDE];   // FP64 sums, slot k of thread t at [k * 128 + t]
     const int lane = threadIdx.x & 31;
-    __shared__ unsigned long long s_next;
     for (;;) {
-        __syncthreads();   // every warp has read the last ticket
-        if (threadIdx.x == 0) s_next = atomicAdd(counter, 4ULL);
-        __syncthreads();
-        if ((int64_t)s_next >= m) break;
-        const int64_t t = (int64_t)s_next + (threadIdx.x >> 5);
-        if (t >= m) continue;
+        int64_t t;
+        if (TOGETHER) {
+            __shared__ unsigned long long s_next;
+            __syncthreads();   // every warp has read the last ticket
+            if (threadIdx.x == 0) s_next = atomicAdd(counter, 4ULL);
+            __syncthreads();
+            if ((int64_t)s_next >= m) break;
+            t = (int64_t)s_next + (threadIdx.x >> 5);
+            if (t >= m) continue;
+        } else {
+            t = next_query(counter, lane);
+            if (t >= m) break;
+        }
         const int64_t j = order ? (int64_t)__ldg(order + t) : t;
         if (__ldg(P.qflag + j)) continue;
         const int64_t qi = __ldg(ql + j);
@@ -136,45 +149,49 @@ cudaError_t launch_points_fp32(Handle *H, const DevTree &T, const DevCatalog &C,
 template <int STRAT, int KT, int CAT>
 static void launch_pairs_one(Handle *H, const DevTree &T, const DevCatalog &C, const float4 *pay, int stride,
                              const RunPool &P, int64_t m, const uint32_t *ql, const uint32_t *order, const double *qx,
-                             const double *qy, const double *qz, unsigned long long *ctr)
+                             const double *qy, const double *qz, unsigned long long *ctr, bool classes)
 {
-    const int bs = 128;
-    k_pairs32w<STRAT, KT, CAT><<<persistent_grid((const void *)k_pairs32w<STRAT, KT, CAT>, bs), bs, 0, H->stream>>>(
-        T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr);
+    const int bs = 128, grid = persistent_grid((const void *)k_pairs32w<STRAT, KT, CAT, true>, bs);
+    if (classes && m >= (int64_t)TOGETHER_MIN * (bs / 32) * grid) {
+        k_pairs32w<STRAT, KT, CAT, true><<<grid, bs, 0, H->stream>>>(T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr);
+    } else {
+        k_pairs32w<STRAT, KT, CAT, false><<<persistent_grid((const void *)k_pairs32w<STRAT, KT, CAT, false>, bs), bs, 0,
+                                           H->stream>>>(T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr);
+    }
 }
 
 template <int STRAT, int KT>
 static void launch_pairs_cat(Handle *H, const DevTree &T, const DevCatalog &C, const float4 *pay, int stride,
                              const RunPool &P, int64_t m, const uint32_t *ql, const uint32_t *order, const double *qx,
-                             const double *qy, const double *qz, unsigned long long *ctr)
+                             const double *qy, const double *qz, unsigned long long *ctr, bool classes)
 {
     switch (catalog_shape(C)) {
-    case CAT_GDC4: launch_pairs_one<STRAT, KT, CAT_GDC4>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
-    case CAT_C4: launch_pairs_one<STRAT, KT, CAT_C4>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
-    case CAT_S1: launch_pairs_one<STRAT, KT, CAT_S1>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
-    case CAT_SG1: launch_pairs_one<STRAT, KT, CAT_SG1>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
-    default: launch_pairs_one<STRAT, KT, CAT_ANY>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
+    case CAT_GDC4: launch_pairs_one<STRAT, KT, CAT_GDC4>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
+    case CAT_C4: launch_pairs_one<STRAT, KT, CAT_C4>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
+    case CAT_S1: launch_pairs_one<STRAT, KT, CAT_S1>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
+    case CAT_SG1: launch_pairs_one<STRAT, KT, CAT_SG1>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
+    default: launch_pairs_one<STRAT, KT, CAT_ANY>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
     }
 }
 
 template <int STRAT>
 static void launch_pairs_kt(Handle *H, const DevTree &T, const DevCatalog &C, const float4 *pay, int stride,
                             const RunPool &P, int64_t m, const uint32_t *ql, const uint32_t *order, const double *qx,
-                            const double *qy, const double *qz, unsigned long long *ctr)
+                            const double *qy, const double *qz, unsigned long long *ctr, bool classes)
 {
     switch (T.kernel) {
-    case 0: launch_pairs_cat<STRAT, 0>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
-    case 1: launch_pairs_cat<STRAT, 1>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
-    case 2: launch_pairs_cat<STRAT, 2>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
-    case 3: launch_pairs_cat<STRAT, 3>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
-    case 4: launch_pairs_cat<STRAT, 4>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
-    default: launch_pairs_cat<STRAT, 5>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
+    case 0: launch_pairs_cat<STRAT, 0>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
+    case 1: launch_pairs_cat<STRAT, 1>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
+    case 2: launch_pairs_cat<STRAT, 2>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
+    case 3: launch_pairs_cat<STRAT, 3>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
+    case 4: launch_pairs_cat<STRAT, 4>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
+    default: launch_pairs_cat<STRAT, 5>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
     }
 }
 
 cudaError_t launch_pairs_fp32(Handle *H, const DevTree &T, const DevCatalog &C, int strategy, const RunPool &P,
                               int64_t m, const uint32_t *ql, const uint32_t *order, const double *qx,
-                              const double *qy, const double *qz)
+                              const double *qy, const double *qz, bool classes)
 {
     int stride = payload_stride(C.nU);
     cudaError_t e = H->payload.reserve(sizeof(float4) * payload_float4s(T.n, stride));
@@ -186,9 +203,9 @@ cudaError_t launch_pairs_fp32(Handle *H, const DevTree &T, const DevCatalog &C, 
     k_payload<<<grid_for(T.n, 256), 256, 0, H->stream>>>(T.n, T, C, pay, stride);
     cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), H->stream);
     switch (strategy) {
-    case GATHER: launch_pairs_kt<GATHER>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
-    case SCATTER: launch_pairs_kt<SCATTER>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
-    default: launch_pairs_kt<SYMMETRIC>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr); break;
+    case GATHER: launch_pairs_kt<GATHER>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
+    case SCATTER: launch_pairs_kt<SCATTER>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
+    default: launch_pairs_kt<SYMMETRIC>(H, T, C, pay, stride, P, m, ql, order, qx, qy, qz, ctr, classes); break;
     }
     H->launches += 2;
     return cudaGetLastError();
