@@ -13,6 +13,13 @@ namespace pb {
 // walk's work grows with the surface of the support).  The nearest search lists them, and the walk
 // takes them first: in Morton order they come last where a grid's corner lies far from the particles,
 // and the launch waited for them (SMs busy 72 % of the walk of 131,072 particles on 64^3 points).
+// Where h varies by less than that (a box of even density) every query would be on the list, walked out of
+// Morton order, a ticket each, and passed over again: with more than one query in LONG_SHARE on it the list is
+// not used.  A disc in a box has between a quarter and a half of the points on it.  Walk with shares of 1 / 2 / 4 /
+// 16: 1e6 even particles, 2e6 points 10.44 / 9.79 / 9.79 / 9.79 ms; 131,072 disc particles, 64^3 points 2.01 / 2.01 /
+// 2.41 / 2.40, 400,000 on 80 x 80 x 24 2.39 / 2.38 / 2.97 / 2.97, 2^21 on 256 x 256 x 64 97.4 / 97.4 / 97.4 / 103.0.
+constexpr int LONG_SHARE = 2;
+
 __device__ __forceinline__ bool long_walk(const DevTree &T, int b)
 {
     if (T.root == 0 || b < 0) return false;
@@ -20,13 +27,23 @@ __device__ __forceinline__ bool long_walk(const DevTree &T, int b)
 }
 
 struct LongList {
-    uint32_t *list;    // NULL: none
-    unsigned *count;
+    uint32_t *list;    // cap entries; NULL: none
+    unsigned *count;   // above cap: the list is not used
+    unsigned cap;
     __device__ __forceinline__ void add(const DevTree &T, int64_t j, int b) const
     {
-        if (list && long_walk(T, b)) list[atomicAdd(count, 1u)] = (uint32_t)j;
+        if (!list || !long_walk(T, b)) return;
+        const unsigned at = atomicAdd(count, 1u);
+        if (at < cap) list[at] = (uint32_t)j;
     }
+    __device__ __forceinline__ int64_t used() const { return list && *count <= cap ? (int64_t)*count : 0; }
 };
+
+// the list of a launch over m queries
+static LongList long_list(Handle *H, int64_t m, bool listed)
+{
+    return LongList{listed ? H->long_list.as<uint32_t>() : nullptr, H->long_count.as<unsigned>(), (unsigned)(m / LONG_SHARE + 1)};
+}
 
 __global__ void __launch_bounds__(128) k_nearest_list(DevTree T, int64_t m, const uint32_t *__restrict__ ql,
                                                       const double *__restrict__ qx, const double *__restrict__ qy,
@@ -70,7 +87,7 @@ __global__ void __launch_bounds__(128, 8) k_walk(DevTree T, RunPool P, int64_t m
     __shared__ int s_walk[4][RUN_WALK_SMEM];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const double K = kernel_valid(T.kernel);
-    const int64_t nlong = longs.list ? min((int64_t)*longs.count, m) : 0;
+    const int64_t nlong = longs.used();
     // tickets: the listed queries one by one, then all others, `ticket` at a time
     for (;;) {
         const int64_t t = next_query(counter, lane);
@@ -170,10 +187,10 @@ cudaError_t launch_nearest_list(Handle *H, const DevTree &T, int64_t m, const ui
                                 const double *qy, const double *qz, int *bnear, bool listed)
 {
     cudaError_t e;
-    if (listed && ((e = H->long_list.reserve(sizeof(uint32_t) * m)) || (e = H->long_count.reserve(sizeof(unsigned))) ||
+    if (listed && ((e = H->long_list.reserve(sizeof(uint32_t) * (m / LONG_SHARE + 1))) || (e = H->long_count.reserve(sizeof(unsigned))) ||
                    (e = cudaMemsetAsync(H->long_count.p, 0, sizeof(unsigned), H->stream))))
         return e;
-    const LongList L{listed ? H->long_list.as<uint32_t>() : nullptr, H->long_count.as<unsigned>()};
+    const LongList L = long_list(H, m, listed);
     if (m <= NEAREST_WARP_MAX)
         k_nearest_list_warp<<<grid_for(m, 4, 1 << 30), 128, 0, H->stream>>>(T, m, ql, qx, qy, qz, bnear, L);
     else k_nearest_list<<<grid_for(m, 128, 1 << 30), 128, 0, H->stream>>>(T, m, ql, qx, qy, qz, bnear, L);
@@ -197,7 +214,7 @@ cudaError_t launch_walk(Handle *H, const DevTree &T, int strategy, const RunPool
     if (m <= 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), H->stream);
     if (e) return e;
-    const LongList L{listed ? H->long_list.as<uint32_t>() : nullptr, H->long_count.as<unsigned>()};
+    const LongList L = long_list(H, m, listed);
     switch (strategy) {
     case GATHER: launch_walk_strat<GATHER>(H, T, P, m, ql, qx, qy, qz, L, counter); break;
     case SCATTER: launch_walk_strat<SCATTER>(H, T, P, m, ql, qx, qy, qz, L, counter); break;
