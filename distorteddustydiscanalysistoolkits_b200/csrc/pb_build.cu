@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_pass(int64_t n, const K *__re
                                                         const uint32_t *__restrict__ vin, K *kout, uint32_t *vout,
                                                         int shift, const uint32_t *__restrict__ hist, unsigned *ticket,
                                                         unsigned long long *look, unsigned long long *look_next,
-                                                        int *status)
+                                                        unsigned wait)
 {
     constexpr int ITEMS = rs_items<K>(), TILE = rs_tile<K>();
     __shared__ K s_key[TILE];
@@ -272,13 +272,13 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_pass(int64_t n, const K *__re
     uint32_t before = 0;
     for (int64_t t = tile - 1; t >= 0;) {
         unsigned long long v = words[t * 256 + d];
-        for (unsigned spin = 0; v >> 32 == 0; ++spin) {
-            if (spin > (1u << 22)) {   // never: the tile is running and waits for nothing before it publishes
-                atomicOr(status, ST_SORT);
-                v = rs_word(2, 0);
-                break;
-            }
-            v = words[t * 256 + d];
+        for (unsigned spin = 0; v >> 32 == 0 && spin < wait; ++spin) v = words[t * 256 + d];
+        if (v >> 32 == 0) {
+            // hardly ever: that tile is running and waits for nothing before it publishes.  This one then
+            // waits no longer and counts the keys of that tile and of those before it itself.
+            uint32_t c = 0;
+            for (int64_t i = 0; i < (t + 1) * TILE; ++i) c += ((unsigned)(kin[i] >> shift) & 255u) == (unsigned)d;
+            v = rs_word(2, c);
         }
         before += (uint32_t)v;
         if (v >> 32 == 2) break;
@@ -341,7 +341,7 @@ static cudaError_t sort_pairs(Handle *H, K *keys, uint32_t *vals, K *kalt, uint3
     uint32_t *vs = vals, *vd = valt;
     for (int p = 0; p < passes; ++p) {
         k_rs_pass<K><<<(unsigned)tiles, RS_THREADS, 0, H->stream>>>(n, src, vs, dst, vd, 8 * p, hist + 256 * p, ticket + p,
-                                                                   look[p & 1], look[(p + 1) & 1], H->status.as<int>());
+                                                                   look[p & 1], look[(p + 1) & 1], (unsigned)H->sort_wait);
         std::swap(src, dst);
         std::swap(vs, vd);
     }

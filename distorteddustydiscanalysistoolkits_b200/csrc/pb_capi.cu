@@ -139,7 +139,6 @@ int check_status(Handle &H)
     if (st & ST_NONFINITE) return fail(H, PB_ERR_INVALID, "non-finite particle coordinate or smoothing length");
     if (st & ST_REFIT) return fail(H, PB_ERR_INTERNAL, "LBVH refit: an internal node was not combined exactly twice");
     if (st & ST_TRAVERSAL) return fail(H, PB_ERR_INTERNAL, "traversal exceeded its iteration bound");
-    if (st & ST_SORT) return fail(H, PB_ERR_INTERNAL, "radix sort: a tile waited too long for the one before it");
     if (st & ST_POOL)
         return fail(H, PB_ERR_DIMENSION, "neighbour pool offsets too small for a query (DimensionMismatch)");
     return PB_OK;
@@ -1041,6 +1040,9 @@ int32_t pb_set_option(pb_handle *h, const char *name, int64_t value)
     } else if (!strcmp(name, "leaf_size")) {
         if (value < 1 || value > 64) return fail(H, PB_ERR_INVALID, "leaf_size must be in 1..64");
         H.leaf_size = (int)value;
+    } else if (!strcmp(name, "sort_wait")) {
+        if (value < 0 || value > 0x7fffffffLL) return fail(H, PB_ERR_INVALID, "sort_wait out of range");
+        H.sort_wait = value;
     } else if (!strcmp(name, "batch_order")) {
         if (value < 0 || value > 1) return fail(H, PB_ERR_INVALID, "batch_order must be 0 (given) or 1 (most work first)");
         H.batch_order = (int)value;

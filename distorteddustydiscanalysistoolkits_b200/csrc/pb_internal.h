@@ -126,6 +126,7 @@ struct Handle {
     float t_phase_ms[3] = {0.f, 0.f, 0.f};   // nearest search, walk (+ ordering), pairs; all slices and rounds
     int64_t interp_launches = 0;
     int sort_queries = 1;
+    int64_t sort_wait = int64_t(1) << 22;   // reads of a look-back word before a sort tile counts for itself
     int block_size = 128;
 
     ~Handle();
