@@ -37,6 +37,7 @@ pb::Handle::~Handle()
         b->release();
     if (batch_host) cudaFreeHost(batch_host);
     if (pin) cudaFreeHost(pin);
+    free(pack);
     for (DBuf *b : {&in_pack, &q_pack, &out_pack}) b->release();
     for (auto &b : in_cols) b.release();
     for (auto &b : cols_s) b.release();
@@ -96,16 +97,48 @@ cudaError_t stage_in(Handle &H, DBuf &buf, const void *p, size_t bytes, const vo
     return e;
 }
 
-// Page-locked staging of a handle: PIN_WORDS bytes for words that the host reads back, then PIN_MAX
-// bytes through which small host arrays travel packed, in one copy instead of one per array (a copy
-// from or to pageable memory costs 5 to 12 us of host time each: 39 of them were 1 ms of a call on
-// 6,000 particles and 2,744 points).  Every use ends in the call's own synchronisation, and calls on a
+// Staging of a handle: small host arrays travel packed, in one copy instead of one per array (a copy from or
+// to pageable memory costs 5 to 12 us of host time each: 39 of them were 1 ms of a call on 6,000 particles and
+// 2,744 points), and the host reads a few words back.  The packed block is ordinary memory at first and
+// page-locked from the `pin_after`-th status read on (one of a build, one of an interpolation):
+// page-locking costs 0.8 to 2.5 ms whatever the size and saves 0.16 ms of such a call (0.79 -> 0.63 ms), so a
+// handle of few calls never pays for it.  First call on a new handle, 500 / 6,000 / 20,000 particles: one copy per
+// array 2.75 / 3.7 / 5.9 ms, page-locked at once 3.2 / 4.1 / 5.5, now 1.0 / 2.1 / 3.6.  Where page-locked memory is
+// not to be had the block stays as it is.  Every use ends in the call's own synchronisation, and calls on a
 // handle do not overlap.
 constexpr size_t PIN_WORDS = 256, PIN_MAX = size_t(2) << 20;
 
-cudaError_t pin_reserve(Handle &H)
+void count_status_read(Handle &H)
 {
-    return H.pin ? cudaSuccess : cudaMallocHost(reinterpret_cast<void **>(&H.pin), PIN_WORDS + PIN_MAX);
+    if (H.pin || H.pin_failed || H.pin_after <= 0 || ++H.pin_uses < H.pin_after) return;
+    if (cudaMallocHost(reinterpret_cast<void **>(&H.pin), PIN_WORDS + PIN_MAX)) {
+        cudaGetLastError();
+        H.pin = nullptr;
+        H.pin_failed = true;
+    }
+}
+
+// where the next packed copy of up to PIN_MAX bytes goes (its contents are not kept from one to the next);
+// NULL: no memory
+unsigned char *pack_block(Handle &H, size_t bytes)
+{
+    if (H.pin) return H.pin + PIN_WORDS;
+    if (H.pack_bytes < bytes) {
+        free(H.pack);
+        H.pack = static_cast<unsigned char *>(malloc(bytes));
+        H.pack_bytes = H.pack ? bytes : 0;
+    }
+    return H.pack;
+}
+
+// up to PIN_WORDS bytes of device memory, once the stream's work is done
+cudaError_t read_words(Handle &H, const void *dev, size_t bytes, void *out)
+{
+    void *at = H.pin ? H.pin : out;
+    cudaError_t e = cudaMemcpyAsync(at, dev, bytes, cudaMemcpyDeviceToHost, H.stream);
+    if (!e) e = cudaStreamSynchronize(H.stream);
+    if (!e && H.pin) memcpy(out, at, bytes);
+    return e;
 }
 
 // whether k arrays of `bytes` each go packed: all in host memory, and small
@@ -120,22 +153,23 @@ bool packs(const Handle &H, const void *const *p, int k, size_t bytes)
 // device views of k host arrays through one packed copy
 cudaError_t pack_in(Handle &H, DBuf &buf, const void *const *p, int k, size_t bytes, const void **out)
 {
-    cudaError_t e;
-    if ((e = pin_reserve(H)) || (e = buf.reserve(bytes * k))) return e;
+    cudaError_t e = buf.reserve(bytes * k);
+    if (e) return e;
+    unsigned char *block = pack_block(H, bytes * k);
+    if (!block) return cudaErrorMemoryAllocation;
     for (int i = 0; i < k; ++i) {
-        memcpy(H.pin + PIN_WORDS + i * bytes, p[i], bytes);
+        memcpy(block + i * bytes, p[i], bytes);
         out[i] = buf.as<unsigned char>() + i * bytes;
     }
-    return cudaMemcpyAsync(buf.p, H.pin + PIN_WORDS, bytes * k, cudaMemcpyHostToDevice, H.stream);
+    return cudaMemcpyAsync(buf.p, block, bytes * k, cudaMemcpyHostToDevice, H.stream);
 }
 
-int check_status(Handle &H)
+// waits for the stream's work; `via`: the handle of the same stream through whose words the status is read
+int check_status(Handle &H, Handle &via)
 {
-    CK(pin_reserve(H));
-    volatile int *word = reinterpret_cast<volatile int *>(H.pin);
-    CK(cudaMemcpyAsync(H.pin, H.status.p, sizeof(int), cudaMemcpyDeviceToHost, H.stream));
-    CK(cudaStreamSynchronize(H.stream));
-    const int st = *word;
+    int st = 0;
+    CK(read_words(via, H.status.p, sizeof(int), &st));
+    if (&via == &H) count_status_read(H);
     if (st & ST_NONFINITE) return fail(H, PB_ERR_INVALID, "non-finite particle coordinate or smoothing length");
     if (st & ST_REFIT) return fail(H, PB_ERR_INTERNAL, "LBVH refit: an internal node was not combined exactly twice");
     if (st & ST_TRAVERSAL) return fail(H, PB_ERR_INTERNAL, "traversal exceeded its iteration bound");
@@ -143,6 +177,8 @@ int check_status(Handle &H)
         return fail(H, PB_ERR_DIMENSION, "neighbour pool offsets too small for a query (DimensionMismatch)");
     return PB_OK;
 }
+
+int check_status(Handle &H) { return check_status(H, H); }
 
 DevTree make_tree(Handle &H)
 {
@@ -367,7 +403,6 @@ int stage_outputs(Handle &H, int64_t L, int64_t npts, double *const *out, std::v
     if ((int64_t)H.q_outs.size() < L) H.q_outs.resize(L);
     const size_t nb = sizeof(double) * npts;
     if (out && L <= 1024 && packs(H, reinterpret_cast<const void *const *>(out), (int)L, nb)) {
-        CK(pin_reserve(H));
         CK(H.out_pack.reserve(nb * L));
         for (int64_t l = 0; l < L; ++l) dev[l] = H.out_pack.as<double>() + l * npts;
         is_host.assign(L, 2);
@@ -391,9 +426,11 @@ int finish_outputs(Handle &H, int64_t L, int64_t npts, double *const *out, const
 {
     const size_t nb = sizeof(double) * npts;
     if (is_host[0] == 2) {
-        CK(cudaMemcpyAsync(H.pin + PIN_WORDS, H.out_pack.p, nb * L, cudaMemcpyDeviceToHost, H.stream));
+        unsigned char *block = pack_block(H, nb * L);
+        CK(block ? cudaSuccess : cudaErrorMemoryAllocation);
+        CK(cudaMemcpyAsync(block, H.out_pack.p, nb * L, cudaMemcpyDeviceToHost, H.stream));
         const int rc = check_status(H);   // waits
-        for (int64_t l = 0; l < L; ++l) memcpy(out[l], H.pin + PIN_WORDS + l * nb, nb);
+        for (int64_t l = 0; l < L; ++l) memcpy(out[l], block + l * nb, nb);
         return rc;
     }
     for (int64_t l = 0; l < L; ++l)
@@ -528,15 +565,18 @@ int do_build(Handle &H, const pb_input *in, int32_t flags)
     std::vector<double *> dcol(ncol);
     for (int c = 0; c < ncol; ++c) dcol[c] = const_cast<double *>(cols[c]);
     const bool permute = flags & PB_PERMUTE_CALLER;
+    unsigned char *block = nullptr;
     if (permute && packed) {   // back in one copy; the caller's arrays are written if the build succeeded
         CK(launch_sorted_columns(&H, n, dev, dcol));
-        CK(cudaMemcpyAsync(H.pin + PIN_WORDS, H.in_pack.p, nb * (6 + ncol), cudaMemcpyDeviceToHost, H.stream));
+        block = pack_block(H, nb * (6 + ncol));
+        CK(block ? cudaSuccess : cudaErrorMemoryAllocation);
+        CK(cudaMemcpyAsync(block, H.in_pack.p, nb * (6 + ncol), cudaMemcpyDeviceToHost, H.stream));
     }
     int rc = check_status(H);
     if (rc) return rc;
     H.t_build_ms = ev_ms(H, 0, 1);
     if (permute && packed) {
-        for (int a = 0; a < 6 + ncol; ++a) memcpy(const_cast<void *>(src[a]), H.pin + PIN_WORDS + a * nb, nb);
+        for (int a = 0; a < 6 + ncol; ++a) memcpy(const_cast<void *>(src[a]), block + a * nb, nb);
     } else if (permute) {
         CK(launch_sorted_columns(&H, n, dev, dcol));
         for (int a = 0; a < 6 + ncol; ++a)
@@ -785,11 +825,8 @@ int two_phase_points(Handle &H, const DevTree &T, const std::vector<Launch> &lau
             uint32_t *order = nullptr;
             CK(launch_split_order(&H, P, m, (unsigned)H.light_max, mode == 0, &order, ctr + 4));
             // the pool use, the deferred and the heavy queries and the pairs are final here
-            CK(pin_reserve(H));
-            CK(cudaMemcpyAsync(H.pin, ctr, 6 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, H.stream));
-            CK(cudaStreamSynchronize(H.stream));
             unsigned long long used_nd[6];
-            memcpy(used_nd, H.pin, sizeof(used_nd));
+            CK(read_words(H, ctr, sizeof(used_nd), used_nd));
             const unsigned nd = (unsigned)(used_nd[1] & 0xffffffffULL);
             const int64_t m_heavy = (int64_t)(used_nd[1] >> 32), light_pairs = (int64_t)used_nd[5];
             // the plain order is not sorted: no block queries there
@@ -1040,6 +1077,9 @@ int32_t pb_set_option(pb_handle *h, const char *name, int64_t value)
     } else if (!strcmp(name, "leaf_size")) {
         if (value < 1 || value > 64) return fail(H, PB_ERR_INVALID, "leaf_size must be in 1..64");
         H.leaf_size = (int)value;
+    } else if (!strcmp(name, "pin_after")) {
+        if (value < 0 || value > 0x7fffffffLL) return fail(H, PB_ERR_INVALID, "pin_after out of range");
+        H.pin_after = value;
     } else if (!strcmp(name, "sort_wait")) {
         if (value < 0 || value > 0x7fffffffLL) return fail(H, PB_ERR_INVALID, "sort_wait out of range");
         H.sort_wait = value;
@@ -1545,7 +1585,7 @@ int check_statuses(pb_handle *const *discs, int32_t ndiscs)
         return batch_fail(discs[0], PB_ERR_CUDA, std::string("batched launch: ") + cudaGetErrorString(e));
     }
     for (int32_t k = 0; k < ndiscs; ++k) {
-        int rc = check_status(discs[k]->H);
+        int rc = check_status(discs[k]->H, H0);
         if (rc) return batch_fail(discs[0], rc, "disc " + std::to_string(k) + ": " + discs[k]->H.err);
     }
     return PB_OK;

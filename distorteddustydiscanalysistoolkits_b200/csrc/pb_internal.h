@@ -111,8 +111,12 @@ struct Handle {
     DBuf batch_slot_of;      // processing slot of every point of a slice
     DBuf batch_mk, batch_mka, batch_mv, batch_mva;         // Morton walk order of a slice
 
-    // page-locked staging: words the host reads back, and small host arrays packed into one copy
-    unsigned char *pin = nullptr;
+    // staging of small host arrays packed into one copy (ordinary memory, then page-locked) and of the words
+    // the host reads back
+    unsigned char *pack = nullptr, *pin = nullptr;
+    size_t pack_bytes = 0;
+    int64_t pin_after = 32, pin_uses = 0;   // 0: never page-locked
+    bool pin_failed = false;
     DBuf in_pack, q_pack, out_pack;
 
     // query-side scratch

@@ -92,8 +92,10 @@ int32_t pb_set_stream(pb_handle *h, void *cuda_stream);
    "schedule" (points: 0 plain = input order, no ordering; 1 tuned = Morton order, heaviest
    sums first (default); 2 learned = tuned plus binning by predicted work; results are
    identical), "slice_queries" (queries per
-   walk/sum slice, default 2^22), "sort_wait" (reads of another tile's count in the radix sorts before
-   a tile counts for itself, default 2^22; results are identical). */
+   walk/sum slice, default 2^22), "pin_after" (builds, interpolations and queries on the handle after
+   which its staging of small host arrays is page-locked, 2 MiB; default 32, 0 never), "sort_wait" (reads of
+   another tile's count in the radix sorts before a tile counts for itself, default 2^22; results are
+   identical). */
 int32_t pb_set_option(pb_handle *h, const char *name, int64_t value);
 
 /* LinearBVH!(input, Val(3)) (InterpolationInput.jl:203-223): MortonEncoding
