@@ -430,6 +430,7 @@ int finish_outputs(Handle &H, int64_t L, int64_t npts, double *const *out, const
         CK(block ? cudaSuccess : cudaErrorMemoryAllocation);
         CK(cudaMemcpyAsync(block, H.out_pack.p, nb * L, cudaMemcpyDeviceToHost, H.stream));
         const int rc = check_status(H);   // waits
+        if (rc == PB_ERR_CUDA) return rc;   // the block was not filled
         for (int64_t l = 0; l < L; ++l) memcpy(out[l], block + l * nb, nb);
         return rc;
     }
