@@ -9,16 +9,16 @@ separate calls (tests/test_gpu_batch.py).
 
 The autotuner times the interpolation of a representative job of each size class (particles
 and points rounded to powers of 4) under every candidate setting of the slice size and the
-scheduler bin width (the walk split, still a candidate, no longer has an effect), and keeps the
-fastest.
+scheduler bin width, and keeps the fastest.  The walk split has no effect any more: it is taken as an
+option, but only one value of it is tried unless more are asked for.
 
 ``DeviceBatch`` is the one-launch form: every disc's particles, sample points and outputs stay
 on the device, each disc has its own handle (its tree), all handles share one stream, and a
 step enqueues every disc's LBVH build (PB_BUILD_ASYNC) and one pb_batch_points launch that
 interpolates the sample points of all discs.  The step can be captured in a CUDA graph and
-replayed.  ``BatchAutotuner`` picks its schedule options -- the fused
-fallback's leaf size (subtrees of at most that many leaves scanned linearly), the disc order (given or most work first) and the
-blocks per SM -- by timing graph replays; outputs do not depend on them.
+replayed.  ``BatchAutotuner`` picks its schedule options -- the fused fallback's leaf size (subtrees
+of at most that many leaves scanned linearly), the disc order (given or most work first) and the blocks
+per SM -- by timing graph replays; outputs do not depend on them.
 """
 import ctypes
 import itertools
@@ -60,8 +60,7 @@ def size_class(n_particles, n_points):
 class Autotuner:
     """Per size class, the fastest of the candidate schedule options (results are unaffected)."""
 
-    def __init__(self, walk_split=(16, 32, 64, 128), slice_queries=(1 << 20, 1 << 22), bin_width=(0.5, 1.0, 2.0),
-                 repeats=2):
+    def __init__(self, walk_split=(64,), slice_queries=(1 << 20, 1 << 22), bin_width=(0.5, 1.0, 2.0), repeats=2):
         self.grid = {"walk_split": walk_split, "slice_queries": slice_queries, "bin_width": bin_width}
         self.repeats = repeats
         self.table = {}
@@ -239,8 +238,7 @@ class BatchAutotuner:
     """Schedule options of a DeviceBatch (outputs do not depend on them): every combination of
     the candidates is captured and timed over `repeats` graph replays; the fastest is kept."""
 
-    def __init__(self, leaf_size=(1, 4, 8, 16), order=(0, 1), blocks_per_sm=(0, 2), walk_split=(8, 16, 32),
-                 repeats=2):
+    def __init__(self, leaf_size=(1, 4, 8, 16), order=(0, 1), blocks_per_sm=(0, 2), walk_split=(16,), repeats=2):
         self.grid = {"leaf_size": leaf_size, "order": order, "blocks_per_sm": blocks_per_sm, "walk_split": walk_split}
         self.repeats = repeats
         self.best = None
