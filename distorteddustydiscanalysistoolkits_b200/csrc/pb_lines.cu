@@ -297,12 +297,13 @@ __global__ void __launch_bounds__(128) k_lines_warp(DevTree T, DevCatalog C, int
 // directions, and tiles whose lines share few of their leaves (fewer than 1 in LTILE_SHARE tests passed after
 // LTILE_PROBE leaves, and after twice as many, and so on: a tile that lies across a jump of the Morton
 // order, or lines in no order at all), are left to k_lines_warp, tile by tile in `rest`.  Taking them here,
-// 32 lines one after the other, made one warp the end of the launch: 363^2 lines of 1.5e6 particles 36.3 ms,
-// now 6.3; 400^2 with origins at scattered depths 50.2, now 12.6.  Shares of 4 / 8 / 16 / 32: 6.9 / 6.3 / 7.3 / 8.2
-// and 12.9 / 12.6 / 14.3 / 18.3 ms; images in order are within 5 % (1024^2 17.3 / 16.6 / 16.6 / 16.6).
+// 32 lines one after the other, made one warp the end of the launch: 363^2 lines of 1.5e6 particles (M5) 36.3 ms,
+// now 6.7; 400^2 with origins at scattered depths 50.2, now 13.1.  Shares of 4 / 8 / 12 / 16 / 32: 363^2 6.9 / 6.3 /
+// 6.7 / 7.3 / 8.2, 400^2 at depths 12.9 / 12.6 / 13.1 / 14.3 / 18.3, 1024^2 17.3 / 16.6 / 16.7 / 16.6 / 16.6 ms; with M4
+// 1024^2 11.88 / 11.85 / 11.81 at 8 / 12 / 16, 400^2 at depths 8.8 / 9.5 / 10.4.
 // 4 blocks of 128 per SM (128 registers): 12.7 ms against 16.1 / 13.0 / 13.0 / 14.8 at
 // 3 / 5 / 6 / 8 for 1.5e6 particles on 1024^2 lines.
-constexpr int LTILE_PROBE = 512, LTILE_SHARE = 8;
+constexpr int LTILE_PROBE = 512, LTILE_SHARE = 12;
 constexpr int LREC = 14;   // doubles per staged leaf: x, y, z, (K h)^2, the aux record, four columns; two of padding
 
 // WEIGH estimates the tiles' work instead, for the order they are taken in: the leaves of the subtrees of
