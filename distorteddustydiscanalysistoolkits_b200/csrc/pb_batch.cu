@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(128, 8) k_batch_walk(const BatchDisc *__restri
         const BatchDisc &D = discs[__ldg(slot_disc + lo)];
         const int64_t qi = s0 + t - __ldg(starts + lo);
         walk_query<STRAT>(D.T, P, t, (uint32_t)t, __ldg(D.qx + qi), __ldg(D.qy + qi), __ldg(D.qz + qi),
-                          kernel_valid(D.T.kernel), s_walk[wib], lane);
+                          kernel_valid(D.T.kernel), walk_scan<STRAT>(D.T), s_walk[wib], lane);
     }
 }
 

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(128, 8) k_query(DevTree T, int64_t nq, const d
         if (T.root == 0) {
             if (d2_point(px, py, pz, ldg4(T.leaf)) <= r2) S.append(1u, 0, 0);
         } else {
-            WarpWalk<GATHER, ListSink> W(T, S, s_walk[wib], lane);
+            WarpWalk<GATHER, ListSink> W(T, S, s_walk[wib], lane, WALK_SCAN);
             W.run(px, py, pz, 0.0, r2);
         }
         if (counts && lane == 0) counts[i] = S.count;

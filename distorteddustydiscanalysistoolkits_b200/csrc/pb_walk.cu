@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(128, 8) k_walk(DevTree T, RunPool P, int64_t m
     __shared__ int s_walk[4][RUN_WALK_SMEM];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const double K = kernel_valid(T.kernel);
+    const int scan = walk_scan<STRAT>(T);
     const int64_t nlong = longs.used();
     // tickets: the listed queries one by one, then all others, `ticket` at a time
     for (;;) {
@@ -98,7 +99,7 @@ __global__ void __launch_bounds__(128, 8) k_walk(DevTree T, RunPool P, int64_t m
             const int64_t j = t < nlong ? (int64_t)longs.list[t] : k;
             if (nlong > 0 && t >= nlong && long_walk(T, P.bnear[j])) continue;   // walked already
             const uint32_t qi = __ldg(ql + j);
-            walk_query<STRAT>(T, P, j, qi, __ldg(qx + qi), __ldg(qy + qi), __ldg(qz + qi), K, s_walk[wib], lane);
+            walk_query<STRAT>(T, P, j, qi, __ldg(qx + qi), __ldg(qy + qi), __ldg(qz + qi), K, scan, s_walk[wib], lane);
         }
     }
 }

@@ -28,6 +28,11 @@ namespace pb {
 // A scanned leaf skips the tests of the nodes between it and the subtree; they could only have cut it
 // off where its radius exceeds theirs, that is where an h is negative: such trees are opened to the leaves.
 constexpr int WALK_SCAN = 16;
+template <int STRAT>
+__device__ __forceinline__ int walk_scan(const DevTree &T)
+{
+    return STRAT != GATHER && (__ldg(T.odd) & ODD_NEGATIVE_H) ? 1 : WALK_SCAN;
+}
 constexpr int WSTACK = 512;   // entries; taken one at a time above WSTACK - 160, where a round adds at most one
 constexpr int WALK_SMEM = WSTACK + 128;       // ints of shared memory per warp of a WarpWalk
 constexpr int RUN_WALK_SMEM = WALK_SMEM + 128;   // and of one into a RunSink
@@ -103,10 +108,11 @@ struct WarpWalk {
     int *clo, *clen;          // 64 candidates in DFS order: first leaf, and the number of leaves to be tested
                               // or minus the number of leaves accepted as a whole
     int lane;
+    int scan;                 // walk_scan of the tree
     int cand = 0;             // candidates
 
-    __device__ __forceinline__ WarpWalk(const DevTree &t, SINK &s, int *smem, int l)
-        : T(t), sink(s), stack(smem), clo(smem + WSTACK), clen(smem + WSTACK + 64), lane(l)
+    __device__ __forceinline__ WarpWalk(const DevTree &t, SINK &s, int *smem, int l, int sc)
+        : T(t), sink(s), stack(smem), clo(smem + WSTACK), clen(smem + WSTACK + 64), lane(l), scan(sc)
     {
     }
     // tests the leaves of the first k <= 32 candidates, passes on what is accepted and removes them;
@@ -168,7 +174,6 @@ struct WarpWalk {
         const float bulk_lim = __fmul_rd(__double2float_rd(r2a), MARGIN_DN);
         const unsigned below = (1u << lane) - 1u;
         const unsigned limit = 2u * (unsigned)n + 64u;   // every round settles or opens at least one entry
-        const int scan = STRAT != GATHER && (__ldg(T.odd) & ODD_NEGATIVE_H) ? 1 : WALK_SCAN;
         unsigned guard = 0;
         int size = 1;
         if (lane == 0) stack[0] = T.root;
@@ -328,13 +333,13 @@ __device__ __forceinline__ int64_t nearest_leaf_warp(const DevTree &T, double px
 
 // The walk of the j-th listed query (sample point qi at px, py, pz; nearest sorted leaf P.bnear[j]):
 // its run list, its number of accepted leaves, and whether the pool was full (the query is then
-// listed as deferred).  Every lane of the warp calls it; smem holds RUN_WALK_SMEM ints.
+// listed as deferred).  scan is walk_scan of the tree.  Every lane of the warp calls it; smem holds RUN_WALK_SMEM ints.
 template <int STRAT>
 __device__ __forceinline__ void walk_query(const DevTree &T, const RunPool &P, int64_t j, uint32_t qi, double px,
-                                           double py, double pz, double K, int *smem, int lane)
+                                           double py, double pz, double K, int scan, int *smem, int lane)
 {
     RunSink R(P, smem + WALK_SMEM, lane);
-    WarpWalk<STRAT, RunSink> W(T, R, smem, lane);
+    WarpWalk<STRAT, RunSink> W(T, R, smem, lane, scan);
     bool ok = P.count_only || *(volatile unsigned long long *)P.used < P.cap;   // else the pool is exhausted
     ok = __shfl_sync(0xffffffffu, ok, 0);
     if (ok) {
