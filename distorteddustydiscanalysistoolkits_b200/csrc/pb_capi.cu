@@ -141,10 +141,15 @@ cudaError_t read_words(Handle &H, const void *dev, size_t bytes, void *out)
     return e;
 }
 
-// whether k arrays of `bytes` each go packed: all in host memory, and small
+// whether k arrays of `bytes` each go packed: all in host memory, and small.  Larger arrays are better off
+// one by one: the driver copies a piece into its own page-locked memory while the one before it travels.
+// Nearest searches of 40,000 / 80,000 points (three arrays of 320 / 640 KB) packed in ordinary memory 0.28 /
+// 0.45 ms, page-locked 0.25 / 0.37, one by one 0.23 / 0.34; calls on ten arrays of 192 KB 1.45, 1.01 and 1.36 ms.
+constexpr size_t PACK_EACH = size_t(128) << 10, PACK_EACH_PINNED = size_t(256) << 10;
+
 bool packs(const Handle &H, const void *const *p, int k, size_t bytes)
 {
-    if (bytes * (size_t)k > PIN_MAX) return false;
+    if (bytes > (H.pin ? PACK_EACH_PINNED : PACK_EACH) || bytes * (size_t)k > PIN_MAX) return false;
     for (int i = 0; i < k; ++i)
         if (!p[i] || ptr_place(H, p[i]) != 0) return false;
     return true;

@@ -44,3 +44,30 @@ def test_option_range(backend):
     for value in (-1, 1 << 31):
         with pytest.raises(pb.ArgumentError):
             backend.handle.set_option("pin_after", value)
+
+
+# 16,384 particles, points or lines are the last to be packed in ordinary memory, 32,768 in page-locked memory
+@pytest.mark.parametrize("after", [0, 1])
+@pytest.mark.parametrize("n", [16384, 16385, 32768, 32769])
+def test_largest_arrays(after, n):
+    p = synthetic.disc(n, seed=4)
+    g = np.random.default_rng(n)
+    q = [g.uniform(-90.0, 90.0, n), g.uniform(-90.0, 90.0, n), g.normal(0.0, 3.0, n)]
+    cat = pb.InterpolationCatalog(("v",), scalars=("v",))
+    got = []
+    for option in (after, 0):
+        be = pb.CUDAComputeBackend(0)
+        try:
+            be.handle.set_option("pin_after", option)
+            for _ in range(2):
+                cols = [p[k].copy() for k in ("x", "y", "z", "m", "h", "rho", "vx")]
+                inp = pb.InterpolationInput(*cols[:6], (cols[6],))
+                grids = pb.PointSamples_interpolation(be, pb.PointSamples(np.zeros(n), q), inp, cat, pb.itpGather).grids
+                d = [np.zeros(n), np.zeros(n), np.ones(n)]
+                lines = pb.LineSamples_interpolation(be, pb.LineSamples(np.zeros(n), q, d), inp, cat, pb.itpScatter).grids
+                got.append([grids[0].grid, lines[0].grid, *cols])
+        finally:
+            be.close()
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert np.array_equal(a.view(np.uint64), b.view(np.uint64))
