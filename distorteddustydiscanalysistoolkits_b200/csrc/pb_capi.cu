@@ -729,10 +729,11 @@ bool grow_pool(Handle &H)
     return true;
 }
 
-// A query of more accepted leaves than an even share of the launch's FP64 pairs over the resident
-// warps (148 x 28), and of at least BLOCK64_MIN, is summed by a whole block: one warp would still be
-// at it when the others have finished.  6,000 particles, 2,744 points: 0.07 ms at 1024, 0.11 at 2048, 0.16
-// at 8192.
+// A query of more accepted leaves than 1/BLOCK64_SHARE of the launch's FP64 pairs, and of a higher size class
+// than BLOCK64_MIN (that is, of 1,280 and more), is summed by a whole block: one warp would still be at it
+// when the others (about 3,000 resident) have finished.  Shares of 1/2048 and 1/4096 are the best of 1/2048 to
+// 1/65536 (64^3 points 5.3 ms, larger denominators slower).  6,000 particles, 2,744 points: 0.07 ms at a least
+// count of 1024, 0.11 at 2048, 0.16 at 8192.
 constexpr int64_t BLOCK64_SHARE = 4096, BLOCK64_MIN = 1024;
 
 // FP32-compensated points in two phases: the walk kernel writes every query's accepted runs,

@@ -145,9 +145,8 @@ __host__ __device__ inline double kernel_valid(int k) { return k == 1 ? 2.5 : (k
 
 // ---------------------------------------------------------------------------------
 // Squared distances.  Explicit round-to-nearest intrinsics keep these free of FMA
-// contraction so that (a) the leaf test reproduces the reference's FP64 value bit for
-// bit (LinearBVHTraversalMacros.jl:800-814) and (b) the box bound computed with the same
-// operation sequence is never larger than the leaf distance of any leaf inside the box.
+// contraction so that the leaf test reproduces the reference's FP64 value bit for
+// bit (LinearBVHTraversalMacros.jl:800-814).
 __device__ __forceinline__ double d2_point(double px, double py, double pz, const double4 &L)
 {
     double dx = __dsub_rn(px, L.x);
@@ -156,22 +155,6 @@ __device__ __forceinline__ double d2_point(double px, double py, double pz, cons
     double s = __dmul_rn(dx, dx);
     s = __dadd_rn(s, __dmul_rn(dy, dy));
     s = __dadd_rn(s, __dmul_rn(dz, dz));
-    return s;
-}
-
-__device__ __forceinline__ double axis_gap(double p, double a, double b)
-{
-    return p < a ? __dsub_rn(a, p) : (p > b ? __dsub_rn(p, b) : 0.0);
-}
-
-__device__ __forceinline__ double d2_box(double px, double py, double pz, const NodeF &nd)
-{
-    double tx = axis_gap(px, (double)nd.lox, (double)nd.hix);
-    double ty = axis_gap(py, (double)nd.loy, (double)nd.hiy);
-    double tz = axis_gap(pz, (double)nd.loz, (double)nd.hiz);
-    double s = __dmul_rn(tx, tx);
-    s = __dadd_rn(s, __dmul_rn(ty, ty));
-    s = __dadd_rn(s, __dmul_rn(tz, tz));
     return s;
 }
 
@@ -255,15 +238,6 @@ __device__ __forceinline__ double jl_pow(double x, int n)
     }
     double err = fma(y, xnlo, x * ynlo);
     return (isfinite(x) && isfinite(err)) ? fma(x, y, err) : x * y;
-}
-
-__device__ __forceinline__ float jl_pow(float x, int n)
-{
-    float y = x;
-#pragma unroll
-    for (int i = 1; i < 8; ++i)
-        if (i < n) y *= x;
-    return y;
 }
 
 template <typename R>
@@ -350,40 +324,6 @@ __device__ __forceinline__ R knorm3(int k)
     case 4: return R(495) / (R(256) * pi);
     default: return R(1365) / (R(512) * pi);
     }
-}
-
-// Smoothed_kernel_function(K, r, h, Val(3)) -- kernel.jl:152-157
-template <typename R>
-__device__ __forceinline__ R Wfun(int k, R r, R h)
-{
-    R invh = R(1) / h;
-    R inv_hD = invh * invh * invh;
-    R q = r * invh;
-    return inv_hD * (knorm3<R>(k) * kshape<R>(k, q));
-}
-
-// Smoothed_gradient_kernel_function(K, dx, dy, dz, h) -- kernel.jl:284-296,371-376.
-// Only the scalar coefficient is returned: grad = coeff * (dx, dy, dz) with
-// coeff = inv_hDp1 * (dW(q)*norm*invr); the reference forms inv_hDp1 * (dx*coeff') per
-// component, so the exact path multiplies in that order itself.
-template <typename R>
-__device__ __forceinline__ void gradW(int k, R dx, R dy, R dz, R r, R h, R &gx, R &gy, R &gz)
-{
-    R invh = R(1) / h;
-    R inv_hDp1 = invh * invh * invh * invh;
-    R cx = R(0), cy = R(0), cz = R(0);
-    R r2 = dx * dx + dy * dy + dz * dz;
-    if (r2 != R(0)) {
-        R invr = R(1) / r;
-        R q = r / h;
-        R coeff = kdshape<R>(k, q) * knorm3<R>(k) * invr;
-        cx = dx * coeff;
-        cy = dy * coeff;
-        cz = dz * coeff;
-    }
-    gx = inv_hDp1 * cx;
-    gy = inv_hDp1 * cy;
-    gz = inv_hDp1 * cz;
 }
 
 }  // namespace pb

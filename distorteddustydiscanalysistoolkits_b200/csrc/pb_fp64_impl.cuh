@@ -5,7 +5,7 @@
 //
 // The FP64 pipe (64 lanes per SM: two issue cycles per warp instruction) bounds these kernels,
 // so the terms are arranged to need fewer FP64 operations for the same bits: 1/h and 1/rho of a
-// particle come from the tree (DevTree::inv), quotients by a number whose reciprocal is known
+// particle come from the tree (DevTree::aux), quotients by a number whose reciprocal is known
 // take five operations (div_by), pieces and supports are selected by integer compares on the
 // high word, the kernel family and the catalog's shape are compile-time, and a side (h_a or
 // h_b) whose support the pair lies outside of is skipped: its terms are zeros.
@@ -120,7 +120,8 @@ __device__ __forceinline__ double dshape64(double q)
 }
 
 // One side of a pair's kernel (h = h_a or h_b with its correctly rounded reciprocal): W(r, h) and,
-// with GRAD, the gradient's coefficient times the offset, in Wfun's and gradW's operation order.
+// with GRAD, the gradient's coefficient times the offset, in the operation order of kernel.jl:152-157 (W) and
+// kernel.jl:284-296,371-376 (gradient).
 // A pair outside the support of h (by more than the rounding of either quotient) is left out: its
 // terms are zeros, which change no sum.  `regular` is false where some particle's h is negative,
 // zero or extreme: then the reference's general expressions are evaluated.
@@ -241,7 +242,7 @@ __device__ __forceinline__ void terms64(const DevCatalog &C, const Query64 &Q, c
     const double r = sqrt(d2);
     const bool rsafe = exp_safe(r);
     const double invrb = N.X.y, mb = N.X.z, rb = N.X.w;
-    // gradW's 1/r; 0 stands for a coincident pair, which has no gradient terms
+    // the gradient's 1/r; 0 stands for a coincident pair, which has no gradient terms
     const double invr = grad && d2 != 0.0 ? 1.0 / r : 0.0;
     double W, gx, gy, gz;
     auto side = [&](double h, double invh, double &w, double &x, double &y, double &z) {

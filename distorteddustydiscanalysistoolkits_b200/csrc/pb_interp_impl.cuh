@@ -226,12 +226,11 @@ __device__ __forceinline__ int64_t nearest_leaf(const DevTree &T, double px, dou
 struct Walk {
     int node;
     int64_t cur, end, guard, limit;
-    int stop = 0;   // node where the walk ends: 0 for the whole tree, a subtree's escape target for a subtree
 };
 
 // The walk's pruning decision for internal node `node` (box `nd`): FP32 box distance with
 // directed rounding against the node radius (query radius and/or K * hmax) with the 2^-20
-// margin.  Shared by the walk and by the subtree prefilter so both decide alike.
+// margin.  Shared by every walk of a query, so that all decide alike.
 template <int STRAT>
 __device__ __forceinline__ bool node_pruned(const DevTree &T, const NodeF &nd, int node, const QBox &q, float Kf,
                                             float r2a_up)
@@ -262,7 +261,7 @@ __device__ __forceinline__ bool next_item(const DevTree &T, Walk &w, double px, 
     const float bulk_lim = __fmul_rd(__double2float_rd(r2a), MARGIN_DN);
     for (;;) {
         if (w.cur <= w.end) {   // linear scan of a small subtree's leaves
-            if (++w.guard > w.limit) { flag(T.status, ST_TRAVERSAL); w.cur = 1; w.end = 0; w.node = w.stop; return false; }
+            if (++w.guard > w.limit) { flag(T.status, ST_TRAVERSAL); w.cur = 1; w.end = 0; w.node = 0; return false; }
             const int64_t b = w.cur++;
             const double4 L = ldg4(T.leaf + b);
             double r2;
@@ -275,8 +274,8 @@ __device__ __forceinline__ bool next_item(const DevTree &T, Walk &w, double px, 
             if (d2_point(px, py, pz, L) <= r2) { lo = hi = b; return true; }
             continue;
         }
-        if (w.node == w.stop) return false;
-        if (++w.guard > w.limit) { flag(T.status, ST_TRAVERSAL); w.node = w.stop; return false; }
+        if (w.node == 0) return false;
+        if (++w.guard > w.limit) { flag(T.status, ST_TRAVERSAL); w.node = 0; return false; }
         const int node = w.node;
         if (node >= n) {
             int64_t b = node - n;
