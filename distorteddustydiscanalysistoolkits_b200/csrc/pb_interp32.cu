@@ -54,9 +54,11 @@ __global__ void __launch_bounds__(128) k_points32w(DevTree T, DevCatalog C, cons
 // The block waits for the slowest of the four, which costs more than it gives where there are few
 // queries a warp, or no size classes to make the four alike (the plain order): a warp each then.
 // Together / a warp each, 2^20 particles: 269,000 queries 223.6 / 227.2 ms, 81,407 67.8 / 68.6, 32,946 28.6 / 28.8,
-// 9,910 14.4 / 13.6, 4,237 14.2 / 10.9, 1,329 13.9 / 9.5; plain order 269,000 237.0 / 230.3, 1,329 9.2 / 8.6.
+// 9,910 14.4 / 13.6, 4,237 14.2 / 10.9, 1,329 13.9 / 9.5; 2^21: 23,720 55.0 / 57.8, 18,929 46.9 / 45.7, 14,869 36.1 /
+// 37.4, 8,759 28.6 / 27.0; 2^19: 20,002 14.7 / 15.0, 11,537 8.8 / 8.9, 6,176 5.61 / 5.51; plain order, 2^20: 269,000
+// 237.0 / 230.3, 1,329 9.2 / 8.6.
 // (A choice at run time inside one kernel spoils the code of the single warps: 4,237 queries 12.4 ms.)
-constexpr int TOGETHER_MIN = 8;   // queries a resident warp
+constexpr int TOGETHER_MIN = 4;   // queries a resident warp
 
 template <int STRAT, int KT, int CAT, bool TOGETHER>
 __global__ void __launch_bounds__(128, 5) k_pairs32w(DevTree T, DevCatalog C, const float4 *__restrict__ pay, int stride,

@@ -1,5 +1,5 @@
 """FP32C pair sums dealt to blocks, four queries each (many queries, ordered by size class), and to warps (few
-queries, or the plain order): the same bits on both sides of the rule (eight queries a resident warp)."""
+queries, or the plain order): the same bits on both sides of the rule (four queries a resident warp)."""
 import numpy as np
 import pytest
 
@@ -20,7 +20,7 @@ def test_same_bits(backend, strategy):
     tree = pb.LinearBVH_build(inp, backend)
     cat = pb.InterpolationCatalog(("a",), scalars=("a",), gradients=("a",))
     # 5 blocks of 4 warps an SM are meant; around 4 to 6 of them and a few queries past each
-    edges = sorted({8 * resident * b + d for b in (4, 5, 6) for d in (-1, 0, 1, 3)})
+    edges = sorted({4 * resident * b + d for b in (4, 5, 6) for d in (-1, 0, 1, 3)})
     q = [g.normal(0.0, 1.0, edges[-1]) for _ in "xyz"]
     H = backend.handle
     H.set_option("fp64_light_max", 0)
