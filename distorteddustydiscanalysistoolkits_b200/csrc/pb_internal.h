@@ -228,8 +228,14 @@ cudaError_t launch_line_image(Handle *H, const double *a0, int64_t n0, const dou
 
 // Nearest searches of at most this many points go a warp each instead of a thread each
 // (2,744 points 131 -> 20 us, 20,000 points 222 -> 95 us; 153,600 points would take 587 us, not 297: a
-// warp reads more nodes than its lanes' own searches, but waits for a quarter of the steps)
+// warp reads more nodes than its lanes' own searches, but waits for a quarter of the steps).  In a tree of few
+// particles the steps are few: thread / warp each 83 / 91 us (100 particles, 24,000 points), 74 / 75
+// (16,000); 106 / 119 (1,000 particles, 32,000 points), 103 / 101 (24,000); 143 / 138 (8,000 particles, 32,000).
 constexpr int64_t NEAREST_WARP_MAX = 32768;
+inline int64_t nearest_warp_max(int64_t nparticles)
+{
+    return nparticles >= 4096 ? NEAREST_WARP_MAX : (nparticles >= 512 ? 24576 : 12288);
+}
 
 inline int grid_for(int64_t n, int block, int cap = 148 * 32)
 {

@@ -306,7 +306,7 @@ cudaError_t launch_stats(Handle *H, const DevTree &T, int strategy, int64_t nq, 
 cudaError_t launch_nearest(Handle *H, const DevTree &T, int64_t nq, const double *qx, const double *qy,
                            const double *qz, double *h_out, int64_t *idx_out)
 {
-    if (nq <= NEAREST_WARP_MAX)
+    if (nq <= nearest_warp_max(T.n))
         k_nearest_warp<<<grid_for(nq, 4, 1 << 30), 128, 0, H->stream>>>(T, nq, qx, qy, qz, h_out, idx_out);
     else k_nearest<<<grid_for(nq, 128, 1 << 30), 128, 0, H->stream>>>(T, nq, qx, qy, qz, h_out, idx_out);
     H->launches += 1;

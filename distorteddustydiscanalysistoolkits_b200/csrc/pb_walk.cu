@@ -192,7 +192,7 @@ cudaError_t launch_nearest_list(Handle *H, const DevTree &T, int64_t m, const ui
                    (e = cudaMemsetAsync(H->long_count.p, 0, sizeof(unsigned), H->stream))))
         return e;
     const LongList L = long_list(H, m, listed);
-    if (m <= NEAREST_WARP_MAX)
+    if (m <= nearest_warp_max(T.n))
         k_nearest_list_warp<<<grid_for(m, 4, 1 << 30), 128, 0, H->stream>>>(T, m, ql, qx, qy, qz, bnear, L);
     else k_nearest_list<<<grid_for(m, 128, 1 << 30), 128, 0, H->stream>>>(T, m, ql, qx, qy, qz, bnear, L);
     H->launches += 1;
