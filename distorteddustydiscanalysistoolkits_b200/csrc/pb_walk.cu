@@ -14,11 +14,12 @@ namespace pb {
 // takes them first: in Morton order they come last where a grid's corner lies far from the particles,
 // and the launch waited for them (SMs busy 72 % of the walk of 131,072 particles on 64^3 points).
 // Where h varies by less than that (a box of even density) every query would be on the list, walked out of
-// Morton order, a ticket each, and passed over again: with more than one query in LONG_SHARE on it the list is
-// not used.  A disc in a box has between a quarter and a half of the points on it.  Walk with shares of 1 / 2 / 4 /
-// 16: 1e6 even particles, 2e6 points 10.44 / 9.79 / 9.79 / 9.79 ms; 131,072 disc particles, 64^3 points 2.01 / 2.01 /
-// 2.41 / 2.40, 400,000 on 80 x 80 x 24 2.39 / 2.38 / 2.97 / 2.97, 2^21 on 256 x 256 x 64 97.4 / 97.4 / 97.4 / 103.0.
-constexpr int LONG_SHARE = 2;
+// Morton order, a ticket each, and passed over again: the list is not used where fewer than one query in
+// LONG_OTHERS is off it.  On discs up to 0.95 of the points may be on it, with gain.  Nearest search and walk,
+// always used / not from a half on / not from 7/8 on: 1e6 even particles, 2e6 points 11.40 / 10.74 / 10.74 ms;
+// 131,072 disc particles, 64^3 points (0.58 on the list) 2.15 / 2.83 / 2.15; 400,000 on 80 x 80 x 24 (0.57) 1.92 / 2.95 /
+// 1.93; 300,878 clumped, 129 x 138 x 63 (gather, 0.52) 9.94 / 10.65 / 9.93.
+constexpr int LONG_OTHERS = 8;
 
 __device__ __forceinline__ bool long_walk(const DevTree &T, int b)
 {
@@ -40,9 +41,11 @@ struct LongList {
 };
 
 // the list of a launch over m queries
+static unsigned long_cap(int64_t m) { return (unsigned)(m - m / LONG_OTHERS); }
+
 static LongList long_list(Handle *H, int64_t m, bool listed)
 {
-    return LongList{listed ? H->long_list.as<uint32_t>() : nullptr, H->long_count.as<unsigned>(), (unsigned)(m / LONG_SHARE + 1)};
+    return LongList{listed ? H->long_list.as<uint32_t>() : nullptr, H->long_count.as<unsigned>(), long_cap(m)};
 }
 
 __global__ void __launch_bounds__(128) k_nearest_list(DevTree T, int64_t m, const uint32_t *__restrict__ ql,
@@ -188,7 +191,7 @@ cudaError_t launch_nearest_list(Handle *H, const DevTree &T, int64_t m, const ui
                                 const double *qy, const double *qz, int *bnear, bool listed)
 {
     cudaError_t e;
-    if (listed && ((e = H->long_list.reserve(sizeof(uint32_t) * (m / LONG_SHARE + 1))) || (e = H->long_count.reserve(sizeof(unsigned))) ||
+    if (listed && ((e = H->long_list.reserve(sizeof(uint32_t) * long_cap(m))) || (e = H->long_count.reserve(sizeof(unsigned))) ||
                    (e = cudaMemsetAsync(H->long_count.p, 0, sizeof(unsigned), H->stream))))
         return e;
     const LongList L = long_list(H, m, listed);
