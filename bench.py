@@ -653,7 +653,7 @@ def main():
                 args.particles in (None, 1 << 21) and args.grid in (None, "256,256,64"):
             traffic = json.load(open(prof)).get("dram_bytes_per_launch")
         achieved = per[dom]["achieved_gbs"]
-        # The pair kernel is bound by instruction issue, not by DRAM (its DRAM traffic is 3 % of
+        # The pair kernel is bound by instruction issue, not by DRAM (its DRAM traffic is 0.4 % of
         # peak; the records are re-read from L2): pairs/s against the issue ceiling, SMs x 4
         # schedulers x SM clock / warp instructions per pair, with the instructions per pair of
         # the committed ncu capture of k_pairs32w (profiles/k_pairs32w_c2disc_96x96x24.md)

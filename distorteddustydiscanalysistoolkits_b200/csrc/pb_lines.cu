@@ -2,7 +2,7 @@
 // One thread per line walking the tree with an FP64 node bound was bound by that bound (six
 // divisions, two square roots a node) and by latency (5 % of the warp slots for a small image):
 // 1.5e6 particles on 1024^2 lines 54.6 ms, 20,011 particles on 97 x 61 oblique lines 3.18 ms.  Now
-// 11.7 ms (FP64 pipe 32 % active; the sums of 6e8 accepted pairs are most of it) and 0.29 ms.
+// 9.3 ms (FP64 pipe 32 % active; the sums of 6e8 accepted pairs are most of it) and 0.20 ms.
 // Compiled with -fmad=false: every expression is the IEEE result of the reference's operation
 // order.
 #include "line_tables.h"
@@ -301,8 +301,8 @@ __global__ void __launch_bounds__(128) k_lines_warp(DevTree T, DevCatalog C, int
 // now 6.7; 400^2 with origins at scattered depths 50.2, now 13.1.  Shares of 4 / 8 / 12 / 16 / 32: 363^2 6.9 / 6.3 /
 // 6.7 / 7.3 / 8.2, 400^2 at depths 12.9 / 12.6 / 13.1 / 14.3 / 18.3, 1024^2 17.3 / 16.6 / 16.7 / 16.6 / 16.6 ms; with M4
 // 1024^2 11.88 / 11.85 / 11.81 at 8 / 12 / 16, 400^2 at depths 8.8 / 9.5 / 10.4.
-// 4 blocks of 128 per SM (128 registers): 12.7 ms against 16.1 / 13.0 / 13.0 / 14.8 at
-// 3 / 5 / 6 / 8 for 1.5e6 particles on 1024^2 lines.
+// 3 / 4 / 5 / 6 blocks of 128 per SM (M4, 1.5e6 particles): 1024^2 lines 14.4 / 11.8 / 11.0 / 11.4 ms, 400^2 lines
+// 4.7 / 5.0 at 4 / 5; 20,011 particles, 400^2 0.58 / 0.65: four are the best where the chip is not full.
 constexpr int LTILE_PROBE = 512, LTILE_SHARE = 12;
 constexpr int LREC = 14;   // doubles per staged leaf: x, y, z, (K h)^2, the aux record, four columns; two of padding
 
@@ -514,9 +514,9 @@ __global__ void __launch_bounds__(128, 4) k_lines_tile(DevTree T, DevCatalog C, 
 constexpr int64_t LINE_TILES_MIN = 131072;
 // Particles from which on the tiles are taken by descending estimated work: in Morton order the tiles of
 // the densest part, met late, run on alone (SMs active 70 % of the time).  Subtrees of at most
-// n / 2^13 leaves are counted whole; n / 2^9 .. n / 2^15 are within 6 %.  Morton order / by work, 1024^2
-// lines of 1.5e6 particles: face-on 12.3 / 11.7 ms, oblique 16.2 / 12.8; 512^2 lines of 2e5 2.02 / 1.98,
-// of 20,011 1.34 / 1.55 (the estimate costs more than it gives).
+// n / 2^13 leaves are counted whole; n / 2^9 .. n / 2^15 are within 6 %.  Morton order / by work (M4), 1.5e6
+// particles: 1024^2 lines face-on 12.1 / 11.8 ms, oblique 12.8 / 12.2, 700^2 oblique 8.2 / 7.3; 2e5 particles: 512^2
+// 2.04 / 1.82, but 400^2 1.74 / 1.88; 20,011: 400^2 0.65 / 0.75 (the estimate costs more than it gives).
 constexpr int64_t LINE_ORDER_MIN = 262144;
 constexpr int LINE_CUT_SHIFT = 13;
 

@@ -5,6 +5,7 @@
 // accepted leaves appear in ascending sorted-leaf order exactly as in the reference.  One thread
 // per query with FP64 box tests used 4 % of the warp slots for 20,000 queries (4.2e6 particles):
 // 15.6 ms; a warp per query 0.23 ms, and 0.21 ms for the closest leaf (a nearest search of its own).
+// Many queries with few leaves each take k_query_short first.
 #include "pb_internal.h"
 #include "pb_walk_impl.cuh"
 
