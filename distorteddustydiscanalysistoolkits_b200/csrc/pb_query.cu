@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(128) k_query_short(DevTree T, int64_t nq, cons
             rest[1 + atomicAdd(rest, 1u)] = (uint32_t)i;
             continue;
         }
-        if (pool && cnt > cap) flag(T.status, ST_POOL);
+        if (pool && cnt > 0 && cnt > cap) flag(T.status, ST_POOL);   // an empty list fits any offsets
         if (counts) counts[i] = cnt;
         if (nearest) nearest[i] = ci;
         if (nearest_d2) nearest_d2[i] = cd;

@@ -53,3 +53,19 @@ def test_pool_too_small(backend):
         near = np.empty(m, np.int64)
         with pytest.raises(pb.DimensionMismatch):
             H.check(H.lib.pb_query_neighbors(H.h, m, P(q[0]), P(q[1]), P(q[2]), P(r), P(off), P(pool), P(near)), "query")
+
+
+@pytest.mark.parametrize("m", [100, 24576])
+def test_empty_lists_fit_any_offsets(backend, m):
+    """Offsets that go back are refused only for a query that has something to write."""
+    g = np.random.default_rng(4)
+    x = g.random((3, 300))
+    one = np.ones(300)
+    tree = pb.LinearBVH_build(pb.InterpolationInput(*[c.copy() for c in x], one.copy(), one.copy(), one.copy(), ()), backend)
+    q = g.uniform(5.0, 6.0, (3, m))   # nothing within 0.1
+    off = np.arange(m + 1, dtype=np.int64) % 3
+    off[-1] = 0
+    r, pool, near = np.full(m, 0.1), np.full(4, -7, np.int64), np.empty(m, np.int64)
+    H, P = tree.handle, pb._lib.ptr
+    H.check(H.lib.pb_query_neighbors(H.h, m, P(q[0]), P(q[1]), P(q[2]), P(r), P(off), P(pool), P(near)), "query")
+    assert (near == -1).all() and (pool == -7).all()
