@@ -1592,7 +1592,8 @@ int check_statuses(pb_handle *const *discs, int32_t ndiscs)
         return batch_fail(discs[0], PB_ERR_CUDA, std::string("batched launch: ") + cudaGetErrorString(e));
     }
     for (int32_t k = 0; k < ndiscs; ++k) {
-        int rc = check_status(discs[k]->H, H0);
+        Handle &Hk = discs[k]->H;   // builds alone may be checked on streams of their own
+        int rc = check_status(Hk, Hk.stream == H0.stream && Hk.device == H0.device ? H0 : Hk);
         if (rc) return batch_fail(discs[0], rc, "disc " + std::to_string(k) + ": " + discs[k]->H.err);
     }
     return PB_OK;
